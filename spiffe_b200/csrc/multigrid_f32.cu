@@ -30,29 +30,39 @@
 // correction; the last pre-smoothing colour leaves a zero residual at its
 // own nodes, so the restriction evaluates the residual only at the others.
 //
-// One cooperative launch runs the whole solve.  Levels with more than
-// MG_TAIL_NODES nodes are worked by every CTA with grid barriers between the
-// colour sweeps; on the nine-point ones each CTA owns a band of rows, so the
-// two colours of one row parity, which depend on each other only within a
-// row, need a CTA barrier between them and a grid barrier only before the
-// other parity (two grid barriers a sweep, not four, same update order).
-// The residual pass also makes level 0's first colour-0 sweep (from u = 0
-// it needs no neighbours) and the last post-smoothing sweep adds u to Psi,
-// saving two passes and two barriers a cycle.  The smaller levels, down to
-// the coarsest (solved exactly by its precomputed inverse when it has at
-// most MG_MAX_DIRECT unknowns, else by Gauss-Seidel sweeps), are worked by
-// CTA 0 alone with CTA barriers while the others wait at the next grid
-// barrier.  Data written inside the launch are read after the acquire of a
-// grid barrier.  The sums that drive the stop rule are per-CTA partials
-// added in the same order by every CTA, so every CTA takes the same
-// decision and the result does not depend on timing.  Every barrier wait is
-// bounded; on time-out the kernel raises SPIFFE_DEV_ERR_BARRIER and every
-// CTA returns.
+// A solve is one CUDA graph: a kernel for level 0's residual and way down,
+// then a WHILE node around a V-cycle of one kernel a level and direction that
+// ends with the next residual; the last CTA of that kernel adds the sums in a
+// fixed order and decides whether the loop goes on, so the decision does not
+// depend on timing and the host is not asked.  What bounded the previous
+// form (one cooperative launch with a grid barrier between colour sweeps,
+// about 51 a V-cycle) was those barriers with the L2 round trips between
+// them, 3.5 to 7 us each; DRAM was 1 % busy.  Here a kernel works a band of
+// rows of its level in shared memory through all sweeps of its direction: it
+// loads the band and a halo of one row per row the sweeps reach (five on the
+// way down, from u = 0; four up), recomputes the neighbours' values in the
+// halo instead of fetching them, and so needs no exchange until the next
+// kernel.  Separate kernels rather than phases of one, because each then has
+// the registers it needs (in one kernel the compiler spilled, and with most
+// of the SM's memory taken as shared memory the spills went to L2: the same
+// phases took two to three times as long) and because no CTA waits for
+// another, so solves of several instances share the SMs.  Values and update
+// order are those of the sweeps run over the whole mesh.
+// Levels of at most MG_TAIL_NODES nodes are worked together by one CTA, the
+// coarsest solved exactly by its precomputed inverse when it has at most
+// MG_MAX_DIRECT unknowns, else by Gauss-Seidel sweeps.  Coefficients are kept
+// per distinct row (class): in a gun nearly all rows of a level are alike, so
+// a band's fit L1 and a thread keeps its columns' in registers.
+// Measured from a cold start to 1e-6 (B200): 3001 x 821 gun, 6 cycles, 1.6 ms
+// -> 1.07 ms; 1500 x 400, 7 cycles, 1.13 -> 0.65; 424 x 232, 9 cycles, 0.99
+// -> 0.61; 601 x 165, 5 cycles, 0.69 -> 0.39.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <system_error>
 #include <thread>
+#include <unordered_map>
 #include <vector>
 
 #include "modules.cuh"
@@ -60,566 +70,513 @@
 
 namespace {
 
-constexpr int MG_NT = 1024;           // threads per CTA
-constexpr int MG_TAIL_NODES = 3000;   // levels at most this large are worked by CTA 0 alone
-constexpr int MG_MIN_UNKNOWNS = 64;   // coarsening stops at this many unknowns
-constexpr int MG_NODES_PER_CTA = 8192; // mesh nodes per CTA below one CTA per SM
-constexpr int MG_MAX_DIRECT = 1024;   // a coarsest level of at most this many unknowns is solved exactly
+constexpr int MG_NT = 512;             // threads per CTA
+constexpr int MG_W = MG_NT / 32;       // warps per CTA
+constexpr int MG_TAIL_NODES = 3000;    // levels at most this large are worked by one CTA together
+constexpr int MG_MIN_UNKNOWNS = 64;    // coarsening stops at this many unknowns
+constexpr int MG_NODES_PER_CTA = 4096; // mesh nodes per band below one band per SM
+constexpr int MG_MIN_ROWS = 4;         // own rows of a coarse level's band at least
+constexpr int MG_MAX_DIRECT = 1024;    // a coarsest level of at most this many unknowns is solved exactly
+constexpr int MG_COARSE_SWEEPS = 24;   // sweeps on a larger one
+constexpr int MG_DOWN = 5, MG_UP = 4;  // halo rows a side of a band on the way down and up
 enum { MG_INVD = 8, MG_DIAG = 9 };
 
-struct Mg32Args {
+// One solve's arguments and its state between the graph's kernels.
+struct MgCall {
   double *Psi;
   const double *rhs; // null: Laplace solve
   const uint8_t *umask;
-  float *u0, *f0;
-  const float *crow, *drow;
-  int nz, P0, lo, hi, cols;
-  float a, c4, e, e2c, inv_e, inv_e2c;   // level-0 operator in FP32
-  double a_d, e_d, c4_d, e2c_d, dr2_inv; // and in FP64 for the residual
-  int nlev, tail, nu0, nu, coarse_sweeps, max_cycles;
-  const float *cinv; // the coarsest level's inverse, cn x cn row-major (null: coarse sweeps)
-  const int *cidx;   // its unknowns' array indices on that level
-  int cn;
-  double accuracy;
-  MgLevel lev[MG_MAX_LEVELS];
-  unsigned long long *bar; // [0] arrivals, [16] abort
-  double *part;            // [grid][2]
+  double accuracy, drive;
+  long long max_cycles, cycles;
   PcState *st;
   long long *iters_out;
+  DevCounts *cnt;
+  unsigned ticket; // bands of the residual that are done
+  int skip;
 };
 
-__device__ __forceinline__ unsigned long long mg_ld_acquire(const unsigned long long *p)
-{
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ unsigned long long mg_ld_relaxed(const unsigned long long *p)
-{
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Grid barrier over a monotonic arrival counter (barrier number gen, counted
-// from 1 by every thread alike).  Bounded: after 2^24 polls, or once another
-// CTA has given up, it returns false in every thread of the CTA.
-__device__ bool mg_grid_sync(const Mg32Args &a, unsigned &gen, DevCounts *cnt)
-{
-  __shared__ int ok_sh;
-  gen++;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(a.bar), "l"(1ull) : "memory");
-    const unsigned long long target = (unsigned long long)gridDim.x * gen;
-    unsigned long long polls = 0;
-    while (mg_ld_acquire(a.bar) < target) {
-      if (mg_ld_relaxed(a.bar + 16)) {
-        ok = 0;
-        break;
-      }
-      if (++polls > (1ull << 24)) {
-        atomicOr(&cnt->error, SPIFFE_DEV_ERR_BARRIER);
-        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(a.bar + 16), "l"(1ull) : "memory");
-        ok = 0;
-        break;
-      }
-      if (polls > 32)
-        __nanosleep(32);
-    }
-    ok_sh = ok;
-  }
-  __syncthreads();
-  return ok_sh != 0;
-}
-
-// ---- level 0: the mesh, five-point operator
-
-__device__ __forceinline__ bool unknown0(const Mg32Args &a, int iz, int ir, size_t j)
-{
-  return iz >= a.lo && iz <= a.hi && ir < a.cols && !(a.umask[j] & S32_U_METAL);
-}
-
-// neighbour sum of the level-0 operator at an unknown node (poisson.c:57-117)
-__device__ __forceinline__ float nb0(const Mg32Args &a, const float *u, int iz, int ir, size_t j)
-{
-  const long P = a.P0;
-  const float up = (iz == a.nz - 1 && a.hi == a.nz - 1) ? *(u + j - P) : *(u + j + P);
-  const float dn = (iz == 0 && a.lo == 0) ? *(u + j + P) : *(u + j - P);
-  if (ir == 0)
-    return a.a * (up + dn) + a.c4 * *(u + j + 1);
-  return a.a * (up + dn) + __ldg(a.crow + ir) * *(u + j + 1) + __ldg(a.drow + ir) * *(u + j - 1);
-}
-
-__device__ __forceinline__ float res0(const Mg32Args &a, int iz, int ir)
-{
-  const size_t j = node(iz, ir, a.P0);
-  if (!unknown0(a, iz, ir, j))
-    return 0.f;
-  return *(a.f0 + j) - nb0(a, a.u0, iz, ir, j) - (ir ? a.e : a.e2c) * *(a.u0 + j);
-}
-
-// Four consecutive columns c0 .. c0+3 of a level-0 row: what a colour
-// sweep reads: 16-byte loads of u on the row and its two neighbours, of f
-// and of the mask; the scalars left and right of the group.
-struct Cols0 {
-  float4 um, dm, u, f;
-  uchar4 mk;
-  float left, right;
-  int j, iz, c0; // j: array index (level 0 has fewer than 2^31 nodes)
+// Level 0's size, update region and operator.
+struct Mg0 {
+  int nz, P, lo, hi, cols;
+  int rp, nb;                     // rows of a band, bands
+  float a, e, e2c, inv_e, inv_e2c;
+  double a_d, e_d, e2c_d;         // in FP64 for the residual
+  float *u, *f;                   // the pre-smoothed u and f (NaN where no equation holds) of every row
+  const float *crow, *drow;       // the radial couplings of a column in FP32, P values
+  const double *cpd, *cmd;        // and in FP64
+  double *part;                   // the bands' sums, two a band
 };
 
-__device__ __forceinline__ void cols0_load(const Mg32Args &a, long t, int G, Cols0 &k)
+__device__ __forceinline__ float4 ldcg4(const float *p) { return __ldcg(reinterpret_cast<const float4 *>(p)); }
+__device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+
+extern __shared__ float4 mg_smem[];
+
+// A CTA's buffer: its shared memory, or its part of `scratch` for meshes whose bands do not fit there.
+template <bool SM> __device__ __forceinline__ float *band_buf(float *scratch, size_t scratch_n)
 {
-  const long P = a.P0;
-  const int row = (int)(t / G), g = (int)(t - (long)row * G);
-  k.iz = a.lo + row;
-  k.c0 = 4 * g;
-  k.j = (int)node(k.iz, k.c0, a.P0);
-  const bool top = k.iz == a.nz - 1 && a.hi == a.nz - 1, bottom = k.iz == 0 && a.lo == 0;
-  k.um = *reinterpret_cast<const float4 *>(a.u0 + (top ? k.j - P : k.j + P));
-  k.dm = *reinterpret_cast<const float4 *>(a.u0 + (bottom ? k.j + P : k.j - P));
-  k.u = *reinterpret_cast<const float4 *>(a.u0 + k.j);
-  k.f = *reinterpret_cast<const float4 *>(a.f0 + k.j);
-  k.mk = *reinterpret_cast<const uchar4 *>(a.umask + k.j);
-  k.left = k.c0 > 0 ? a.u0[k.j - 1] : 0.f;
-  k.right = a.u0[k.j + 4];
+  return SM ? reinterpret_cast<float *>(mg_smem) : scratch + (size_t)blockIdx.x * scratch_n;
 }
 
-// New values of the group's nodes of colour c ((iz+ir)%2 == c); fin keeps
-// the others' values.  Bit q of the result: node c0+q is an unknown.
-// Every index into the small arrays is a compile-time constant, so they
-// live in registers.
-__device__ __forceinline__ unsigned cols0_relax(const Mg32Args &a, int c, const Cols0 &k, float fin[4])
+// ---- level 0: the mesh, five-point operator.  A band buffer holds rows r0,
+// r0+1, ... of u (U) and f (F) at the mesh pitch P0, each row as its even
+// columns and then (from H = P0/2) its odd ones, so that the nodes of one
+// colour in a row are consecutive; u0 and f0 have the same layout.  f is NaN
+// at a node without an equation (metal, outside rows lo..hi, columns >= cols),
+// whose u stays 0.
+
+// A thread's share of level 0: four consecutive nodes of a half row (eight
+// columns) in rows g, g+groups, ..., their radial couplings in registers.
+struct Part0 {
+  int j, g, groups; // first half-column; row group; j < 0: no share
+  float cE[4], dE[4], cO[4], dO[4]; // couplings outwards and inwards, even and odd columns
+  float inv0, e0;                   // 1/e and e of the first even column (the axis has its own)
+};
+
+// column groups of level 0
+__device__ __forceinline__ int cols0(const Mg0 &z) { return (((z.cols + 1) >> 1) + 3) >> 2; }
+
+__device__ __forceinline__ void part0(const Mg0 &z, Part0 &t, int kb)
 {
-  const float uu[6] = {k.left, k.u.x, k.u.y, k.u.z, k.u.w, k.right};
-  const float ups[4] = {k.um.x, k.um.y, k.um.z, k.um.w}, dns[4] = {k.dm.x, k.dm.y, k.dm.z, k.dm.w};
-  const float fs[4] = {k.f.x, k.f.y, k.f.z, k.f.w};
-  const uint8_t ms[4] = {k.mk.x, k.mk.y, k.mk.z, k.mk.w};
-  fin[0] = k.u.x;
-  fin[1] = k.u.y;
-  fin[2] = k.u.z;
-  fin[3] = k.u.w;
-  unsigned unk = 0;
+  const int n = cols0(z), W = (n + 31) & ~31; // padded to whole warps
+  t.groups = W < MG_NT ? MG_NT / W : 1;
+  t.g = W < MG_NT ? threadIdx.x / W : 0;
+  const int k = kb + (int)threadIdx.x - t.g * W;
+  t.j = k < n && t.g < t.groups ? 4 * k : -1;
+  if (t.j < 0)
+    return;
 #pragma unroll
   for (int q = 0; q < 4; q++) {
-    const int ir = k.c0 + q;
-    if (ir >= a.cols || (ms[q] & S32_U_METAL))
-      continue;
-    unk |= 1u << q;
-    if (((k.iz + ir) & 1) != c)
-      continue;
-    float nb;
-    if (ir == 0)
-      nb = a.a * (ups[q] + dns[q]) + a.c4 * uu[q + 2];
-    else
-      nb = a.a * (ups[q] + dns[q]) + __ldg(a.crow + ir) * uu[q + 2] + __ldg(a.drow + ir) * uu[q];
-    fin[q] = (fs[q] - nb) * (ir ? a.inv_e : a.inv_e2c);
+    t.cE[q] = __ldg(z.crow + 2 * (t.j + q));
+    t.dE[q] = __ldg(z.drow + 2 * (t.j + q));
+    t.cO[q] = __ldg(z.crow + 2 * (t.j + q) + 1);
+    t.dO[q] = __ldg(z.drow + 2 * (t.j + q) + 1);
   }
-  return unk;
+  t.inv0 = t.j ? z.inv_e : z.inv_e2c;
+  t.e0 = t.j ? z.e : z.e2c;
 }
 
-// One colour c of red-black Gauss-Seidel on level 0: nodes with (iz+ir)%2 ==
-// c, a group of four columns per task; the group's other two nodes, which
-// this colour's updates only read, are left as they are.  With FOLD (the
-// V-cycle's last sweep) the thread also adds the group's four final values
-// to Psi in FP64: the other colour's are final before this sweep and its own
-// after it.
-template <bool FOLD>
-__device__ void smooth0(const Mg32Args &a, int c, long t0, long dt)
+template <bool RES>
+__device__ __forceinline__ void strip0(const Mg0 &z, const Part0 &t, float *U, float *F, int r0, int sa, int sb,
+                                       int c)
 {
-  const int G = (a.cols + 3) >> 2; // column groups per row
-  const long n = (long)(a.hi - a.lo + 1) * G;
-  for (long t = t0; t < n; t += dt) {
-    Cols0 k;
-    cols0_load(a, t, G, k);
-    float fin[4];
-    const unsigned unk = cols0_relax(a, c, k, fin);
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      if ((unk >> q & 1) && ((k.iz + k.c0 + q) & 1) == c)
-        a.u0[k.j + q] = fin[q];
-    if (FOLD)
-#pragma unroll
-      for (int q = 0; q < 4; q++)
-        if (unk >> q & 1)
-          a.Psi[k.j + q] = a.Psi[k.j + q] + (double)fin[q];
+  if (t.j < 0)
+    return;
+  const int P = z.P, H = P >> 1;
+  for (int s = sa + t.g; s < sb; s += t.groups) {
+    const int iz = r0 + s, h = (iz ^ c) & 1; // the colour's columns have parity h
+    float *row = U + s * P;
+    float *x = row + h * H + t.j;
+    const bool top = iz == z.nz - 1 && z.hi == z.nz - 1, bottom = iz == 0 && z.lo == 0;
+    const float4 um = ld4(top ? x - P : x + P), dm = ld4(bottom ? x + P : x - P);
+    const float4 o = ld4(row + (1 - h) * H + t.j), f = ld4(F + s * P + h * H + t.j);
+    float nb[4];
+    if (h) {
+      const float right = row[t.j + 4];
+      nb[0] = z.a * (um.x + dm.x) + t.cO[0] * o.y + t.dO[0] * o.x;
+      nb[1] = z.a * (um.y + dm.y) + t.cO[1] * o.z + t.dO[1] * o.y;
+      nb[2] = z.a * (um.z + dm.z) + t.cO[2] * o.w + t.dO[2] * o.z;
+      nb[3] = z.a * (um.w + dm.w) + t.cO[3] * right + t.dO[3] * o.w;
+    } else {
+      const float left = t.j ? row[H + t.j - 1] : 0.f;
+      nb[0] = z.a * (um.x + dm.x) + t.cE[0] * o.x + t.dE[0] * left;
+      nb[1] = z.a * (um.y + dm.y) + t.cE[1] * o.y + t.dE[1] * o.x;
+      nb[2] = z.a * (um.z + dm.z) + t.cE[2] * o.z + t.dE[2] * o.y;
+      nb[3] = z.a * (um.w + dm.w) + t.cE[3] * o.w + t.dE[3] * o.z;
+    }
+    float4 v;
+    if (RES) {
+      const float4 u = ld4(x);
+      v.x = f.x - nb[0] - (h ? z.e : t.e0) * u.x;
+      v.y = f.y - nb[1] - z.e * u.y;
+      v.z = f.z - nb[2] - z.e * u.z;
+      v.w = f.w - nb[3] - z.e * u.w;
+    } else {
+      v.x = (f.x - nb[0]) * (h ? z.inv_e : t.inv0);
+      v.y = (f.y - nb[1]) * z.inv_e;
+      v.z = (f.z - nb[2]) * z.inv_e;
+      v.w = (f.w - nb[3]) * z.inv_e;
+    }
+    v.x = f.x == f.x ? v.x : 0.f;
+    v.y = f.y == f.y ? v.y : 0.f;
+    v.z = f.z == f.z ? v.z : 0.f;
+    v.w = f.w == f.w ? v.w : 0.f;
+    st4(RES ? F + s * P + h * H + t.j : x, v);
   }
 }
 
-// ---- levels >= 1: nine-point Galerkin operators
-
-__device__ __forceinline__ float nb9(const MgLevel &L, size_t idx, size_t plane)
+// One colour c ((iz+ir)%2 == c) of red-black Gauss-Seidel on rows r0+sa ..
+// r0+sb-1; with RES the residual f - A u of that colour into F instead (0
+// without an equation).  A mesh wider than the CTA takes its columns in strips.
+template <bool RES>
+__device__ __forceinline__ void relax0(const Mg0 &z, Part0 &t, float *U, float *F, int r0, int sa, int sb, int c)
 {
-  const float *u = L.u, *c = L.coef;
-  const long P = L.P;
-  float s = __ldg(c + idx) * *(u + idx - P - 1);
-  s += __ldg(c + plane + idx) * *(u + idx - P);
-  s += __ldg(c + 2 * plane + idx) * *(u + idx - P + 1);
-  s += __ldg(c + 3 * plane + idx) * *(u + idx - 1);
-  s += __ldg(c + 4 * plane + idx) * *(u + idx + 1);
-  s += __ldg(c + 5 * plane + idx) * *(u + idx + P - 1);
-  s += __ldg(c + 6 * plane + idx) * *(u + idx + P);
-  s += __ldg(c + 7 * plane + idx) * *(u + idx + P + 1);
+  const int n = cols0(z);
+  for (int kb = 0;;) {
+    strip0<RES>(z, t, U, F, r0, sa, sb, c);
+    if ((kb += MG_NT) >= n)
+      break;
+    part0(z, t, kb);
+  }
+  if (n > MG_NT)
+    part0(z, t, 0);
+}
+
+// ---- levels >= 1: nine-point Galerkin operators.  A row holds its even
+// columns, then (from Q) its odd ones, each half with a halo column: node J
+// at (J&1) Q + (J>>1) + 1.
+__device__ __forceinline__ int col9(const MgLevel &L, int J) { return (J & 1) * L.Q + (J >> 1) + 1; }
+
+// The coefficients of the node pair (2j, 2j+1) of a row of class v.
+struct Coef9 {
+  float c0[8], c1[8];
+};
+
+__device__ __forceinline__ const float *load_coef9(const MgLevel &L, int v, int j, Coef9 &c)
+{
+  int P = L.P; // opaque here: else the offsets are kept in registers all along
+  asm volatile("" : "+r"(P));
+  const float *p = L.coef + (size_t)v * (MG_NCOEF * P) + 1 + j;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    c.c0[k] = __ldg(p + k * P);
+    c.c1[k] = __ldg(p + k * P + (P >> 1));
+  }
+  return p;
+}
+
+// The neighbours' terms at the pair's node of parity CR (0 even, 1 odd); u: its row
+template <int CR> __device__ __forceinline__ float nb9(const MgLevel &L, int j, const Coef9 &k, const float *u)
+{
+  const int P = L.P, at = (CR ? L.Q + 1 : 1) + j, lf = (CR ? 1 : L.Q) + j;
+  const float *c = CR ? k.c1 : k.c0;
+  float s = c[0] * u[lf - P];
+  s += c[1] * u[at - P];
+  s += c[2] * u[lf + 1 - P];
+  s += c[3] * u[lf];
+  s += c[4] * u[lf + 1];
+  s += c[5] * u[lf + P];
+  s += c[6] * u[at + P];
+  s += c[7] * u[lf + 1 + P];
   return s;
 }
 
-__device__ __forceinline__ float res9(const MgLevel &L, int I, int J)
+// The bilinear correction from level C (row -1 at w) at the pair (i, 2j),
+// (i, 2j+1) of the level above (linear along a direction C does not coarsen:
+// the node itself).
+template <bool CG>
+__device__ __forceinline__ void interp(const MgLevel &C, const float *w, int i, int j, float &even, float &odd)
 {
-  const size_t plane = (size_t)(L.Z + 2) * L.P, idx = (size_t)(I + 1) * L.P + J + 1;
-  if (__ldg(L.coef + MG_INVD * plane + idx) == 0.f)
-    return 0.f;
-  return *(L.f + idx) - __ldg(L.coef + MG_DIAG * plane + idx) * (*(L.u + idx) + nb9(L, idx, plane));
-}
-
-// one colour (cz, cr) = (c >> 1, c & 1) of Gauss-Seidel on a nine-point level
-__device__ void smooth9(const MgLevel &L, int c, long t0, long dt)
-{
-  const int cz = c >> 1, cr = c & 1;
-  const int Zh = (L.Z - cz + 1) >> 1, Rh = (L.R - cr + 1) >> 1;
-  const long n = (long)Zh * Rh;
-  const size_t plane = (size_t)(L.Z + 2) * L.P;
-  for (long t = t0; t < n; t += dt) {
-    const int q = (int)(t / Rh);
-    const int I = 2 * q + cz, J = 2 * (int)(t - (long)q * Rh) + cr;
-    const size_t idx = (size_t)(I + 1) * L.P + J + 1;
-    const float id = __ldg(L.coef + MG_INVD * plane + idx);
-    if (id == 0.f)
-      continue;
-    L.u[idx] = *(L.f + idx) * id - nb9(L, idx, plane);
-  }
-}
-
-// Two colours (cz, cr) then (cz, 1-cr) of Gauss-Seidel on a nine-point level
-// over this CTA's rows (a band of ceil(Z / grid) rows).  A node of colour
-// (cz, 1-cr) reads the just-updated colour (cz, cr) only at its left and
-// right neighbours, in its own row, so a CTA barrier between the two
-// colours suffices; the colours of the other row parity read rows I +- 1
-// and follow a grid barrier.  The update order, and so every value, is the
-// four-colour sweep's.
-__device__ void smooth9_rows(const MgLevel &L, int cz, int cr)
-{
-  const int nbl = (L.Z + (int)gridDim.x - 1) / (int)gridDim.x;
-  const int I0 = (int)blockIdx.x * nbl, I1 = min(I0 + nbl, L.Z);
-  const int r0 = I0 + ((I0 & 1) != cz); // first own row of parity cz
-  const int nrows = r0 < I1 ? (I1 - r0 + 1) >> 1 : 0;
-  const size_t plane = (size_t)(L.Z + 2) * L.P;
-  for (int h = 0; h < 2; h++) {
-    const int c = h ? 1 - cr : cr;
-    const int Rh = (L.R - c + 1) >> 1;
-    const long n = (long)nrows * Rh;
-    for (long t = threadIdx.x; t < n; t += blockDim.x) {
-      const int q = (int)(t / Rh);
-      const int I = r0 + 2 * q, J = 2 * (int)(t - (long)q * Rh) + c;
-      const size_t idx = (size_t)(I + 1) * L.P + J + 1;
-      const float id = __ldg(L.coef + MG_INVD * plane + idx);
-      if (id == 0.f)
-        continue;
-      L.u[idx] = *(L.f + idx) * id - nb9(L, idx, plane);
-    }
-    __syncthreads();
-  }
-}
-
-// f of level C from the residual of level 0 (C = lev[1]), u of C cleared.
-// Level 0's last colour (1) has a zero residual: only (iz+ir) even nodes.
-__device__ void restrict0(const Mg32Args &a, long t0, long dt)
-{
-  const MgLevel &C = a.lev[1];
-  const long n = (long)C.Z * C.R;
-  const size_t plane = (size_t)(C.Z + 2) * C.P;
-  for (long t = t0; t < n; t += dt) {
-    const int I = (int)(t / C.R), J = (int)(t - (long)I * C.R);
-    const size_t idx = (size_t)(I + 1) * C.P + J + 1;
-    float s = 0.f;
-    if (__ldg(C.coef + MG_INVD * plane + idx) != 0.f && (C.cz != 2 || C.cr != 2)) {
-      // semi-coarsened: the three fine nodes along the coarsened direction
-      const float w[3] = {__ldg(C.rw + 3 * J), __ldg(C.rw + 3 * J + 1), __ldg(C.rw + 3 * J + 2)};
-      const int iz = C.cz * I, ir = C.cr * J;
-#pragma unroll
-      for (int d = -1; d <= 1; d++) {
-        const int z = C.cz == 2 ? iz + d : iz, r = C.cr == 2 ? ir + d : ir;
-        if (z < 0 || z > a.nz || r < 0)
-          continue;
-        s += (C.cz == 2 ? (d ? 0.5f : 1.f) * w[1] : w[d + 1]) * res0(a, z, r);
-      }
-    } else if (__ldg(C.coef + MG_INVD * plane + idx) != 0.f) {
-      const float w0 = __ldg(C.rw + 3 * J), w1 = __ldg(C.rw + 3 * J + 1), w2 = __ldg(C.rw + 3 * J + 2);
-      const int iz = 2 * I, ir = 2 * J;
-      s = w1 * res0(a, iz, ir);
-      if (iz > 0) {
-        if (ir > 0)
-          s += 0.5f * w0 * res0(a, iz - 1, ir - 1);
-        s += 0.5f * w2 * res0(a, iz - 1, ir + 1);
-      }
-      if (iz < a.nz) {
-        if (ir > 0)
-          s += 0.5f * w0 * res0(a, iz + 1, ir - 1);
-        s += 0.5f * w2 * res0(a, iz + 1, ir + 1);
-      }
-    }
-    C.f[idx] = s;
-    C.u[idx] = 0.f;
-  }
-}
-
-// f of level C = lev[l+1] from the residual of F = lev[l], u of C cleared.
-// F's last colour (3: odd, odd) has a zero residual: its four diagonal
-// neighbours of (2I, 2J) are skipped.
-__device__ void restrict9(const MgLevel &F, const MgLevel &C, long t0, long dt)
-{
-  const long n = (long)C.Z * C.R;
-  const size_t plane = (size_t)(C.Z + 2) * C.P;
-  for (long t = t0; t < n; t += dt) {
-    const int I = (int)(t / C.R), J = (int)(t - (long)I * C.R);
-    const size_t idx = (size_t)(I + 1) * C.P + J + 1;
-    float s = 0.f;
-    if (__ldg(C.coef + MG_INVD * plane + idx) != 0.f && (C.cz != 2 || C.cr != 2)) {
-      // semi-coarsened: the three fine nodes along the coarsened direction
-      const float w[3] = {__ldg(C.rw + 3 * J), __ldg(C.rw + 3 * J + 1), __ldg(C.rw + 3 * J + 2)};
-      const int i = C.cz * I, j = C.cr * J;
-#pragma unroll
-      for (int d = -1; d <= 1; d++) {
-        const int z = C.cz == 2 ? i + d : i, r = C.cr == 2 ? j + d : j;
-        if (z < 0 || z >= F.Z || r < 0 || r >= F.R)
-          continue;
-        s += (C.cz == 2 ? (d ? 0.5f : 1.f) * w[1] : w[d + 1]) * res9(F, z, r);
-      }
-    } else if (__ldg(C.coef + MG_INVD * plane + idx) != 0.f) {
-      const float w0 = __ldg(C.rw + 3 * J), w1 = __ldg(C.rw + 3 * J + 1), w2 = __ldg(C.rw + 3 * J + 2);
-      const int i = 2 * I, j = 2 * J;
-      s = w1 * res9(F, i, j);
-      if (j > 0)
-        s += w0 * res9(F, i, j - 1);
-      if (j + 1 < F.R)
-        s += w2 * res9(F, i, j + 1);
-      if (i > 0)
-        s += 0.5f * w1 * res9(F, i - 1, j);
-      if (i + 1 < F.Z)
-        s += 0.5f * w1 * res9(F, i + 1, j);
-    }
-    C.f[idx] = s;
-    C.u[idx] = 0.f;
-  }
-}
-
-// bilinear correction from level C at node (i, j) of the level above
-// (linear along a direction C does not coarsen: the node itself)
-__device__ __forceinline__ float interp(const MgLevel &C, int i, int j)
-{
-  const bool hz = C.cz == 2 && (i & 1), hr = C.cr == 2 && (j & 1); // half-way nodes
-  const int I = C.cz == 2 ? i >> 1 : i, J = C.cr == 2 ? j >> 1 : j;
-  const float *u = C.u + (size_t)(I + 1) * C.P + J + 1;
-  float v;
-  if (hr)
-    v = 0.5f * (*(u) + *(u + 1));
-  else
-    v = *(u);
+  auto at = [&](const float *p) { return CG ? __ldcg(p) : *p; };
+  const bool hz = C.cz == 2 && (i & 1); // a half-way row
+  const float *p = w + (size_t)((C.cz == 2 ? i >> 1 : i) + 1) * C.P;
+  const int k0 = C.cr == 2 ? col9(C, j) : 1 + j, k1 = C.cr == 2 ? col9(C, j + 1) : C.Q + 1 + j;
+  const float x = at(p + k0), y = at(p + k1);
+  even = x;
+  odd = C.cr == 2 ? 0.5f * (x + y) : y;
   if (hz) {
-    const float *w = u + C.P;
-    v = 0.5f * v + 0.5f * (hr ? 0.5f * (*(w) + *(w + 1)) : *(w));
-  }
-  return v;
-}
-
-__device__ void prolong0(const Mg32Args &a, long t0, long dt)
-{
-  const MgLevel &C = a.lev[1];
-  const long n = (long)(a.hi - a.lo + 1) * a.cols;
-  for (long t = t0; t < n; t += dt) {
-    const int row = (int)(t / a.cols), ir = (int)(t - (long)row * a.cols), iz = a.lo + row;
-    const size_t j = node(iz, ir, a.P0);
-    if (a.umask[j] & S32_U_METAL)
-      continue;
-    a.u0[j] = *(a.u0 + j) + interp(C, iz, ir);
+    const float x2 = at(p + C.P + k0), y2 = at(p + C.P + k1);
+    even = 0.5f * even + 0.5f * x2;
+    odd = 0.5f * odd + 0.5f * (C.cr == 2 ? 0.5f * (x2 + y2) : y2);
   }
 }
 
-__device__ void prolong9(const MgLevel &F, const MgLevel &C, long t0, long dt)
-{
-  const long n = (long)F.Z * F.R;
-  const size_t plane = (size_t)(F.Z + 2) * F.P;
-  for (long t = t0; t < n; t += dt) {
-    const int i = (int)(t / F.R), j = (int)(t - (long)i * F.R);
-    const size_t idx = (size_t)(i + 1) * F.P + j + 1;
-    if (__ldg(F.coef + MG_INVD * plane + idx) == 0.f)
-      continue;
-    F.u[idx] = *(F.u + idx) + interp(C, i, j);
-  }
-}
+// A thread's share of the rows rlo <= I < rhi of a nine-point level in a
+// buffer whose first row is r0.  The coefficients of a held node are all 0,
+// so its u comes out 0.
+//
+// Fix9: up to K node pairs of the even rows and K of the odd ones, with their
+// coefficients and f/diagonal in registers for the whole visit.  For the
+// levels and bands with at most K MG_NT pairs of a row parity, where a colour
+// step is a chain of latencies: shared-memory loads, eight fused
+// multiply-adds, a barrier.
+template <int K> struct Fix9 {
+  int at[2][K], row[2][K], j[2][K]; // place of the row; row (INT_MIN: none)
+  Coef9 c[2][K];
+  float g0[2][K], g1[2][K]; // f/diagonal
+  unsigned unk;             // bits 2 (K parity + k), +1: the pair's even and odd nodes are unknowns
 
-__shared__ float mg_coarse_f[MG_MAX_DIRECT]; // the coarsest level's f, gathered for its exact solve
-
-// Levels l0 .. nlev-1 below a restriction into l0, by CTA 0 alone with CTA
-// barriers: descent, the coarsest level's solve, ascent back to l0.
-__device__ void sub_cycle(const Mg32Args &a, int l0)
-{
-  const MgLevel *lv = a.lev;
-  const long t0 = threadIdx.x, dt = blockDim.x;
-  const int L = a.nlev;
-  for (int l = l0; l < L - 1; l++) {
-    for (int k = 0; k < a.nu; k++)
-      for (int c = 0; c < 4; c++) {
-        smooth9(lv[l], c, t0, dt);
-        __syncthreads();
+  __device__ __forceinline__ void init(const MgLevel &L, const float *F, int r0, int rlo, int rhi)
+  {
+    const int n = (L.R + 1) >> 1;
+    rlo = max(rlo, 0);
+    rhi = min(rhi, L.Z);
+    unk = 0;
+#pragma unroll
+    for (int z = 0; z < 2; z++)
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const int t = threadIdx.x + k * MG_NT, q = (unsigned)t / (unsigned)n, I = rlo + ((rlo ^ z) & 1) + 2 * q;
+        row[z][k] = INT_MIN;
+        if (I < rhi) {
+          row[z][k] = I;
+          j[z][k] = t - q * n;
+          at[z][k] = (I - r0) * L.P;
+          const float *p = load_coef9(L, __ldg(L.cls + I), j[z][k], c[z][k]);
+          const float i0 = __ldg(p + MG_INVD * L.P), i1 = __ldg(p + MG_INVD * L.P + L.Q);
+          g0[z][k] = i0 * F[at[z][k] + 1 + j[z][k]];
+          g1[z][k] = i1 * F[at[z][k] + L.Q + 1 + j[z][k]];
+          unk |= (i0 != 0.f ? 1u : 0u) << (2 * (K * z + k)) | (i1 != 0.f ? 2u : 0u) << (2 * (K * z + k));
+        }
       }
-    restrict9(lv[l], lv[l + 1], t0, dt);
-    __syncthreads();
   }
-  if (a.cinv) {
-    // the coarsest level solved exactly: u = A^-1 f over its unknowns
-    float *fc = mg_coarse_f;
-    const MgLevel &C = lv[L - 1];
-    for (int i = (int)t0; i < a.cn; i += (int)dt)
-      fc[i] = C.f[a.cidx[i]];
-    __syncthreads();
-    // a warp per row: coalesced reads of the row, the lanes' partial sums
-    // added by shuffles
-    const int lane = (int)t0 & 31, warp = (int)t0 >> 5, nwarps = (int)dt >> 5;
-    for (int i = warp; i < a.cn; i += nwarps) {
-      const float *row = a.cinv + (size_t)i * a.cn;
-      float acc = 0.f;
-      for (int k = lane; k < a.cn; k += 32)
-        acc += __ldg(row + k) * fc[k];
-      for (int o = 16; o > 0; o >>= 1)
-        acc += __shfl_down_sync(0xffffffffu, acc, o);
-      if (lane == 0)
-        C.u[a.cidx[i]] = acc;
+  template <int CZ, int CR>
+  __device__ __forceinline__ void colour(const MgLevel &L, float *U, const float *, int, int ra, int rb)
+  {
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (row[CZ][k] >= ra && row[CZ][k] < rb) {
+        float *u = U + at[CZ][k];
+        u[(CR ? L.Q + 1 : 1) + j[CZ][k]] = (CR ? g1[CZ][k] : g0[CZ][k]) - nb9<CR>(L, j[CZ][k], c[CZ][k], u);
+      }
+  }
+  __device__ __forceinline__ void resid(const MgLevel &L, const float *U, const float *, float *R, int, int ra, int rb)
+  {
+#pragma unroll
+    for (int z = 0; z < 2; z++)
+#pragma unroll
+      for (int k = 0; k < K; k++)
+        if (row[z][k] >= ra && row[z][k] < rb) {
+          const float *u = U + at[z][k];
+          const float *d = L.coef + (size_t)(__ldg(L.cls + row[z][k]) * MG_NCOEF + MG_DIAG) * L.P;
+          const int a0 = 1 + j[z][k], a1 = L.Q + 1 + j[z][k];
+          const float e = __ldg(d + a0) * (g0[z][k] - nb9<0>(L, j[z][k], c[z][k], u) - u[a0]);
+          const float o = __ldg(d + a1) * (g1[z][k] - nb9<1>(L, j[z][k], c[z][k], u) - u[a1]);
+          R[at[z][k] + a0] = e;
+          R[at[z][k] + a1] = o;
+        }
+  }
+  template <bool CG>
+  __device__ __forceinline__ void prolong(const MgLevel &L, const MgLevel &C, float *U, const float *w, int)
+  {
+#pragma unroll
+    for (int z = 0; z < 2; z++)
+#pragma unroll
+      for (int k = 0; k < K; k++)
+        if (row[z][k] != INT_MIN) {
+          float e, o;
+          interp<CG>(C, w, row[z][k], j[z][k], e, o);
+          float *u = U + at[z][k] + 1 + j[z][k];
+          if (unk >> (2 * (K * z + k)) & 1)
+            u[0] += e;
+          if (unk >> (2 * (K * z + k)) & 2)
+            u[L.Q] += o;
+        }
+  }
+};
+
+// Run9: one pair of columns in a run of rows, MG_ROWS of a parity at a time
+// (their loads overlap); the coefficients of a class in registers, loaded
+// again where a run's classes differ (at metal edges).  A level wider than
+// the CTA takes its columns in strips.
+constexpr int MG_ROWS = 3;
+struct Run9 {
+  int j, lo, hi, W, n, v; // columns 2j, 2j+1 (j < 0: none); rows; lanes a row group; pairs a row; class
+  Coef9 c;
+  float i0, i1;
+
+  __device__ __forceinline__ void strip(int jb)
+  {
+    const int k = W < MG_NT ? (int)threadIdx.x % W : jb + (int)threadIdx.x;
+    j = k < n ? k : -1;
+    v = -1;
+  }
+  __device__ __forceinline__ void init(const MgLevel &L, const float *, int, int rlo, int rhi)
+  {
+    n = (L.R + 1) >> 1;
+    W = (n + 31) & ~31;
+    rlo = max(rlo, 0);
+    rhi = min(rhi, L.Z);
+    const int groups = W < MG_NT ? MG_NT / W : 1, g = W < MG_NT ? (int)threadIdx.x / W : 0;
+    const int per = (rhi - rlo + groups - 1) / groups;
+    lo = rlo + g * per;
+    hi = g < groups ? min(lo + per, rhi) : lo;
+    strip(0);
+  }
+  __device__ __forceinline__ void load(const MgLevel &L, int cls)
+  {
+    if (cls == v)
+      return;
+    v = cls;
+    const float *p = load_coef9(L, cls, j, c);
+    i0 = __ldg(p + MG_INVD * L.P);
+    i1 = __ldg(p + MG_INVD * L.P + L.Q);
+  }
+  template <class Fn> __device__ __forceinline__ void strips(Fn fn)
+  {
+    for (int jb = 0;;) {
+      if (j >= 0)
+        fn();
+      if ((jb += MG_NT) >= n)
+        break;
+      strip(jb);
     }
-    __syncthreads();
-  } else {
-    for (int k = 0; k < a.coarse_sweeps; k++)
-      for (int c = 0; c < 4; c++) {
-        smooth9(lv[L - 1], c, t0, dt);
-        __syncthreads();
-      }
+    if (n > MG_NT)
+      strip(0);
   }
-  for (int l = L - 2; l >= l0; l--) {
-    prolong9(lv[l], lv[l + 1], t0, dt);
-    __syncthreads();
-    for (int k = 0; k < a.nu; k++)
-      for (int c = 3; c >= 0; c--) {
-        smooth9(lv[l], c, t0, dt);
-        __syncthreads();
+  template <int CZ, int CR>
+  __device__ __forceinline__ void colour(const MgLevel &L, float *U, const float *F, int r0, int ra, int rb)
+  {
+    strips([&]() {
+      const int a = max(lo, ra), b = min(hi, rb), at = (CR ? L.Q + 1 : 1) + j;
+#pragma unroll 1
+      for (int I = a + ((a ^ CZ) & 1); I < b; I += 2 * MG_ROWS) {
+        int cl[MG_ROWS];
+#pragma unroll
+        for (int k = 0; k < MG_ROWS; k++)
+          cl[k] = __ldg(L.cls + min(I + 2 * k, b - 1));
+        bool same = true;
+#pragma unroll
+        for (int k = 1; k < MG_ROWS; k++)
+          same = same && (I + 2 * k >= b || cl[k] == cl[0]);
+        float *u = U + (I - r0) * L.P;
+        const float *f = F + (I - r0) * L.P + at;
+        if (same && I + 2 * (MG_ROWS - 1) < b) {
+          load(L, cl[0]);
+          float x[MG_ROWS];
+#pragma unroll
+          for (int k = 0; k < MG_ROWS; k++)
+            x[k] = f[2 * k * L.P] * (CR ? i1 : i0) - nb9<CR>(L, j, c, u + 2 * k * L.P);
+#pragma unroll
+          for (int k = 0; k < MG_ROWS; k++)
+            u[2 * k * L.P + at] = x[k];
+        } else {
+#pragma unroll 1
+          for (int k = 0; k < MG_ROWS && I + 2 * k < b; k++) {
+            load(L, __ldg(L.cls + I + 2 * k));
+            u[2 * k * L.P + at] = f[2 * k * L.P] * (CR ? i1 : i0) - nb9<CR>(L, j, c, u + 2 * k * L.P);
+          }
+        }
       }
+    });
   }
+  __device__ __forceinline__ void resid(const MgLevel &L, const float *U, const float *F, float *R, int r0, int ra,
+                                        int rb)
+  {
+    strips([&]() {
+      const int a0 = 1 + j, a1 = L.Q + 1 + j;
+#pragma unroll 1
+      for (int I = max(lo, ra); I < min(hi, rb); I++) {
+        load(L, __ldg(L.cls + I));
+        const float *u = U + (I - r0) * L.P, *f = F + (I - r0) * L.P;
+        const float *d = L.coef + (size_t)(v * MG_NCOEF + MG_DIAG) * L.P;
+        const float e = __ldg(d + a0) * (f[a0] * i0 - nb9<0>(L, j, c, u) - u[a0]);
+        const float o = __ldg(d + a1) * (f[a1] * i1 - nb9<1>(L, j, c, u) - u[a1]);
+        R[(I - r0) * L.P + a0] = e;
+        R[(I - r0) * L.P + a1] = o;
+      }
+    });
+  }
+  template <bool CG>
+  __device__ __forceinline__ void prolong(const MgLevel &L, const MgLevel &C, float *U, const float *w, int r0)
+  {
+    strips([&]() {
+#pragma unroll 1
+      for (int I = lo; I < hi; I += 4) {
+        float e[4], o[4];
+        int cl[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          cl[k] = __ldg(L.cls + min(I + k, hi - 1));
+          interp<CG>(C, w, min(I + k, hi - 1), j, e[k], o[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (I + k < hi) {
+            load(L, cl[k]);
+            float *u = U + (I + k - r0) * L.P + 1 + j;
+            if (i0 != 0.f)
+              u[0] += e[k];
+            if (i1 != 0.f)
+              u[L.Q] += o[k];
+          }
+      }
+    });
+  }
+};
+
+// Both colours of row parity CZ on rows ra <= I < rb, column parity CR
+// first: the second reads the first only in its own row, so a CTA barrier
+// lies between them.
+template <int CZ, int CR, class Op>
+__device__ __forceinline__ void rows9(const MgLevel &L, Op &t, float *U, const float *F, int r0, int ra, int rb)
+{
+  t.template colour<CZ, CR>(L, U, F, r0, ra, rb);
+  __syncthreads();
+  t.template colour<CZ, 1 - CR>(L, U, F, r0, ra, rb);
+  __syncthreads();
 }
 
-// One V-cycle on (u0, f0), u0 = 0 on entry.
-__device__ bool vcycle(const Mg32Args &a, unsigned &gen, DevCounts *cnt)
+// f of level C's rows Ia .. Ib-1 from the residual R (a buffer whose first
+// row is r0) of the level L above, into rows of pitch C.P from `out` on (row
+// -1 first); a thread keeps a column.  Halo rows and columns of R are 0.
+__device__ __forceinline__ void restrict9(const MgLevel &L, const MgLevel &C, const float *R, int r0, int Ia, int Ib,
+                                          float *out)
 {
-  const long gt0 = (long)blockIdx.x * blockDim.x + threadIdx.x, gdt = (long)gridDim.x * blockDim.x;
-  const int T = a.tail; // 1 <= T <= nlev - 1
-  // the first colour-0 sweep from u0 = 0 was made by residual64
-  for (int k = 0; k < a.nu0; k++)
-    for (int c = k ? 0 : 1; c < 2; c++) {
-      smooth0<false>(a, c, gt0, gdt);
-      if (!mg_grid_sync(a, gen, cnt))
-        return false;
+  const int W = (C.R + 31) & ~31, groups = W < MG_NT ? MG_NT / W : 1, g = W < MG_NT ? threadIdx.x / W : 0, P = L.P;
+  if (g >= groups)
+    return;
+  for (int J = threadIdx.x - g * W; J < C.R; J += MG_NT) {
+    const int k = col9(C, J), j = C.cr * J, at = col9(L, j), l = col9(L, j - 1), r = col9(L, j + 1);
+    const float w0 = C.cr == 2 ? __ldg(C.rw + 3 * J) : 0.f, w1 = __ldg(C.rw + 3 * J + 1);
+    const float w2 = C.cr == 2 ? __ldg(C.rw + 3 * J + 2) : 0.f, wz = C.cz == 2 ? 0.5f * w1 : 0.f;
+#pragma unroll 1
+    for (int I = Ia + g; I < Ib; I += groups) {
+      const float *x = R + (C.cz * I - r0) * P;
+      float v = w1 * x[at];
+      if (C.cr == 2)
+        v += w0 * x[l] + w2 * x[r];
+      if (C.cz == 2)
+        v += wz * x[at - P] + wz * x[at + P];
+      out[(I + 1) * C.P + k] = v;
     }
-  restrict0(a, gt0, gdt);
-  if (!mg_grid_sync(a, gen, cnt))
-    return false;
-  // grid-wide nine-point levels 1 .. T-1
-  for (int l = 1; l < T; l++) {
-    for (int k = 0; k < a.nu; k++)
-      for (int cz = 0; cz < 2; cz++) { // colours (cz, 0), (cz, 1)
-        smooth9_rows(a.lev[l], cz, 0);
-        if (!mg_grid_sync(a, gen, cnt))
-          return false;
+  }
+}
+
+// The same from level 0's residual in a band buffer.  Level 0's last colour
+// (1) has a zero residual, so only its (iz+ir) even nodes count.
+__device__ __forceinline__ void restrict0(const MgLevel &C, int P, const float *R, int r0, int Ia, int Ib, float *out)
+{
+  const int W = (C.R + 31) & ~31, groups = W < MG_NT ? MG_NT / W : 1, g = W < MG_NT ? threadIdx.x / W : 0, H = P >> 1;
+  if (g >= groups)
+    return;
+  for (int J = threadIdx.x - g * W; J < C.R; J += MG_NT) {
+    const int k = col9(C, J);
+    const float w0 = J ? __ldg(C.rw + 3 * J) : 0.f, w1 = __ldg(C.rw + 3 * J + 1), w2 = __ldg(C.rw + 3 * J + 2);
+    const int in = J ? 1 : 0; // the inner neighbour (none on the axis)
+#pragma unroll 1
+    for (int I = Ia + g; I < Ib; I += groups) {
+      const float *x = R + (C.cz * I - r0) * P;
+      float v;
+      if (C.cz == 2 && C.cr == 2) { // row 2I, column 2J; rows 2I +- 1, columns 2J -+ 1
+        const float *y = x + H + J;
+        v = w1 * x[J] + 0.5f * w2 * (y[-P] + y[P]) + 0.5f * w0 * (y[-P - in] + y[P - in]);
+      } else if (C.cz == 2) { // coarsened in z only: the column has the colour in every other row
+        const int at = (J & 1) * H + (J >> 1);
+        v = (J & 1) == 0 ? w1 * x[at] : 0.5f * w1 * (x[at - P] + x[at + P]);
+      } else { // in r only: column 2J in even rows, 2J -+ 1 in odd ones
+        const float *y = x + H + J;
+        v = (I & 1) == 0 ? w1 * x[J] : w2 * y[0] + w0 * y[-in];
       }
-    restrict9(a.lev[l], a.lev[l + 1], gt0, gdt);
-    if (!mg_grid_sync(a, gen, cnt))
-      return false;
-  }
-  // levels T .. nlev-1 by CTA 0 while the others wait
-  if (blockIdx.x == 0)
-    sub_cycle(a, T);
-  if (!mg_grid_sync(a, gen, cnt))
-    return false;
-  for (int l = T - 1; l >= 1; l--) {
-    prolong9(a.lev[l], a.lev[l + 1], gt0, gdt);
-    if (!mg_grid_sync(a, gen, cnt))
-      return false;
-    for (int k = 0; k < a.nu; k++)
-      for (int cz = 1; cz >= 0; cz--) { // colours (cz, 1), (cz, 0)
-        smooth9_rows(a.lev[l], cz, 1);
-        if (!mg_grid_sync(a, gen, cnt))
-          return false;
-      }
-  }
-  prolong0(a, gt0, gdt);
-  if (!mg_grid_sync(a, gen, cnt))
-    return false;
-  for (int k = 0; k < a.nu0; k++)
-    for (int c = 1; c >= 0; c--) {
-      if (k == a.nu0 - 1 && c == 0)
-        smooth0<true>(a, c, gt0, gdt); // Psi += u0 on the way
-      else
-        smooth0<false>(a, c, gt0, gdt);
-      if (!mg_grid_sync(a, gen, cnt))
-        return false;
+      // (NaN: R of columns without equations, which only held nodes reach)
+      out[(I + 1) * C.P + k] = v == v ? v : 0.f;
     }
-  return true;
-}
-
-// r = rhs - A Psi in FP64 over the unknown nodes into f0 (rounded), and u0
-// as the first colour-0 Gauss-Seidel sweep from u0 = 0 leaves it: f0 / e at
-// (iz+ir) even nodes (their neighbour sum is zero), 0 at the others; this
-// thread's sum |r| and, with first, sum |rhs| over iz < nz, ir < nr-1.
-__device__ void residual64(const Mg32Args &a, bool first, double *rs, double *ds)
-{
-  const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x, dt = (long)gridDim.x * blockDim.x;
-  const long n = (long)a.nz * a.cols, P = a.P0;
-  double r_acc = 0, d_acc = 0;
-  for (long t = t0; t < n; t += dt) {
-    const int iz = (int)(t / a.cols), ir = (int)(t - (long)iz * a.cols);
-    const size_t j = node(iz, ir, a.P0);
-    const double rh = a.rhs ? a.rhs[j] : 0.0;
-    if (first)
-      d_acc += fabs(rh);
-    if (!unknown0(a, iz, ir, j))
-      continue;
-    const double up = (iz == a.nz - 1 && a.hi == a.nz - 1) ? *(a.Psi + j - P) : *(a.Psi + j + P);
-    const double dn = (iz == 0 && a.lo == 0) ? *(a.Psi + j + P) : *(a.Psi + j - P);
-    const double psi = *(a.Psi + j);
-    double ap;
-    if (ir == 0)
-      ap = a.a_d * (up + dn) + a.c4_d * *(a.Psi + j + 1) + a.e2c_d * psi;
-    else {
-      const double h = 0.5 / ir;
-      ap = a.a_d * (up + dn) + a.dr2_inv * (1 + h) * *(a.Psi + j + 1) +
-           a.dr2_inv * (1 - h) * *(a.Psi + j - 1) + a.e_d * psi;
-    }
-    const double r = rh - ap;
-    r_acc += fabs(r);
-    const float rf = (float)r;
-    a.f0[j] = rf;
-    a.u0[j] = (a.nu0 && !((iz + ir) & 1)) ? rf * (ir ? a.inv_e : a.inv_e2c) : 0.f;
-  }
-  *rs = r_acc;
-  *ds = d_acc;
-}
-
-__device__ void fold(const Mg32Args &a)
-{
-  const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x, dt = (long)gridDim.x * blockDim.x;
-  const long n = (long)a.nz * a.cols;
-  for (long t = t0; t < n; t += dt) {
-    const int iz = (int)(t / a.cols), ir = (int)(t - (long)iz * a.cols);
-    const size_t j = node(iz, ir, a.P0);
-    if (unknown0(a, iz, ir, j))
-      a.Psi[j] = *(a.Psi + j) + (double)*(a.u0 + j);
   }
 }
 
-// CTA sums of two doubles into part[blockIdx][0..1] (fixed order)
-__device__ void block_sums(const Mg32Args &a, double x, double y)
+// ---- the kernels of a V-cycle
+
+__global__ void k_mg_begin(MgCall c, MgCall *call)
 {
-  __shared__ double sh[2][MG_NT / 32];
+  c.skip = c.st && !c.st->do_solve;
+  *call = c;
+}
+
+// CTA sums of two doubles in a fixed order; thread 0 has them
+__device__ __forceinline__ double2 block_sums(double x, double y)
+{
+  __shared__ double sh[2][MG_W];
   for (int o = 16; o > 0; o >>= 1) {
     x += __shfl_down_sync(0xffffffffu, x, o);
     y += __shfl_down_sync(0xffffffffu, y, o);
@@ -630,89 +587,439 @@ __device__ void block_sums(const Mg32Args &a, double x, double y)
     sh[1][w] = y;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double sx = 0, sy = 0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); k++) {
-      sx += sh[0][k];
-      sy += sh[1][k];
+  double2 s = make_double2(0, 0);
+  if (threadIdx.x == 0)
+    for (int k = 0; k < MG_W; k++) {
+      s.x += sh[0][k];
+      s.y += sh[1][k];
     }
-    a.part[2 * blockIdx.x] = sx;
-    a.part[2 * blockIdx.x + 1] = sy;
+  return s;
+}
+
+// Level 0, the residual of the rows a0 .. b0-1 of a band and of MG_DOWN halo
+// rows a side (the neighbours' values, formed again here): r = rhs - A Psi in
+// FP64, f = r in FP32 and u as the first colour-0 sweep from u = 0 leaves it
+// (f/e: the neighbour sum is zero).  Returns this thread's sum |r| and sum
+// |rhs| over the own rows (iz < nz, ir < nr-1).  A thread forms the columns
+// 2j, 2j+1 and walks down a run of rows, so each Psi is read once, with the
+// loads of MG_AHEAD rows in flight together.
+constexpr int MG_AHEAD = 4;
+__device__ __forceinline__ double2 resid0(const Mg0 &z, const double *Psi, const double *rhs, const uint8_t *umask,
+                                          float *U, float *F, int a0, int b0)
+{
+  const int P = z.P, H = P >> 1, lane = threadIdx.x & 31, r0 = a0 - MG_DOWN, n = b0 - a0 + 2 * MG_DOWN;
+  double r_acc = 0, d_acc = 0;
+  const float nan = __int_as_float(0x7fc00000);
+  const int W = min((H + 31) & ~31, MG_NT), groups = MG_NT / W, g = threadIdx.x / W;
+  if (g < groups) {
+    const int per = (n + groups - 1) / groups, s0 = g * per, s1 = min(s0 + per, n);
+    for (int jl = threadIdx.x - g * W; jl - lane < H; jl += W) {
+      const int j = min(jl, H - 1), c0 = 2 * j;
+      const double2 cp = __ldg(reinterpret_cast<const double2 *>(z.cpd + c0));
+      const double2 cm = __ldg(reinterpret_cast<const double2 *>(z.cmd + c0));
+      const double e0 = c0 ? z.e_d : z.e2c_d;
+      const bool edge = lane == 0 || lane == 31; // lanes whose outer neighbour column is another warp's
+      const int beside = lane ? (c0 + 2 < P ? 2 : 0) : (c0 ? -1 : 0);
+      const bool le = c0 < z.cols, lo = c0 + 1 < z.cols;
+      auto row = [&](int s) { return min(max(r0 + s, 0), z.nz) * P + c0; }; // fewer than 2^31 nodes
+      auto psi = [&](int s) { return __ldcg(reinterpret_cast<const double2 *>(Psi + row(s))); };
+      double2 below = psi(s0 - 1), here = psi(s0);
+#pragma unroll 1
+      for (int sb = s0; sb < s1; sb += MG_AHEAD) {
+        double2 nx[MG_AHEAD], rh[MG_AHEAD];
+        double sd[MG_AHEAD];
+        uchar2 mk[MG_AHEAD];
+#pragma unroll
+        for (int k = 0; k < MG_AHEAD; k++) {
+          const int at = row(sb + k);
+          nx[k] = psi(sb + k + 1);
+          mk[k] = __ldg(reinterpret_cast<const uchar2 *>(umask + at));
+          rh[k] = rhs ? __ldg(reinterpret_cast<const double2 *>(rhs + at)) : make_double2(0, 0);
+          sd[k] = edge ? __ldcg(Psi + at + beside) : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < MG_AHEAD; k++) {
+          const int s = sb + k, iz = r0 + s;
+          double left = __shfl_up_sync(0xffffffffu, here.y, 1), right = __shfl_down_sync(0xffffffffu, here.x, 1);
+          left = lane == 0 ? sd[k] : left;
+          right = lane == 31 ? sd[k] : right;
+          const bool own = iz >= a0 && iz < b0 && s < s1, in = iz >= z.lo && iz <= z.hi;
+          const double2 up = iz == z.nz - 1 && z.hi == z.nz - 1 ? below : nx[k], dn = iz == 0 && z.lo == 0 ? nx[k] : below;
+          const double re = rh[k].x - (z.a_d * (up.x + dn.x) + cp.x * here.y + cm.x * left + e0 * here.x);
+          const double ro = rh[k].y - (z.a_d * (up.y + dn.y) + cp.y * right + cm.y * here.x + z.e_d * here.y);
+          const bool ve = in && le && !(mk[k].x & S32_U_METAL), vo = in && lo && !(mk[k].y & S32_U_METAL);
+          if (jl < H && s < s1) {
+            const float fe = ve ? (float)re : nan, fo = vo ? (float)ro : nan;
+            if (own) {
+              r_acc += (ve ? fabs(re) : 0.0) + (vo ? fabs(ro) : 0.0);
+              d_acc += (le ? fabs(rh[k].x) : 0.0) + (lo ? fabs(rh[k].y) : 0.0);
+              z.f[iz * P + j] = fe;
+              z.f[iz * P + H + j] = fo;
+            }
+            F[s * P + j] = fe;
+            F[s * P + H + j] = fo;
+            U[s * P + j] = ve && !(iz & 1) ? fe * (c0 ? z.inv_e : z.inv_e2c) : 0.f;
+            U[s * P + H + j] = vo && (iz & 1) ? fo * z.inv_e : 0.f;
+          }
+          below = here;
+          here = nx[k];
+        }
+      }
+    }
+  }
+  return make_double2(r_acc, d_acc);
+}
+
+// Level 0 down, a band a CTA: the residual; the other three colour sweeps,
+// each on one row less; f of level 1; the band's own rows of u and f to z.u
+// and z.f for the way up.  Psi stays as it is, so the last CTA to finish its
+// sums decides here whether the solve is done: the WHILE node that holds the
+// V-cycle runs on while `more` is set.
+template <bool SM>
+__global__ void __launch_bounds__(MG_NT, 1) k_mg_down0(const __grid_constant__ Mg0 z, const __grid_constant__ MgLevel C,
+                                                       MgCall *call, cudaGraphConditionalHandle more, float *scratch,
+                                                       size_t scratch_n)
+{
+  if (call->skip) {
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+      cudaGraphSetConditional(more, 0);
+    return;
+  }
+  const int P = z.P, a0 = blockIdx.x * z.rp, b0 = min(a0 + z.rp, z.nz), r0 = a0 - MG_DOWN, n = b0 - a0 + 2 * MG_DOWN;
+  float *U = band_buf<SM>(scratch, scratch_n), *F = U + (z.rp + 2 * MG_DOWN) * P;
+  const double2 mine = resid0(z, call->Psi, call->rhs, call->umask, U, F, a0, b0);
+  __shared__ bool last;
+  {
+    const double2 s = block_sums(mine.x, mine.y); // (its barrier also ends the residual)
+    if (threadIdx.x == 0) {
+      z.part[2 * blockIdx.x] = s.x;
+      z.part[2 * blockIdx.x + 1] = s.y;
+      __threadfence();
+      last = atomicAdd(&call->ticket, 1u) == gridDim.x - 1;
+    }
+  }
+  {
+    Part0 t;
+    part0(z, t, 0);
+    for (int k = 1; k < 4; k++) { // colours 1, 0, 1
+      relax0<false>(z, t, U, F, r0, k, n - k, k & 1);
+      __syncthreads();
+    }
+    for (int s = MG_DOWN + (threadIdx.x >> 5); s < n - MG_DOWN; s += MG_W)
+      for (int c0 = 4 * (threadIdx.x & 31); c0 < P; c0 += 128)
+        st4(z.u + (size_t)(r0 + s) * P + c0, ld4(U + s * P + c0));
+    relax0<true>(z, t, U, F, r0, MG_DOWN - 1, n - MG_DOWN + 1, 0);
+    __syncthreads();
+  }
+  restrict0(C, P, F, r0, (a0 + C.cz - 1) / C.cz, min((b0 + C.cz - 1) / C.cz, C.Z), C.f);
+  if (!last)
+    return;
+  __threadfence();
+  double x = 0, y = 0; // the bands' sums, in a fixed order
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += MG_NT) {
+    x += __ldcg(z.part + 2 * k);
+    y += __ldcg(z.part + 2 * k + 1);
+  }
+  const double2 s = block_sums(x, y);
+  if (threadIdx.x)
+    return;
+  const double total = s.x;
+  if (call->cycles == 0)
+    call->drive = call->rhs ? s.y : total; // poisson.c:40-43; a Laplace solve: its first residual
+  const double drive = call->drive;
+  const bool conv = total == 0 || total < call->accuracy * drive, stop = conv || call->cycles >= call->max_cycles;
+  call->ticket = 0;
+  cudaGraphSetConditional(more, !stop);
+  if (!stop) {
+    call->cycles++;
+    return;
+  }
+  const long long result = conv ? call->cycles : -1;
+  if (call->iters_out)
+    *call->iters_out = result;
+  if (call->st) {
+    call->st->iterations = result;
+    call->st->residual = total;
+    call->st->driving = drive;
+  }
+  call->cnt->mg_cycles += call->cycles;
+  call->cnt->sor_solves += 1;
+}
+
+// rows r0 .. r0+n-1 of a level's array g into the band buffer B (zero outside the array)
+__device__ __forceinline__ void load9(const MgLevel &L, const float *g, float *B, int r0, int n)
+{
+  for (int s = threadIdx.x >> 5; s < n; s += MG_W) {
+    const int I = r0 + s;
+    const bool in = I >= 0 && I < L.Z;
+    for (int c = 4 * (threadIdx.x & 31); c < L.P; c += 128)
+      st4(B + s * L.P + c, in ? ldcg4(g + (size_t)(I + 1) * L.P + c) : make_float4(0.f, 0.f, 0.f, 0.f));
   }
 }
 
-// the grid's totals, formed in the same order by every CTA
-__device__ void grid_totals(const Mg32Args &a, double *tx, double *ty)
+__device__ __forceinline__ void store9(const MgLevel &L, float *g, const float *B, int r0, int Ia, int Ib)
 {
-  __shared__ double tot[2];
-  if (threadIdx.x < 32) {
-    double x = 0, y = 0;
-    for (int k = threadIdx.x; k < (int)gridDim.x; k += 32) {
-      x += __ldcg(a.part + 2 * k);
-      y += __ldcg(a.part + 2 * k + 1);
+  for (int I = Ia + (threadIdx.x >> 5); I < Ib; I += MG_W)
+    for (int c = 4 * (threadIdx.x & 31); c < L.P; c += 128)
+      st4(g + (size_t)(I + 1) * L.P + c, ld4(B + (I - r0) * L.P + c));
+}
+
+// A coarse level down, a band a CTA: two four-colour sweeps from u = 0, the
+// halo shrinking by a row a row parity (the first needs none), then f of the
+// next level from the residual of the band's rows.
+template <bool SM, class Op>
+__global__ void __launch_bounds__(MG_NT, 1) k_mg_down9(const __grid_constant__ MgLevel L,
+                                                       const __grid_constant__ MgLevel C, float *scratch,
+                                                       size_t scratch_n)
+{
+  float *buf = band_buf<SM>(scratch, scratch_n);
+  const int I0 = blockIdx.x * L.rp, I1 = min(I0 + L.rp, L.Z), r0 = I0 - MG_DOWN, n = I1 - I0 + 2 * MG_DOWN;
+  float *U = buf + L.P, *F = U + (L.rp + 2 * MG_DOWN + 1) * L.P; // a zero row on either side of U
+  load9(L, L.f, F, r0, n);
+  for (int k = 4 * threadIdx.x; k < (n + 2) * L.P; k += 4 * MG_NT)
+    st4(buf + k, make_float4(0.f, 0.f, 0.f, 0.f));
+  __syncthreads();
+  Op t;
+  t.init(L, F, r0, r0, r0 + n);
+#pragma unroll 1
+  for (int k = 0; k < 4; k += 2) {
+    rows9<0, 0>(L, t, U, F, r0, r0 + k, r0 + n - k);
+    rows9<1, 0>(L, t, U, F, r0, r0 + k + 1, r0 + n - k - 1);
+  }
+  store9(L, L.u, U, r0, I0, I1);
+  t.resid(L, U, F, F, r0, I0 - 1, I1 + 1);
+  __syncthreads();
+  restrict9(L, C, F, r0, (I0 + C.cz - 1) / C.cz, min((I1 + C.cz - 1) / C.cz, C.Z), C.f);
+}
+
+// A coarse level up: u of the way down plus the interpolated correction on
+// the band and MG_UP halo rows, then two sweeps in the reverse colour order,
+// into v.
+template <bool SM, class Op>
+__global__ void __launch_bounds__(MG_NT, 1) k_mg_up9(const __grid_constant__ MgLevel L, const __grid_constant__ MgLevel C,
+                                                     float *scratch, size_t scratch_n)
+{
+  float *U = band_buf<SM>(scratch, scratch_n), *F = U + (L.rp + 2 * MG_DOWN) * L.P;
+  const int I0 = blockIdx.x * L.rp, I1 = min(I0 + L.rp, L.Z), r0 = I0 - MG_UP, n = I1 - I0 + 2 * MG_UP;
+  load9(L, L.f, F, r0, n);
+  load9(L, L.u, U, r0, n);
+  __syncthreads();
+  Op t;
+  t.init(L, F, r0, r0, r0 + n);
+  t.template prolong<true>(L, C, U, C.v, r0);
+  __syncthreads();
+#pragma unroll 1
+  for (int k = 1; k < 4; k += 2) {
+    rows9<1, 1>(L, t, U, F, r0, r0 + k, r0 + n - k);
+    rows9<0, 1>(L, t, U, F, r0, r0 + k + 1, r0 + n - k - 1);
+  }
+  store9(L, L.v, U, r0, I0, I1);
+}
+
+// The bilinear correction from level C at the column pairs j .. j+3 (j a
+// multiple of 4) of row i of level 0.
+__device__ __forceinline__ void interp4(const MgLevel &C, int i, int j, float e[4], float o[4])
+{
+  const bool hz = C.cz == 2 && (i & 1); // a half-way row
+  const float *p = C.v + (size_t)((C.cz == 2 ? i >> 1 : i) + 1) * C.P;
+  float w[2][8];
+#pragma unroll
+  for (int h = 0; h < 2; h++, p += C.P)
+    if (h == 0 || hz) {
+      const float *x = p + 1 + (C.cr == 2 ? j >> 1 : j), *y = x + C.Q;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        w[h][k] = C.cr == 2 && k == 3 ? 0.f : __ldcg(x + k);
+        w[h][4 + k] = C.cr == 2 && k > 1 ? 0.f : __ldcg(y + k);
+      }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      x += __shfl_down_sync(0xffffffffu, x, o);
-      y += __shfl_down_sync(0xffffffffu, y, o);
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+    if (h == 0 || hz) {
+      const float *v = w[h];
+      float a[4], b[4]; // even and odd columns
+      if (C.cr == 2) { // coarse nodes j .. j+4: v[0], v[4], v[1], v[5], v[2]
+        a[0] = v[0], a[1] = v[4], a[2] = v[1], a[3] = v[5];
+        b[0] = 0.5f * (v[0] + v[4]), b[1] = 0.5f * (v[4] + v[1]), b[2] = 0.5f * (v[1] + v[5]), b[3] = 0.5f * (v[5] + v[2]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          a[k] = v[k], b[k] = v[4 + k];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        e[k] = h ? 0.5f * e[k] + 0.5f * a[k] : a[k];
+        o[k] = h ? 0.5f * o[k] + 0.5f * b[k] : b[k];
+      }
     }
-    if (threadIdx.x == 0) {
-      tot[0] = x;
-      tot[1] = y;
+}
+
+// Level 0 up: the same with colours 1, 0, 1, 0; the result goes to Psi in FP64.
+template <bool SM>
+__global__ void __launch_bounds__(MG_NT, 1) k_mg_up0(const __grid_constant__ Mg0 z, const __grid_constant__ MgLevel C,
+                                                     const MgCall *call, float *scratch, size_t scratch_n)
+{
+  const int P = z.P, H = P >> 1, K = (H / 4 + 31) >> 5, lane = threadIdx.x & 31;
+  const float nan = __int_as_float(0x7fc00000);
+  const int a0 = blockIdx.x * z.rp, b0 = min(a0 + z.rp, z.nz), r0 = a0 - MG_UP, n = b0 - a0 + 2 * MG_UP;
+  float *U = band_buf<SM>(scratch, scratch_n), *F = U + (z.rp + 2 * MG_DOWN) * P;
+  for (int t = threadIdx.x >> 5; t < n * K; t += MG_W) {
+    const int s = (unsigned)t / (unsigned)K, j = 4 * ((t - s * K) * 32 + lane), iz = r0 + s;
+    if (j >= H)
+      continue;
+    float4 f[2], u[2]; // even columns, odd columns
+    f[0] = f[1] = make_float4(nan, nan, nan, nan);
+    u[0] = u[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (iz >= z.lo && iz <= z.hi && 2 * j < z.cols) {
+      const size_t at = (size_t)iz * P + j;
+      f[0] = ldcg4(z.f + at);
+      f[1] = ldcg4(z.f + at + H);
+      u[0] = ldcg4(z.u + at);
+      u[1] = ldcg4(z.u + at + H);
+      float e[4], o[4];
+      interp4(C, iz, j, e, o);
+      u[0].x = f[0].x == f[0].x ? u[0].x + e[0] : 0.f;
+      u[0].y = f[0].y == f[0].y ? u[0].y + e[1] : 0.f;
+      u[0].z = f[0].z == f[0].z ? u[0].z + e[2] : 0.f;
+      u[0].w = f[0].w == f[0].w ? u[0].w + e[3] : 0.f;
+      u[1].x = f[1].x == f[1].x ? u[1].x + o[0] : 0.f;
+      u[1].y = f[1].y == f[1].y ? u[1].y + o[1] : 0.f;
+      u[1].z = f[1].z == f[1].z ? u[1].z + o[2] : 0.f;
+      u[1].w = f[1].w == f[1].w ? u[1].w + o[3] : 0.f;
+    }
+    st4(U + s * P + j, u[0]);
+    st4(U + s * P + H + j, u[1]);
+    st4(F + s * P + j, f[0]);
+    st4(F + s * P + H + j, f[1]);
+  }
+  {
+    Part0 t;
+    part0(z, t, 0);
+    __syncthreads();
+    for (int k = 1; k <= 4; k++) {
+      relax0<false>(z, t, U, F, r0, k, n - k, k & 1);
+      __syncthreads();
+    }
+  }
+  double *Psi = call->Psi;
+  const int K2 = (H + 31) >> 5, nt = (b0 - a0) * K2;
+  for (int tb = threadIdx.x >> 5; tb < nt; tb += MG_W * MG_AHEAD) {
+    double2 x[MG_AHEAD];
+    int at[MG_AHEAD];
+#pragma unroll
+    for (int k = 0; k < MG_AHEAD; k++) {
+      const int t = tb + k * MG_W, q = (unsigned)t / (unsigned)K2, j = (t - q * K2) * 32 + lane;
+      at[k] = t < nt && 2 * j < z.cols ? (q + MG_UP) * P + j : -1;
+      if (at[k] >= 0)
+        x[k] = *reinterpret_cast<const double2 *>(Psi + node(a0 + q, 2 * j, P));
+    }
+#pragma unroll
+    for (int k = 0; k < MG_AHEAD; k++)
+      if (at[k] >= 0) {
+        const int t = tb + k * MG_W, q = (unsigned)t / (unsigned)K2, j = (t - q * K2) * 32 + lane;
+        const bool fe = F[at[k]] == F[at[k]], fo = F[at[k] + H] == F[at[k] + H];
+        if (fe)
+          x[k].x += (double)U[at[k]];
+        if (fo)
+          x[k].y += (double)U[at[k] + H];
+        if (fe || fo)
+          *reinterpret_cast<double2 *>(Psi + node(a0 + q, 2 * j, P)) = x[k];
+      }
+  }
+}
+
+// The smallest levels, lev[0] .. lev[n-1], by one CTA with CTA barriers:
+// descent, the coarsest level's solve, ascent back to lev[0], whose u goes to
+// its v.  With SM the levels' u and f (from soff on) and a residual lie in
+// shared memory, else in global memory.
+struct MgTail {
+  MgLevel lev[MG_MAX_LEVELS];
+  int n;
+  const float *cinv; // the coarsest level's inverse, cn x cn row-major (null: coarse sweeps)
+  const int *cidx;   // its unknowns' array indices on that level
+  int cn;
+};
+
+template <bool SM, class Op> __global__ void __launch_bounds__(MG_NT, 1) k_mg_tail(const __grid_constant__ MgTail a)
+{
+  __shared__ float coarse_f[MG_MAX_DIRECT]; // the coarsest level's f, gathered for its exact solve
+  float *buf = reinterpret_cast<float *>(mg_smem);
+  const int N = a.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  auto uof = [&](int l) { return SM ? buf + a.lev[l].soff : a.lev[l].u; }; // row -1 first
+  auto fof = [&](int l) { return SM ? buf + a.lev[l].soff + (a.lev[l].Z + 2) * a.lev[l].P : a.lev[l].f; };
+  float *R = SM ? buf : a.lev[0].v; // the residual of one level at a time (v is free until the end)
+  for (int l = 0; l < N; l++) {
+    const int n = (a.lev[l].Z + 2) * a.lev[l].P;
+    float *u = uof(l), *f = fof(l);
+    const float *g = a.lev[l].f;
+    for (int k = 4 * tid; k < n; k += 4 * MG_NT) {
+      st4(u + k, make_float4(0.f, 0.f, 0.f, 0.f));
+      if (SM)
+        st4(f + k, l == 0 ? ldcg4(g + k) : make_float4(0.f, 0.f, 0.f, 0.f));
     }
   }
   __syncthreads();
-  *tx = tot[0];
-  *ty = tot[1];
-}
-
-__global__ void __launch_bounds__(MG_NT) k_mg32(Mg32Args a, DevCounts *cnt)
-{
-  if (a.st && !a.st->do_solve)
-    return;
-  unsigned gen = 0;
-  double drive = 0, total = 0;
-  long long cycles = 0;
-  bool conv = false;
-  for (;;) {
-    const bool first = cycles == 0;
-    double rs, ds;
-    residual64(a, first, &rs, &ds);
-    block_sums(a, rs, ds);
-    if (!mg_grid_sync(a, gen, cnt))
-      return;
-    double dsum;
-    grid_totals(a, &total, &dsum);
-    if (first)
-      drive = a.rhs ? dsum : total; // poisson.c:40-43; a Laplace solve: its first residual
-    if (total == 0 || total < a.accuracy * drive) {
-      conv = true;
+  Op t;
+#pragma unroll 1
+  for (int l = 0; l < N; l++) {
+    if (l == N - 1 && a.cinv)
       break;
+    const MgLevel L = a.lev[l];
+    float *u = uof(l), *f = fof(l);
+    t.init(L, f, -1, 0, L.Z);
+    for (int k = 4 * tid; k < (L.Z + 2) * L.P; k += 4 * MG_NT) // halos of the residual
+      st4(R + k, make_float4(0.f, 0.f, 0.f, 0.f));
+    const int sweeps = l == N - 1 ? MG_COARSE_SWEEPS : 2;
+#pragma unroll 1
+    for (int k = 0; k < sweeps; k++) {
+      rows9<0, 0>(L, t, u, f, -1, 0, L.Z);
+      rows9<1, 0>(L, t, u, f, -1, 0, L.Z);
     }
-    if (cycles >= a.max_cycles)
+    if (l == N - 1)
       break;
-    // (the partials are rewritten only after the V-cycle's first barrier,
-    // which every CTA reaches after reading them)
-    if (!vcycle(a, gen, cnt))
-      return;
-    if (a.nu0 == 0) { // no sweep to fold into
-      fold(a);
-      if (!mg_grid_sync(a, gen, cnt))
-        return;
-    }
-    cycles++;
+    t.resid(L, u, f, R, -1, 0, L.Z);
+    __syncthreads();
+    restrict9(L, a.lev[l + 1], R, -1, 0, a.lev[l + 1].Z, fof(l + 1));
+    __syncthreads();
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const long long result = conv ? cycles : -1;
-    if (a.iters_out)
-      *a.iters_out = result;
-    if (a.st) {
-      a.st->iterations = result;
-      a.st->residual = total;
-      a.st->driving = drive;
+  if (a.cinv) {
+    // the coarsest level solved exactly: u = A^-1 f over its unknowns
+    const float *f = fof(N - 1);
+    float *u = uof(N - 1);
+    for (int i = tid; i < a.cn; i += MG_NT)
+      coarse_f[i] = f[__ldg(a.cidx + i)];
+    __syncthreads();
+    // a warp per row: coalesced reads of the row, the lanes' partial sums
+    // added by shuffles
+    for (int i = warp; i < a.cn; i += MG_W) {
+      const float *row = a.cinv + (size_t)i * a.cn;
+      float acc = 0.f;
+      for (int k = lane; k < a.cn; k += 32)
+        acc += __ldg(row + k) * coarse_f[k];
+      for (int o = 16; o > 0; o >>= 1)
+        acc += __shfl_down_sync(0xffffffffu, acc, o);
+      if (lane == 0)
+        u[__ldg(a.cidx + i)] = acc;
     }
-    cnt->mg_cycles += cycles;
-    cnt->sor_solves += 1;
+    __syncthreads();
   }
+#pragma unroll 1
+  for (int l = N - 2; l >= 0; l--) {
+    const MgLevel L = a.lev[l];
+    float *u = uof(l), *f = fof(l);
+    t.init(L, f, -1, 0, L.Z);
+    t.template prolong<false>(L, a.lev[l + 1], u, uof(l + 1), -1);
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) {
+      rows9<1, 1>(L, t, u, f, -1, 0, L.Z);
+      rows9<0, 1>(L, t, u, f, -1, 0, L.Z);
+    }
+  }
+  const float *u = uof(0);
+  float *v = a.lev[0].v;
+  for (int k = 4 * tid, n = (a.lev[0].Z + 2) * a.lev[0].P; k < n; k += 4 * MG_NT)
+    st4(v + k, ld4(u + k));
 }
 
 // ---- host: the level hierarchy
@@ -901,9 +1208,9 @@ size_t unknowns(const Stencil &S)
 
 extern "C" void s32_mg_free(Mg32Work *w)
 {
+  if (w->exec)
+    cudaGraphExecDestroy((cudaGraphExec_t)w->exec);
   cudaFree(w->mem);
-  cudaFree(w->cinv);
-  cudaFree(w->cidx);
   *w = Mg32Work();
 }
 
@@ -911,7 +1218,7 @@ namespace {
 // The inverse of the coarsest level's operator over its unknowns (Gauss-Jordan
 // with partial pivoting in FP64), for the exact coarse solve; false when the
 // level has more than MG_MAX_DIRECT unknowns or the matrix is singular.
-bool coarse_inverse(const Stencil &S, int P, std::vector<float> &inv, std::vector<int> &idx)
+bool coarse_inverse(const Stencil &S, const MgLevel &D, std::vector<float> &inv, std::vector<int> &idx)
 {
   std::vector<int> num((size_t)S.Z * S.R, -1);
   idx.clear();
@@ -919,7 +1226,7 @@ bool coarse_inverse(const Stencil &S, int P, std::vector<float> &inv, std::vecto
     for (int J = 0; J < S.R; J++)
       if (S.unk[(size_t)I * S.R + J]) {
         num[(size_t)I * S.R + J] = (int)idx.size();
-        idx.push_back((I + 1) * P + J + 1);
+        idx.push_back((I + 1) * D.P + (J & 1) * D.Q + (J >> 1) + 1);
       }
   const int n = (int)idx.size();
   if (n == 0 || n > MG_MAX_DIRECT)
@@ -977,6 +1284,112 @@ bool coarse_inverse(const Stencil &S, int P, std::vector<float> &inv, std::vecto
 }
 } // namespace
 
+namespace {
+// the kernels whose bands lie in shared memory
+std::vector<const void *> mg_smem_kernels()
+{
+  return {(const void *)k_mg_down0<true>,          (const void *)k_mg_up0<true>,
+          (const void *)k_mg_down9<true, Fix9<1>>, (const void *)k_mg_down9<true, Fix9<2>>,
+          (const void *)k_mg_down9<true, Run9>,    (const void *)k_mg_up9<true, Fix9<1>>,
+          (const void *)k_mg_up9<true, Fix9<2>>,   (const void *)k_mg_up9<true, Run9>,
+          (const void *)k_mg_tail<true, Fix9<2>>,  (const void *)k_mg_tail<true, Run9>};
+}
+
+// The solve as a graph: the residual's kernel, then a WHILE node around a
+// V-cycle that ends with the next residual.
+int mg_graph(Mg32Work *w, Mg0 z, MgTail t, int tail, bool sm, bool tail_sm, float *scratch, size_t budget,
+             size_t tail_bytes)
+{
+  MgLevel *lev = w->lev;
+  MgCall *call = (MgCall *)w->call;
+  auto bytes_of = [&](int rp, int P) { return sm ? (size_t)(2 * rp + 4 * MG_DOWN + 2) * P * sizeof(float) : 0; };
+  auto floats_of = [](int rp, int P) { return (size_t)(2 * rp + 4 * MG_DOWN + 2) * P; };
+  const void *kd0 = sm ? (const void *)k_mg_down0<true> : (const void *)k_mg_down0<false>;
+  // pairs of a row parity in n rows, a thread's number of them: Fix9 or Run9
+  auto pairs = [](const MgLevel &D, int n) { return (size_t)((n + 1) / 2) * ((D.R + 1) / 2); };
+  auto kd9 = [&](const MgLevel &D) {
+    const size_t n = pairs(D, D.rp + 2 * MG_DOWN);
+    return !sm                ? (const void *)k_mg_down9<false, Run9>
+           : n <= MG_NT       ? (const void *)k_mg_down9<true, Fix9<1>>
+           : n <= 2 * MG_NT   ? (const void *)k_mg_down9<true, Fix9<2>>
+                              : (const void *)k_mg_down9<true, Run9>;
+  };
+  auto ku9 = [&](const MgLevel &D) {
+    const size_t n = pairs(D, D.rp + 2 * MG_UP);
+    return !sm                ? (const void *)k_mg_up9<false, Run9>
+           : n <= MG_NT       ? (const void *)k_mg_up9<true, Fix9<1>>
+           : n <= 2 * MG_NT   ? (const void *)k_mg_up9<true, Fix9<2>>
+                              : (const void *)k_mg_up9<true, Run9>;
+  };
+  const void *ku0 = sm ? (const void *)k_mg_up0<true> : (const void *)k_mg_up0<false>;
+  const void *kt = !tail_sm                                       ? (const void *)k_mg_tail<false, Run9>
+                   : pairs(lev[tail], lev[tail].Z) <= 2 * MG_NT ? (const void *)k_mg_tail<true, Fix9<2>>
+                                                                  : (const void *)k_mg_tail<true, Run9>;
+  cudaError_t e = cudaSuccess;
+  // the attribute is process-wide: the kernels' limit, not this instance's need
+  for (const void *k : mg_smem_kernels())
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
+  cudaGraph_t graph = nullptr;
+  if (e == cudaSuccess)
+    e = cudaGraphCreate(&graph, 0);
+  if (e != cudaSuccess)
+    return (int)e;
+  cudaGraphConditionalHandle more{};
+  e = cudaGraphConditionalHandleCreate(&more, graph, 0, 0);
+  cudaGraphNode_t prev = nullptr;
+  auto add = [&](cudaGraph_t g, const void *k, int blocks, size_t smem, void **args) {
+    if (e != cudaSuccess)
+      return;
+    cudaKernelNodeParams p{};
+    p.func = (void *)k;
+    p.gridDim = dim3(blocks);
+    p.blockDim = dim3(MG_NT);
+    p.sharedMemBytes = (unsigned)smem;
+    p.kernelParams = args;
+    cudaGraphNode_t n;
+    e = cudaGraphAddKernelNode(&n, g, prev ? &prev : nullptr, prev ? 1 : 0, &p);
+    prev = n;
+  };
+  size_t n0 = floats_of(z.rp, z.P);
+  void *a_down0[] = {&z, &lev[1], &call, &more, &scratch, &n0};
+  void *a_up0[] = {&z, &lev[1], &call, &scratch, &n0};
+  add(graph, kd0, z.nb, bytes_of(z.rp, z.P), a_down0);
+  cudaGraphNodeParams cp{};
+  cp.type = cudaGraphNodeTypeConditional;
+  cp.conditional.handle = more;
+  cp.conditional.type = cudaGraphCondTypeWhile;
+  cp.conditional.size = 1;
+  cudaGraphNode_t loop;
+  if (e == cudaSuccess)
+    e = cudaGraphAddNode(&loop, graph, &prev, 1, &cp);
+  if (e == cudaSuccess) {
+    cudaGraph_t body = cp.conditional.phGraph_out[0];
+    prev = nullptr;
+    for (int l = 1; l < tail; l++) {
+      size_t n = floats_of(lev[l].rp, lev[l].P);
+      void *a9[] = {&lev[l], &lev[l + 1], &scratch, &n};
+      add(body, kd9(lev[l]), lev[l].nb, bytes_of(lev[l].rp, lev[l].P), a9);
+    }
+    void *at[] = {&t};
+    add(body, kt, 1, tail_sm ? tail_bytes : 0, at);
+    for (int l = tail - 1; l >= 1; l--) {
+      size_t n = floats_of(lev[l].rp, lev[l].P);
+      void *a9[] = {&lev[l], &lev[l + 1], &scratch, &n};
+      add(body, ku9(lev[l]), lev[l].nb, bytes_of(lev[l].rp, lev[l].P), a9);
+    }
+    add(body, ku0, z.nb, bytes_of(z.rp, z.P), a_up0);
+    add(body, kd0, z.nb, bytes_of(z.rp, z.P), a_down0);
+  }
+  cudaGraphExec_t exec = nullptr;
+  if (e == cudaSuccess)
+    e = cudaGraphInstantiate(&exec, graph, 0);
+  w->exec = exec;
+  cudaGraphDestroy(graph);
+  return (int)e;
+}
+} // namespace
+
 extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *flags, Mg32Work *w, cudaStream_t s)
 {
   s32_mg_free(w);
@@ -1014,51 +1427,105 @@ extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *flags, Mg32Work *w,
   const int L = (int)lev.size();
   if (L < 2)
     return (int)cudaErrorInvalidConfiguration; // a mesh too small to coarsen: the caller uses SOR
-  // device layout: level 0's u0, f0 at the mesh pitch; per coarse level u,
-  // f, MG_NCOEF coefficient planes of (Z+2) x P floats, rw of 3 R floats
-  const size_t n0 = (size_t)(m->nz + 1) * m->pitch;
-  size_t bytes = 2 * n0 * sizeof(float);
-  std::vector<size_t> off(L), coff(L), roff(L);
+  // constant data, gathered on the host and copied once: the coefficients of
+  // each level's distinct rows (a row's metal decides them, so a gun has few;
+  // cls names a row's), the restriction weights, level 0's radial couplings
+  const int P0 = m->pitch;
+  std::vector<char> blob;
+  auto put = [&](const void *p, size_t n) {
+    const size_t at = blob.size();
+    blob.resize((at + n + 255) / 256 * 256);
+    std::memcpy(blob.data() + at, p, n);
+    return at;
+  };
+  std::vector<size_t> coff(L), roff(L), ioff(L);
   for (int l = 1; l < L; l++) {
-    const int P = (lev[l].R + 2 + 31) / 32 * 32;
-    const size_t plane = (size_t)(lev[l].Z + 2) * P;
-    off[l] = bytes;
-    bytes += 2 * plane * sizeof(float);
-    coff[l] = bytes;
-    bytes += MG_NCOEF * plane * sizeof(float);
-    roff[l] = bytes;
-    bytes += ((size_t)3 * lev[l].R * sizeof(float) + 255) / 256 * 256;
+    const Stencil &S = lev[l];
+    MgLevel &D = w->lev[l];
+    D.Z = S.Z;
+    D.R = S.R;
+    D.cz = czs[l];
+    D.cr = crs[l];
+    D.Q = ((S.R >> 1) + 2 + 15) / 16 * 16;
+    D.P = 2 * D.Q;
+    const size_t row_n = (size_t)MG_NCOEF * D.P;
+    std::vector<float> all((size_t)S.Z * row_n, 0.f);
+    parallel_rows(S.Z, [&](int I0, int I1) {
+      for (int I = I0; I < I1; I++) {
+        float *row = all.data() + (size_t)I * row_n;
+        for (int J = 0; J < S.R; J++) {
+          if (!S.unk[(size_t)I * S.R + J])
+            continue;
+          const int at = (J & 1) * D.Q + (J >> 1) + 1;
+          const double dg = S.at(4, I, J);
+          int q = 0;
+          for (int k = 0; k < 9; k++)
+            if (k != 4)
+              row[(size_t)D.P * q++ + at] = (float)(S.at(k, I, J) / dg);
+          row[(size_t)D.P * MG_INVD + at] = (float)(1 / dg);
+          row[(size_t)D.P * MG_DIAG + at] = (float)dg;
+        }
+      }
+    });
+    // a row's class: most rows are like the one before
+    std::vector<uint8_t> same(S.Z, 0);
+    parallel_rows(S.Z, [&](int I0, int I1) {
+      for (int I = std::max(I0, 1); I < I1; I++)
+        same[I] = !std::memcmp(all.data() + (size_t)I * row_n, all.data() + (size_t)(I - 1) * row_n, row_n * sizeof(float));
+    });
+    std::unordered_multimap<uint64_t, int> seen; // hash -> class
+    std::vector<int> cls(S.Z), first;            // a row's class, a class's first row
+    for (int I = 0; I < S.Z; I++) {
+      const float *row = all.data() + (size_t)I * row_n;
+      int c = same[I] ? cls[I - 1] : -1;
+      if (c < 0) {
+        uint64_t h = 1469598103934665603ull; // FNV-1a over 32-bit words
+        for (size_t k = 0; k < row_n; k++) {
+          uint32_t b;
+          std::memcpy(&b, row + k, 4);
+          h = (h ^ b) * 1099511628211ull;
+        }
+        const auto range = seen.equal_range(h);
+        for (auto it = range.first; it != range.second && c < 0; ++it)
+          if (!std::memcmp(all.data() + (size_t)first[it->second] * row_n, row, row_n * sizeof(float)))
+            c = it->second;
+        if (c < 0) {
+          c = (int)first.size();
+          first.push_back(I);
+          seen.emplace(h, c);
+        }
+      }
+      cls[I] = c;
+    }
+    std::vector<float> packed(first.size() * row_n);
+    for (size_t c = 0; c < first.size(); c++)
+      std::memcpy(packed.data() + c * row_n, all.data() + (size_t)first[c] * row_n, row_n * sizeof(float));
+    coff[l] = put(packed.data(), packed.size() * sizeof(float));
+    ioff[l] = put(cls.data(), cls.size() * sizeof(int));
+    std::vector<float> rw(rws[l].begin(), rws[l].end());
+    roff[l] = put(rw.data(), rw.size() * sizeof(float));
   }
-  const size_t sums_off = bytes;
-  int dev = 0, sms = 0, per = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mg32, MG_NT, 0);
-  if (e != cudaSuccess)
-    return (int)e;
-  if (per < 1)
-    return (int)cudaErrorInvalidConfiguration;
-  // one CTA per SM at most (every CTA resident), and no more CTAs than the
-  // mesh gives work: a small mesh's solve then pays for fewer barrier
-  // arrivals and leaves the other SMs to other instances' kernels
-  const size_t mesh_nodes = (size_t)(m->nz + 1) * (m->nr + 1);
-  const int grid = (int)std::min<size_t>((size_t)sms, std::max<size_t>(1, (mesh_nodes + MG_NODES_PER_CTA - 1) / MG_NODES_PER_CTA));
-  bytes += (size_t)2 * grid * sizeof(double) + 32 * sizeof(unsigned long long) + sizeof(long long);
-  char *mem = nullptr;
-  e = cudaMalloc(&mem, bytes);
-  if (e != cudaSuccess)
-    return (int)e;
-  e = cudaMemsetAsync(mem, 0, bytes, s); // halos, held nodes and level 0 start at zero
-  w->mem = mem;
-  w->bytes = bytes;
-  w->nlev = L;
-  w->grid = grid;
-  w->threads = MG_NT;
-  w->u0 = (float *)mem;
-  w->f0 = (float *)mem + n0;
-  w->part = (double *)(mem + sums_off);
-  w->bar = (unsigned long long *)(mem + sums_off + (size_t)2 * grid * sizeof(double));
-  w->iters = (long long *)(w->bar + 32);
+  std::vector<float> crow(P0, 0.f), drow(P0, 0.f);
+  std::vector<double> cpd(P0, 0.0), cmd(P0, 0.0);
+  const double dr2_inv = 1 / (m->dr * m->dr);
+  for (int ir = 0; ir <= m->nr; ir++) {
+    const double h = ir ? 0.5 / ir : 0;
+    cpd[ir] = ir ? dr2_inv * (1 + h) : 4 / (m->dr * m->dr);
+    cmd[ir] = ir ? dr2_inv * (1 - h) : 0;
+    crow[ir] = (float)cpd[ir]; // the axis node has no inner neighbour
+    drow[ir] = (float)cmd[ir];
+  }
+  const size_t o_crow = put(crow.data(), P0 * sizeof(float)), o_drow = put(drow.data(), P0 * sizeof(float));
+  const size_t o_cpd = put(cpd.data(), P0 * sizeof(double)), o_cmd = put(cmd.data(), P0 * sizeof(double));
+  std::vector<float> cinv;
+  std::vector<int> cidx;
+  size_t o_cinv = 0, o_cidx = 0;
+  const bool direct = coarse_inverse(lev[L - 1], w->lev[L - 1], cinv, cidx);
+  if (direct) {
+    o_cinv = put(cinv.data(), cinv.size() * sizeof(float));
+    o_cidx = put(cidx.data(), cidx.size() * sizeof(int));
+  }
+
   // the first level small enough for CTA 0 alone (at least level 1, at most the coarsest)
   int tail = L - 1;
   for (int l = 1; l < L; l++)
@@ -1066,119 +1533,158 @@ extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *flags, Mg32Work *w,
       tail = l;
       break;
     }
-  w->tail = tail;
-  std::vector<float> hc, hr;
-  for (int l = 1; l < L && e == cudaSuccess; l++) {
-    const Stencil &S = lev[l];
+
+  // Bands: a level's rows in one band per SM at most, and no more of them than
+  // the mesh gives work (a small mesh's solve leaves the other SMs to other
+  // instances' kernels; each band recomputes its halo), of MG_MIN_ROWS rows at
+  // least; shorter ones where a band of u and f with its halos would not fit
+  // shared memory.  A mesh whose row is too long for MG_MIN_ROWS of them keeps
+  // its bands in global memory.
+  int dev = 0, sms = 0, max_smem = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  const size_t mesh_nodes = (size_t)(m->nz + 1) * (m->nr + 1);
+  const int grid = (int)std::min<size_t>((size_t)sms, std::max<size_t>(1, (mesh_nodes + MG_NODES_PER_CTA - 1) / MG_NODES_PER_CTA));
+  size_t fixed = 0; // the kernels' own shared memory
+  for (const void *k : mg_smem_kernels()) {
+    cudaFuncAttributes fa{};
+    const cudaError_t e = cudaFuncGetAttributes(&fa, k);
+    if (e != cudaSuccess)
+      return (int)e;
+    fixed = std::max(fixed, fa.sharedSizeBytes);
+  }
+  const size_t budget = ((size_t)max_smem - fixed) / sizeof(float);
+  auto band_n = [](int rp, int P) { return (size_t)(2 * rp + 4 * MG_DOWN + 2) * P; };
+  bool fits = true;
+  size_t need = 0; // floats of the largest band
+  auto band = [&](int rows, int P, int &rp, int &nb) {
+    rp = std::max((rows + grid - 1) / grid, std::min(MG_MIN_ROWS, rows));
+    if (band_n(rp, P) > budget && band_n(MG_MIN_ROWS, P) <= budget)
+      rp = (int)((budget / P - 4 * MG_DOWN - 2) / 2);
+    nb = (rows + rp - 1) / rp;
+    fits = fits && band_n(rp, P) <= budget;
+    need = std::max(need, band_n(rp, P) * nb);
+  };
+  int rp0 = 0, nb0 = 0;
+  band(m->nz, P0, rp0, nb0);
+  for (int l = 1; l < tail; l++)
+    band(w->lev[l].Z, w->lev[l].P, w->lev[l].rp, w->lev[l].nb);
+  // the last levels together: a residual of the largest, each one's u and f
+  size_t soff = (size_t)(lev[tail].Z + 2) * w->lev[tail].P;
+  for (int l = tail; l < L; l++) {
+    w->lev[l].soff = (int)soff;
+    soff += (size_t)2 * (lev[l].Z + 2) * w->lev[l].P;
+  }
+  const bool tail_fits = soff <= budget;
+
+  // device memory, one block: the constant data, level 0's u0 and f0 at the
+  // mesh pitch, each coarse level's u, f and v of (Z+2) x P floats, the
+  // bands' global buffers where they are needed, sums and barrier words
+  const size_t n0 = (size_t)(m->nz + 1) * P0;
+  size_t bytes = blob.size();
+  const size_t o_u0 = bytes;
+  bytes += 2 * n0 * sizeof(float);
+  std::vector<size_t> off(L);
+  for (int l = 1; l < L; l++) {
+    off[l] = bytes;
+    bytes += (size_t)3 * (lev[l].Z + 2) * w->lev[l].P * sizeof(float);
+  }
+  const size_t o_scratch = bytes;
+  bytes += fits ? 0 : need * sizeof(float);
+  const size_t o_part = bytes;
+  bytes += ((size_t)2 * nb0 * sizeof(double) + 255) / 256 * 256;
+  const size_t o_call = bytes;
+  bytes += sizeof(MgCall);
+  char *mem = nullptr;
+  cudaError_t e = cudaMalloc(&mem, bytes);
+  if (e != cudaSuccess)
+    return (int)e;
+  w->mem = mem;
+  w->bytes = bytes;
+  w->call = mem + o_call;
+  for (int l = 1; l < L; l++) {
     MgLevel &D = w->lev[l];
-    D.Z = S.Z;
-    D.R = S.R;
-    D.cz = czs[l];
-    D.cr = crs[l];
-    D.P = (S.R + 2 + 31) / 32 * 32;
-    const size_t plane = (size_t)(S.Z + 2) * D.P;
+    const size_t plane = (size_t)(D.Z + 2) * D.P;
     D.u = (float *)(mem + off[l]);
     D.f = D.u + plane;
+    D.v = D.f + plane;
     D.coef = (const float *)(mem + coff[l]);
+    D.cls = (const int *)(mem + ioff[l]);
     D.rw = (const float *)(mem + roff[l]);
-    hc.assign(MG_NCOEF * plane, 0.f);
-    for (int I = 0; I < S.Z; I++)
-      for (int J = 0; J < S.R; J++) {
-        if (!S.unk[(size_t)I * S.R + J])
-          continue;
-        const size_t idx = (size_t)(I + 1) * D.P + J + 1;
-        const double dg = S.at(4, I, J);
-        int q = 0;
-        for (int k = 0; k < 9; k++) {
-          if (k == 4)
-            continue;
-          hc[(size_t)q * plane + idx] = (float)(S.at(k, I, J) / dg);
-          q++;
-        }
-        hc[(size_t)MG_INVD * plane + idx] = (float)(1 / dg);
-        hc[(size_t)MG_DIAG * plane + idx] = (float)dg;
-      }
-    hr.assign((size_t)3 * S.R, 0.f);
-    for (size_t k = 0; k < hr.size(); k++)
-      hr[k] = (float)rws[l][k];
-    e = cudaMemcpyAsync(mem + coff[l], hc.data(), hc.size() * sizeof(float), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(mem + roff[l], hr.data(), hr.size() * sizeof(float), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-      e = cudaStreamSynchronize(s); // the host staging is reused by the next level
   }
-  // the coarsest level's inverse for its exact solve
-  std::vector<float> cinv;
-  std::vector<int> cidx;
-  if (e == cudaSuccess && coarse_inverse(lev[L - 1], w->lev[L - 1].P, cinv, cidx)) {
-    e = cudaMalloc(&w->cinv, cinv.size() * sizeof(float));
-    if (e == cudaSuccess)
-      e = cudaMalloc(&w->cidx, cidx.size() * sizeof(int));
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(w->cinv, cinv.data(), cinv.size() * sizeof(float), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(w->cidx, cidx.data(), cidx.size() * sizeof(int), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-      e = cudaStreamSynchronize(s);
-    w->cn = (int)cidx.size();
-  }
-  if (e != cudaSuccess)
+  // halos and held nodes start at zero
+  e = cudaMemsetAsync(mem + blob.size(), 0, bytes - blob.size(), s);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(mem, blob.data(), blob.size(), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess)
+    e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) {
     s32_mg_free(w);
-  return (int)e;
+    return (int)e;
+  }
+
+  Mg0 z{};
+  z.nz = m->nz;
+  z.P = P0;
+  z.lo = lo;
+  z.hi = hi;
+  z.cols = m->nr - 1;
+  z.rp = rp0;
+  z.nb = nb0;
+  const double dz2 = m->dz * m->dz, dr2 = m->dr * m->dr;
+  z.a_d = 1 / dz2;
+  z.e_d = -2 * (1 / dz2 + 1 / dr2);
+  z.e2c_d = z.e_d - 2 / dr2;
+  z.a = (float)z.a_d;
+  z.e = (float)z.e_d;
+  z.e2c = (float)z.e2c_d;
+  z.inv_e = (float)(1 / z.e_d);
+  z.inv_e2c = (float)(1 / z.e2c_d);
+  z.u = (float *)(mem + o_u0);
+  z.f = z.u + n0;
+  z.crow = (const float *)(mem + o_crow);
+  z.drow = (const float *)(mem + o_drow);
+  z.cpd = (const double *)(mem + o_cpd);
+  z.cmd = (const double *)(mem + o_cmd);
+  z.part = (double *)(mem + o_part);
+  MgTail t{};
+  t.n = L - tail;
+  for (int l = tail; l < L; l++)
+    t.lev[l - tail] = w->lev[l];
+  t.cinv = direct ? (const float *)(mem + o_cinv) : nullptr;
+  t.cidx = direct ? (const int *)(mem + o_cidx) : nullptr;
+  t.cn = direct ? (int)cidx.size() : 0;
+  e = (cudaError_t)mg_graph(w, z, t, tail, fits, tail_fits, (float *)(mem + o_scratch), budget * sizeof(float),
+                            soff * sizeof(float));
+  if (e != cudaSuccess) {
+    s32_mg_free(w);
+    return (int)e;
+  }
+  w->nlev = L;
+  return 0;
 }
 
 // the solve on Psi with driving term rhs (null: Laplace), stop rule
 // sum|r| < accuracy sum|rhs|, at most max_cycles V-cycles
-extern "C" int s32_mg_solve(const DevMesh *m, Mg32Work *w, const float *crow, const float *drow, double *Psi,
-                            const double *rhs, const uint8_t *umask, double accuracy, long long max_cycles,
-                            PcState *st, long long *iters_out, DevCounts *cnt, cudaStream_t s)
+extern "C" int s32_mg_solve(const DevMesh *m, Mg32Work *w, double *Psi, const double *rhs, const uint8_t *umask,
+                            double accuracy, long long max_cycles, PcState *st, long long *iters_out, DevCounts *cnt,
+                            cudaStream_t s)
 {
-  Mg32Args a{};
-  a.Psi = Psi;
-  a.rhs = rhs;
-  a.umask = umask;
-  a.u0 = w->u0;
-  a.f0 = w->f0;
-  a.crow = crow;
-  a.drow = drow;
-  a.nz = m->nz;
-  a.P0 = m->pitch;
-  a.lo = m->left_bc == SPIFFE_DIRICHLET ? 0 : 1;
-  a.hi = m->right_bc == SPIFFE_DIRICHLET ? m->nz - 1 : m->nz - 2;
-  a.cols = m->nr - 1;
-  const double dz2 = m->dz * m->dz, dr2 = m->dr * m->dr;
-  a.a_d = 1 / dz2;
-  a.e_d = -2 * (1 / dz2 + 1 / dr2);
-  a.c4_d = 4 / dr2;
-  a.e2c_d = a.e_d - 2 / dr2;
-  a.dr2_inv = 1 / dr2;
-  a.a = (float)a.a_d;
-  a.c4 = (float)a.c4_d;
-  a.e = (float)a.e_d;
-  a.e2c = (float)a.e2c_d;
-  a.inv_e = (float)(1 / a.e_d);
-  a.inv_e2c = (float)(1 / a.e2c_d);
-  a.nlev = w->nlev;
-  a.tail = w->tail;
-  a.nu0 = 2;
-  a.nu = 2;
-  a.coarse_sweeps = 24;
-  a.cinv = w->cinv;
-  a.cidx = w->cidx;
-  a.cn = w->cn;
-  a.max_cycles = (int)std::min<long long>(max_cycles, 100);
-  a.accuracy = accuracy;
-  for (int l = 0; l < w->nlev; l++)
-    a.lev[l] = w->lev[l];
-  a.bar = w->bar;
-  a.part = w->part;
-  a.st = st;
-  a.iters_out = iters_out ? iters_out : w->iters;
-  cudaError_t e = cudaMemsetAsync(w->bar, 0, 32 * sizeof(unsigned long long), s);
-  if (e != cudaSuccess)
-    return (int)e;
-  void *args[] = {&a, &cnt};
-  e = cudaLaunchCooperativeKernel((const void *)k_mg32, dim3(w->grid), dim3(w->threads), args, 0, s);
-  spiffe_note_launches(1);
+  (void)m;
+  MgCall c{};
+  c.Psi = Psi;
+  c.rhs = rhs;
+  c.umask = umask;
+  c.accuracy = accuracy;
+  c.max_cycles = std::min<long long>(max_cycles, 100);
+  c.st = st;
+  c.iters_out = iters_out;
+  c.cnt = cnt;
+  k_mg_begin<<<1, 1, 0, s>>>(c, (MgCall *)w->call);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaGraphLaunch((cudaGraphExec_t)w->exec, s);
+  spiffe_note_launches(2);
   return (int)e;
 }

@@ -1257,7 +1257,7 @@ extern "C" int s32_solve(const DevMesh *m, Poisson32Work *w, double *Psi, const 
                          double accuracy, long long limit, PcState *st, DevCounts *cnt, cudaStream_t s)
 {
   if (w->solver == SPIFFE_POISSON_MULTIGRID && w->mg.nlev >= 2)
-    return s32_mg_solve(m, &w->mg, w->crow, w->drow, Psi, rhs, umask, accuracy, limit, st, w->iters, cnt, s);
+    return s32_mg_solve(m, &w->mg, Psi, rhs, umask, accuracy, limit, st, w->iters, cnt, s);
   return s32_sor(m, w, Psi, rhs, umask, accuracy, limit, st, cnt, s);
 }
 

@@ -181,32 +181,31 @@ extern "C" int s32_births(const DevMesh *m, const DevFields32 *f, const DevBeam3
 #define MG_MAX_LEVELS 14
 #define MG_NCOEF 10 // 8 off-diagonal coefficients divided by the diagonal, 1/diagonal, diagonal
 struct MgLevel {
-  int Z = 0, R = 0, P = 0; // nodes in z and r; row pitch with one halo node a side
-  float *u = nullptr, *f = nullptr; // (Z+2) x P, node (I, J) at (I+1) P + J + 1; halo nodes stay 0
-  const float *coef = nullptr;      // MG_NCOEF arrays of (Z+2) x P; 1/diagonal 0 marks a held node
-  const float *rw = nullptr;        // restriction weights from the level above: [J][3], columns cr J - 1, cr J, cr J + 1
-  int cz = 2, cr = 2;               // coarsening from the level above in z and r: node (I, J) is its (cz I, cr J)
+  int Z = 0, R = 0;    // nodes in z and r
+  int P = 0, Q = 0;    // row pitch; column J of a row lies at (J&1) Q + (J>>1) + 1, P = 2 Q
+  int cz = 2, cr = 2;  // coarsening from the level above in z and r: node (I, J) is its (cz I, cr J)
+  int rp = 0, nb = 0;  // rows of a band, bands (levels worked by a band a CTA)
+  int soff = 0;        // place of u and f in shared memory, in floats (the levels worked by one CTA)
+  float *u = nullptr, *f = nullptr, *v = nullptr; // (Z+2) x P, row I at (I+1) P; halo nodes stay 0.
+                                                  // u: pre-smoothed, v: the way up's result
+  const float *coef = nullptr; // [class][MG_NCOEF][P]; 1/diagonal 0 marks a held node
+  const int *cls = nullptr;    // each row's class
+  const float *rw = nullptr;   // restriction weights from the level above: [J][3], columns cr J - 1, cr J, cr J + 1
 };
 struct Mg32Work {
-  int nlev = 0, tail = 0; // levels; first level that CTA 0 works alone
+  int nlev = 0;         // levels (0: not set up)
   MgLevel lev[MG_MAX_LEVELS];
-  float *u0 = nullptr, *f0 = nullptr; // level 0 at the mesh pitch
-  void *mem = nullptr;                // every level array, one allocation
-  double *part = nullptr;             // per-CTA partial sums [grid][2]
-  unsigned long long *bar = nullptr;  // [0] barrier arrivals, [16] abort
-  long long *iters = nullptr;
-  int grid = 0, threads = 0;
+  void *mem = nullptr;  // every level's arrays, one allocation
   size_t bytes = 0;
-  float *cinv = nullptr; // the coarsest level's inverse (exact coarse solve), cn x cn
-  int *cidx = nullptr;   // its unknowns' array indices
-  int cn = 0;
+  void *call = nullptr; // the solve's arguments and state on the device
+  void *exec = nullptr; // the solve's graph (cudaGraphExec_t)
 };
 extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *host_flags, Mg32Work *w, cudaStream_t s);
 extern "C" void s32_mg_free(Mg32Work *w);
 struct PcState;
-extern "C" int s32_mg_solve(const DevMesh *m, Mg32Work *w, const float *crow, const float *drow, double *Psi,
-                            const double *rhs, const uint8_t *umask, double accuracy, long long max_cycles,
-                            PcState *st, long long *iters_out, DevCounts *cnt, cudaStream_t s);
+extern "C" int s32_mg_solve(const DevMesh *m, Mg32Work *w, double *Psi, const double *rhs, const uint8_t *umask,
+                            double accuracy, long long max_cycles, PcState *st, long long *iters_out, DevCounts *cnt,
+                            cudaStream_t s);
 
 // Poisson correction (poisson_f32.cu)
 struct PcState;
