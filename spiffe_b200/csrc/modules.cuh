@@ -73,10 +73,16 @@ extern "C" int spiffe_sor64(const DevMesh *m, Poisson64Work *w, double *Psi, con
 extern "C" int spiffe_poisson_correction64(const DevMesh *m, const DevFields<double> *f, const DevBeam64 *b,
                                            DevCounts *cnt, long long np_bound, const PoissonHostOptions *o,
                                            Poisson64Work *w, Particles64Work *pw, bool ordered, cudaStream_t s);
-// Applies n (node, value) entries held in w->keys / w->vals to dst: a stable
-// sort by node, then each node's values added in entry order starting from
-// dst's current value.  INT_MAX keys are skipped.
-extern "C" int spiffe_ordered_add64(Particles64Work *w, long long n, double *dst, cudaStream_t s);
+// Applies n (node, value) entries held in w->keys / w->vals to dst, an array
+// of `nodes` values: a stable sort by node, then each node's values added in
+// entry order starting from dst's current value.  Entries with key `nodes`
+// are skipped.
+extern "C" int spiffe_ordered_add64(Particles64Work *w, long long n, int nodes, double *dst, cudaStream_t s);
+// the nodes that a particle's charge or current is shared among
+inline int spiffe_smear_nodes(const DevMesh *m)
+{
+  return (m->modes & SPIFFE_FL_RADIAL_SMEAR ? 2 : 1) * (m->modes & SPIFFE_FL_LONGIT_SMEAR ? 2 : 1);
+}
 extern "C" int spiffe_poisson64_report(Poisson64Work *w, spiffe_poisson_report *rep, cudaStream_t s);
 extern "C" int spiffe_imposed_field64(const DevMesh *m, const DevFields<double> *f, double factor, cudaStream_t s);
 

@@ -92,13 +92,13 @@ __global__ void __launch_bounds__(BX *BY) k_apparent_charge(DevMesh m, DevFields
 // Removal of the particles' own charge (:190-242); Qreal partial sums per
 // block.  With keys null each share is subtracted by an FP64 atomic, whose
 // order varies between runs once three or more particles share a node; with
-// keys set, particle ip writes its four (node, -share) pairs to entries
-// 4 ip .. 4 ip + 3 (unused ones keyed INT_MAX) for an ordered reduction that
-// applies them in particle order, the reference's serial Q[iz][ir] -= ...
-// sequence.
+// keys set, particle ip writes its (node, -share) pairs to entries stride ip,
+// ... (unused ones keyed `pad`) for an ordered reduction that applies them in
+// particle order, the reference's serial Q[iz][ir] -= ... sequence; shares
+// that the mesh's smearing leaves at zero, which change no sum, get no entry.
 __global__ void __launch_bounds__(RT) k_remove_charge(DevMesh m, DevFields<double> f, DevBeam64 b,
                                                        const DevCounts *cnt, double *part, int *keys, double *vals,
-                                                       long np_bound)
+                                                       long np_bound, int stride, int pad)
 {
   __shared__ double sh[RT];
   const long ip = (long)blockIdx.x * RT + threadIdx.x;
@@ -155,11 +155,18 @@ __global__ void __launch_bounds__(RT) k_remove_charge(DevMesh m, DevFields<doubl
     }
   }
   if (keys) {
-    if (ip < np_bound)
+    if (ip < np_bound) {
+      const bool lsm = m.modes & SPIFFE_FL_LONGIT_SMEAR, rsm = m.modes & SPIFFE_FL_RADIAL_SMEAR;
+      int e = 0;
+#pragma unroll
       for (int k = 0; k < 4; k++) {
-        keys[4 * ip + k] = at[k];
-        vals[4 * ip + k] = at[k] == 0x7fffffff ? 0.0 : -share[k];
+        if (((k & 1) && !lsm) || ((k & 2) && !rsm))
+          continue;
+        keys[stride * ip + e] = at[k] == 0x7fffffff ? pad : at[k];
+        vals[stride * ip + e] = at[k] == 0x7fffffff ? 0.0 : -share[k];
+        e++;
       }
+    }
   } else {
     for (int k = 0; k < 4; k++)
       if (at[k] != 0x7fffffff)
@@ -672,11 +679,12 @@ extern "C" int spiffe_poisson_correction64(const DevMesh *m, const DevFields<dou
   if (ordered && (!pw || !pw->keys || pw->capacity < np_bound))
     return (int)cudaErrorInvalidValue;
   // the particles' own charge leaves Q (:190-242)
+  const int stride = spiffe_smear_nodes(m), nodes = (m->nz + 1) * m->pitch;
   auto remove_charge = [&]() -> int {
     k_remove_charge<<<blocks_for(np_bound, RT), RT, 0, s>>>(*m, *f, *b, cnt, w->part, ordered ? pw->keys : nullptr,
-                                                            ordered ? pw->vals : nullptr, (long)np_bound);
+                                                            ordered ? pw->vals : nullptr, (long)np_bound, stride, nodes);
     spiffe_note_launches(1);
-    return ordered ? spiffe_ordered_add64(pw, 4 * np_bound, f->Q, s) : 0;
+    return ordered ? spiffe_ordered_add64(pw, stride * np_bound, nodes, f->Q, s) : 0;
   };
   dim3 block(BX, BY), grid((m->nr + 1 + BX - 1) / BX, (m->nz + 1 + BY - 1) / BY);
   const int nblk = grid.x * grid.y;

@@ -1,0 +1,65 @@
+"""The FP64 form's ordered reduction at the sizes where it can go wrong, bit
+for bit against the CPU checker.
+
+* The ordered deposition and charge removal sum each node's particles in
+  particle order; the kernel takes 32 entries a warp and follows a run that
+  goes on behind them 32 at a time, so runs of 1, 31, 32, 33, ... entries at
+  every offset, and meshes with one, two and four entries a particle.
+"""
+import numpy as np
+import pytest
+
+from spiffe_b200 import abi, geometry, gpu, workloads
+from helpers import MODES, QoMC
+
+pytestmark = pytest.mark.gpu
+
+
+def pillbox(nz, nr, modes=MODES, **bcs):
+    cfg = workloads.PillboxConfig(nz=nz, nr=nr)
+    f = geometry.fields_for(nz, nr, cfg.zmin, cfg.zmax, cfg.rmax, cfg.geo_text(), modes=modes, **bcs)
+    f.mesh.dt = cfg.dt
+    return f
+
+
+def crowded_beam(f, counts, seed=3):
+    """Particles counts[k] of which lie around node (5 + k % 20, 1 + k // 20), shuffled."""
+    rng = np.random.default_rng(seed)
+    n, m = int(sum(counts)), f.mesh
+    k = rng.permutation(np.repeat(np.arange(len(counts)), counts))
+    a = {"z": (5 + k % 20 + rng.uniform(-0.49, 0.49, n)) * m.dz, "r": (1 + k // 20 + rng.uniform(-0.49, 0.49, n)) * m.dr}
+    for name in ("vz", "vr", "vphi"):
+        a[name] = rng.normal(size=n) * 1e8
+    b = abi.Beam(n + 16)
+    b.set(n, Q=-rng.uniform(0.5, 1.5, n) * 1e-15, particleID=np.arange(1, n + 1), status=np.ones(n, np.uint64), **a)
+    b.npActive, b.nextParticleID, b.QoMC = n, n + 1, QoMC
+    return b
+
+
+@pytest.mark.parametrize("smear", [0, abi.FL_RADIAL_SMEAR, abi.FL_LONGIT_SMEAR,
+                                   abi.FL_RADIAL_SMEAR | abi.FL_LONGIT_SMEAR])
+@pytest.mark.parametrize("counts", [[1], [31], [32, 1, 1], [33, 31, 65, 64, 2, 1, 96], [5000] + [1] * 200 + [7] * 90])
+def test_ordered_sums_in_particle_order(oracle, counts, smear):
+    f = pillbox(60, 50, MODES | smear)
+    b = crowded_beam(f, counts)
+    g = gpu.GpuInstance(f, capacity=b.capacity)
+    g.set_deposit_order(1)
+    g.upload_beam(b)
+    g.zero_currents()
+    g.deposit()
+    g.deposit()  # a second time on top of the first: the sums start from the arrays' values
+    ref = f.copy()
+    oracle.zero_currents(ref)
+    oracle.deposit(ref, b)
+    oracle.deposit(ref, b)
+    out = g.fields(f)
+    for n in ("Jz", "Jr"):
+        assert np.array_equal(out[n], ref[n]), n
+    # the particles' charge leaves Q the same way (the solve is a few sweeps)
+    opts = abi.poisson_options(step_interval=1, accuracy=1e-300, maximum_iterations=4)
+    g.poisson_correction(1, opts)
+    ref = f.copy()
+    oracle.poisson_correction(ref, b, 1, opts)
+    out = g.fields(f)
+    for n in ("Q", "Psi", "Ez", "Er"):
+        assert np.array_equal(out[n], ref[n]), n
