@@ -57,6 +57,14 @@ struct Poisson64Work {
   int sor_grid = 0;
   size_t part_n = 0;
   double *crow = nullptr, *drow = nullptr;
+  // the SOR with bands of rows in shared memory (band_kernel null: the mesh
+  // does not fit): its grid, rows a band, half-row length, update rows, and
+  // the driving term in the bands' order, exchange rows and barrier words
+  const void *band_kernel = nullptr;
+  int band_grid = 0, band_R = 0, band_H = 0, band_lo = 0, band_hi = 0;
+  size_t band_smem = 0;
+  double *band_mem = nullptr, *band_xb = nullptr;
+  unsigned long long *band_bar = nullptr;
 };
 struct PoissonHostOptions {
   double accuracy, error_charge_threshold;

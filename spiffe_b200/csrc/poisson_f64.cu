@@ -15,6 +15,8 @@
 // rounding distance of the threshold.  Built with -fmad=false.
 #include "modules.cuh"
 
+#include <algorithm>
+
 #include <cooperative_groups.h>
 
 namespace {
@@ -398,6 +400,276 @@ __global__ void __launch_bounds__(RT) k_sor(DevMesh m, SorArgs s, DevCounts *cnt
   }
 }
 
+// ---- the same SOR with its rows in shared memory
+//
+// k_sor reads Psi through L2 and a half-sweep of it costs 16.9 us on the
+// 3001 x 821 gun (4.7 us on a mesh a hundredth its size): the barrier of 592
+// blocks and the L2 latencies between two of them.  Here each SM holds a band
+// of rows of Psi in shared memory for the whole solve, one CTA an SM, and
+// half a row crosses to each neighbour after a half-sweep.  A row lies as its
+// even columns and then its odd ones, so that the nodes of one colour are
+// consecutive; the driving term is kept in that order too (rs), and a
+// half-sweep's part of it is loaded while the CTA waits at the barrier.  The
+// arithmetic of a node is k_sor's, operation by operation, the division by
+// the constant diagonal with a product and four fused corrections
+// (div_const), so Psi has the same bits; the stop sum is again formed in one
+// fixed order by every CTA.  Measured a half-sweep (B200; random charge / a
+// bunch's): 3001 x 821 8.3 / 10.1 us, 1501 x 1001 5.9 / 7.0, 1201 x 329 (8.5
+// before) 3.9 / 4.3, 301 x 83 3.2: about 3 of it the barrier with the sums
+// and the exchange, the rest instruction issue (FP64 without contraction).
+// 1024 threads spilled their prefetched driving terms (8.7 / 12.8), 512 had
+// too few warps (11.7 / 17.9), a barrier of one tagged word a band in place of
+// the counter cost 3 us more.
+constexpr int SB_NT = 768; // threads of a CTA
+
+struct SorBand {
+  int R, H;           // rows of a band; half-row length (doubles)
+  double inv_e, inv_e2c;
+  double *rs;         // driving term [rows][2][H]
+  double *xb;         // [2][G][2][H]: updated halves of the bands' first and last rows
+  unsigned long long *bar; // [0] arrivals, [16] abort
+};
+
+// x / e, correctly rounded, for e whose correctly rounded reciprocal is y:
+// Markstein's theorem (IBM J. Res. Dev. 34, 1990): a quotient within one unit
+// in the last place plus its exactly formed remainder times y rounds to the
+// quotient; the first correction brings x*y within that unit.
+__device__ __forceinline__ double div_const(double x, double e, double y)
+{
+  double q = x * y;
+  q = __fma_rn(__fma_rn(-q, e, x), y, q);
+  return __fma_rn(__fma_rn(-q, e, x), y, q);
+}
+
+// Whether x lies outside the range in which div_const's remainders are exact
+// (below 2^-940 or above 2^900; x = 0 is inside), by its exponent.
+__device__ __forceinline__ bool div_rare(double x)
+{
+  const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  return h - (83u << 20) >= (1840u << 20) && (h | (unsigned)__double2loint(x)) != 0;
+}
+
+// x / e there: a tiny x is scaled by a power of two first; that rounds a
+// subnormal quotient a second time, which can only matter where the scaled
+// one lies half way between two of them.  There, and for infinities and NaN,
+// the division.
+__device__ double div_scaled(double x, double e, double y)
+{
+  const double w = div_const(x * 0x1p500, e, y), q = w * 0x1p-500;
+  return !(fabs(x) < 0x1p-900) || fabs(w - q * 0x1p500) == 0x1p-575 ? x / e : q;
+}
+
+// RK: rows of a band that a thread takes, at most
+template <int RK>
+__global__ void __launch_bounds__(SB_NT, 1) k_sor_band(DevMesh m, SorArgs s, SorBand sb, DevCounts *cnt)
+{
+  extern __shared__ double2 sb_smem[];
+  __shared__ double sh[SB_NT / 32];
+  __shared__ double total_sh;
+  __shared__ int ok_sh;
+  if (s.st && !s.st->do_solve)
+    return;
+  double *S = reinterpret_cast<double *>(sb_smem);
+  const int nz = m.nz, nr = m.nr, P = m.pitch, H = sb.H, G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
+  const int lo = m.left_bc == SPIFFE_DIRICHLET ? 0 : 1, hi = m.right_bc == SPIFFE_DIRICHLET ? nz - 1 : nz - 2;
+  const int cols = nr - 1, first = lo + b * sb.R, nrow = min(sb.R, hi + 1 - first);
+  double *C = S + (size_t)(sb.R + 2) * 2 * H, *D = C + 2 * H; // c and d of each column, in a row's order
+  // this thread's columns: nodes j, j+1 of each half row, in rows g, g+groups, ...
+  const int W = ((((cols + 1) >> 1) + 1) / 2 + 31) & ~31, groups = SB_NT / W, g = tid / W, j = 2 * (tid - g * W);
+  const bool on = g < groups && 2 * j < cols;
+  // rows first-1 .. first+nrow of Psi and the band's rows of the driving term
+  for (int k = tid; k < (nrow + 2) * (nr + 1); k += SB_NT) {
+    const int r = k / (nr + 1), ir = k - r * (nr + 1), iz = first - 1 + r;
+    S[(size_t)r * 2 * H + (ir & 1) * H + (ir >> 1)] = iz >= 0 && iz <= nz ? s.Psi[node(iz, ir, P)] : 0.0;
+  }
+  for (int ir = tid; ir < 2 * H; ir += SB_NT) {
+    const bool in = ir < cols;
+    C[(ir & 1) * H + (ir >> 1)] = in ? (ir ? s.crow[ir] : s.c4_axis) : 0.0;
+    D[(ir & 1) * H + (ir >> 1)] = in && ir ? s.drow[ir] : 0.0;
+  }
+  double *rs = sb.rs + (size_t)b * sb.R * 2 * H;
+  for (int k = tid; k < nrow * cols; k += SB_NT) {
+    const int r = k / cols, ir = k - r * cols;
+    rs[(size_t)r * 2 * H + (ir & 1) * H + (ir >> 1)] = s.rhs ? s.rhs[node(first + r, ir, P)] : 0.0;
+  }
+  // which of the thread's nodes are updated: bits 4k + 2 half + q
+  unsigned upd = 0;
+  if (on)
+    for (int k = 0; k < RK; k++)
+      for (int t = 0; t < 4; t++) {
+        const int ir = 2 * (j + (t & 1)) + (t >> 1), r = g + k * groups;
+        if (ir < cols && r < nrow && !(s.flags[node(first + r, ir, P)] & SPIFFE_FL_IS_METAL))
+          upd |= 1u << (4 * k + t);
+      }
+  const double a = s.a, e = s.e, y = sb.inv_e, thr = s.accuracy * *s.driving;
+  double2 rh[RK]; // the coming half-sweep's driving terms
+  auto load_rh = [&](int colour) {
+#pragma unroll
+    for (int k = 0; k < RK; k++) {
+      const int r = g + k * groups;
+      if (on && r < nrow)
+        rh[k] = __ldcg(reinterpret_cast<const double2 *>(rs + (size_t)r * 2 * H + ((colour + first + r) & 1) * H + j));
+    }
+  };
+  __syncthreads();
+  load_rh(0);
+  long long result = -1;
+  double total = 0;
+  for (long long n = 0; n < s.limit; n++) {
+    const double omega = __ldg(s.omega + n);
+    const int colour = (int)(n & 1);
+    double acc = 0;
+    if (on)
+#pragma unroll
+      for (int k = 0; k < RK; k++) {
+        const int r = g + k * groups;
+        if (r < nrow) {
+          const int iz = first + r, h = (colour + iz) & 1; // the colour's columns have parity h
+          double *row = S + (size_t)(r + 1) * 2 * H, *x = row + h * H + j;
+          // the left and right Dirichlet rows mirror their only neighbour (poisson.c:369-375, :404-410)
+          const double *up = (iz == nz - 1 && hi == nz - 1) ? x - 2 * H : x + 2 * H;
+          const double *dn = (iz == 0 && lo == 0) ? x + 2 * H : x - 2 * H;
+          const double2 l = *reinterpret_cast<const double2 *>(up), q = *reinterpret_cast<const double2 *>(dn);
+          const double2 o = *reinterpret_cast<const double2 *>(row + (1 - h) * H + j);
+          const double2 c = *reinterpret_cast<const double2 *>(C + h * H + j), d = *reinterpret_cast<const double2 *>(D + h * H + j);
+          double2 v = *reinterpret_cast<const double2 *>(x);
+          const unsigned bits = upd >> (4 * k + 2 * h);
+          double rx, ry, ex = e, yx = y;
+          if (h) { // (the same for the whole warp)
+            rx = a * (l.x + q.x) + c.x * o.y + d.x * o.x + e * v.x - rh[k].x;
+            ry = a * (l.y + q.y) + c.y * row[j + 2] + d.y * o.y + e * v.y - rh[k].y;
+          } else {
+            if (j == 0) { // the axis, whose d is 0
+              ex = s.e2c_axis;
+              yx = sb.inv_e2c;
+            }
+            rx = a * (l.x + q.x) + c.x * o.x + d.x * (j ? row[H + j - 1] : 0.0) + ex * v.x - rh[k].x;
+            ry = a * (l.y + q.y) + c.y * o.y + d.y * o.x + e * v.y - rh[k].y;
+          }
+          const double tx = omega * rx, ty = omega * ry;
+          double qx = div_const(tx, ex, yx), qy = div_const(ty, e, y);
+          if (div_rare(tx) || div_rare(ty)) {
+            if (div_rare(tx))
+              qx = div_scaled(tx, ex, yx);
+            if (div_rare(ty))
+              qy = div_scaled(ty, e, y);
+          }
+          if (bits & 1u) {
+            v.x -= qx;
+            acc += fabs(rx);
+          }
+          if (bits & 2u) {
+            v.y -= qy;
+            acc += fabs(ry);
+          }
+          *reinterpret_cast<double2 *>(x) = v;
+          double *xo = sb.xb + ((size_t)colour * G + b) * 2 * H + j;
+          if (r == 0)
+            __stcg(reinterpret_cast<double2 *>(xo), v);
+          if (r == nrow - 1)
+            __stcg(reinterpret_cast<double2 *>(xo + H), v);
+        }
+      }
+    // the next half-sweep's driving terms arrive while the CTA waits
+    load_rh(1 - colour);
+    for (int o = 16; o > 0; o >>= 1)
+      acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if ((tid & 31) == 0)
+      sh[tid >> 5] = acc;
+    __syncthreads();
+    // the sums alternate between two halves of the buffer, so a CTA that runs
+    // ahead cannot overwrite sums another is still reading
+    double *part = s.partials + (size_t)colour * G;
+    if (tid < 32) {
+      double v = tid < SB_NT / 32 ? sh[tid] : 0.0;
+      for (int o = 16; o > 0; o >>= 1)
+        v += __shfl_down_sync(0xffffffffu, v, o);
+      if (tid == 0) {
+        __stcg(part + b, v);
+        int ok = 1;
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(sb.bar), "l"(1ull) : "memory");
+        const unsigned long long target = (unsigned long long)G * (unsigned long long)(n + 1);
+        unsigned long long polls = 0, seen = 0, gone = 0;
+        for (;;) {
+          asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(sb.bar) : "memory");
+          if (seen >= target)
+            break;
+          if ((++polls & 63) == 0) // bounded: 2^24 polls, or another band has given up
+            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(gone) : "l"(sb.bar + 16) : "memory");
+          if (gone || polls > (1ull << 24)) {
+            if (!gone) {
+              atomicOr(&cnt->error, SPIFFE_DEV_ERR_BARRIER);
+              asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(sb.bar + 16), "l"(1ull) : "memory");
+            }
+            ok = 0;
+            break;
+          }
+        }
+        ok_sh = ok;
+      }
+    }
+    __syncthreads();
+    if (!ok_sh)
+      return;
+    if (tid >= SB_NT - 32) { // the last warp: every CTA forms the same sum of the partials
+      double v = 0;
+      for (int k = tid - (SB_NT - 32); k < G; k += 32)
+        v += __ldcg(part + k);
+      for (int o = 16; o > 0; o >>= 1)
+        v += __shfl_down_sync(0xffffffffu, v, o);
+      if (tid == SB_NT - 32)
+        total_sh = v;
+    } else { // the others: the neighbours' rows
+      const double *xi = sb.xb + (size_t)colour * G * 2 * H;
+      for (int k = 2 * tid; k < 2 * H; k += 2 * (SB_NT - 32)) {
+        const bool above = k >= H;
+        const int t = above ? k - H : k, nb = above ? b + 1 : b - 1, iz = above ? first + nrow : first - 1;
+        if (nb < 0 || nb >= G)
+          continue;
+        const double2 v = __ldcg(reinterpret_cast<const double2 *>(xi + (size_t)nb * 2 * H + (above ? 0 : H) + t));
+        *reinterpret_cast<double2 *>(S + (size_t)(above ? nrow + 1 : 0) * 2 * H + ((colour + iz) & 1) * H + t) = v;
+      }
+    }
+    __syncthreads();
+    total = total_sh;
+    if (n > 0 && (total < thr || total == 0)) {
+      result = n;
+      break;
+    }
+  }
+  for (int k = tid; k < nrow * cols; k += SB_NT) {
+    const int r = k / cols, ir = k - r * cols;
+    s.Psi[node(first + r, ir, P)] = S[(size_t)(r + 1) * 2 * H + (ir & 1) * H + (ir >> 1)];
+  }
+  if (b == 0 && tid == 0) {
+    if (s.iterations_out)
+      *s.iterations_out = result;
+    if (s.st) {
+      s.st->iterations = result;
+      s.st->residual = total;
+    }
+    cnt->sor_halfsweeps += result >= 0 ? result + 1 : s.limit;
+    cnt->sor_solves += 1;
+  }
+}
+
+// rows of a thread for bands of R rows (0: the mesh's rows are too wide)
+int sb_rows(int cols, int R)
+{
+  const int W = ((((cols + 1) >> 1) + 1) / 2 + 31) & ~31, groups = SB_NT / W;
+  return groups ? (R + groups - 1) / groups : 0;
+}
+
+const void *sb_kernel(int rows)
+{
+  return rows <= 2   ? (const void *)k_sor_band<2>
+         : rows <= 4 ? (const void *)k_sor_band<4>
+         : rows <= 7 ? (const void *)k_sor_band<7>
+         : rows <= 8 ? (const void *)k_sor_band<8>
+                     : nullptr;
+}
+
 // Ez, Er -= grad Psi (:288-326) with the FDTD boundary copies; one writer per node.
 __global__ void __launch_bounds__(BX *BY) k_subtract_gradient(DevMesh m, DevFields<double> f, const PcState *st)
 {
@@ -556,6 +828,34 @@ extern "C" int spiffe_poisson64_setup(const DevMesh *m, Poisson64Work *w, long l
     w->sor_grid = sms * (per > 0 ? per : 1);
     if ((size_t)(2 * w->sor_grid) > w->part_n)
       w->sor_grid = (int)(w->part_n / 2);
+    // bands in shared memory, where the mesh fits the SMs' and its rows a
+    // CTA's threads: about 4 million nodes (fewer of very long rows); beyond
+    // that k_sor, which has no such limit
+    int max_smem = 0;
+    cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    const int lo = m->left_bc == SPIFFE_DIRICHLET ? 0 : 1, hi = m->right_bc == SPIFFE_DIRICHLET ? nz - 1 : nz - 2;
+    const int rows = hi - lo + 1, H = ((nr + 2) / 2 + 1) / 2 * 2;
+    const int G = std::max(1, std::min(sms, rows / 2)), R = (rows + G - 1) / G, per_thread = sb_rows(nr - 1, R);
+    const void *k = per_thread ? sb_kernel(per_thread) : nullptr;
+    const size_t smem = (size_t)(R + 4) * 2 * H * sizeof(double);
+    cudaFuncAttributes fa{};
+    if (e == cudaSuccess && k && cudaFuncGetAttributes(&fa, k) == cudaSuccess && smem + fa.sharedSizeBytes <= (size_t)max_smem) {
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes);
+      const int used = (rows + R - 1) / R;
+      const size_t rs = (size_t)rows * 2 * H, xb = (size_t)4 * used * H;
+      if (e == cudaSuccess) e = cudaMalloc(&w->band_mem, (rs + xb) * sizeof(double) + 32 * sizeof(unsigned long long));
+      if (e == cudaSuccess) {
+        w->band_kernel = k;
+        w->band_grid = used;
+        w->band_R = R;
+        w->band_H = H;
+        w->band_lo = lo;
+        w->band_hi = hi;
+        w->band_smem = smem;
+        w->band_xb = w->band_mem + rs;
+        w->band_bar = (unsigned long long *)(w->band_xb + xb);
+      }
+    }
   }
   return (int)e;
 }
@@ -574,6 +874,7 @@ extern "C" void spiffe_poisson64_free(Poisson64Work *w)
   cudaFree(w->iters);
   cudaFree(w->crow);
   cudaFree(w->drow);
+  cudaFree(w->band_mem);
   *w = Poisson64Work();
 }
 
@@ -649,8 +950,21 @@ static int launch_sor(const DevMesh *m, Poisson64Work *w, double *Psi, const dou
   a.st = st;
   a.iterations_out = iters;
   DevMesh mm = *m;
-  void *args[] = {&mm, &a, &cnt};
-  cudaError_t e = cudaLaunchCooperativeKernel((void *)k_sor, dim3(w->sor_grid), dim3(RT), args, 0, s);
+  cudaError_t e;
+  // (end conditions set after the set-up move the update rows: the bands
+  // follow those they were laid out for)
+  const int lo = m->left_bc == SPIFFE_DIRICHLET ? 0 : 1, hi = m->right_bc == SPIFFE_DIRICHLET ? m->nz - 1 : m->nz - 2;
+  if (w->band_kernel && lo == w->band_lo && hi == w->band_hi) {
+    SorBand sb{w->band_R, w->band_H, 1 / a.e, 1 / a.e2c_axis, w->band_mem, w->band_xb, w->band_bar};
+    e = cudaMemsetAsync(w->band_bar, 0, 32 * sizeof(unsigned long long), s);
+    if (e != cudaSuccess)
+      return (int)e;
+    void *args[] = {&mm, &a, &sb, &cnt};
+    e = cudaLaunchCooperativeKernel(w->band_kernel, dim3(w->band_grid), dim3(SB_NT), args, w->band_smem, s);
+  } else {
+    void *args[] = {&mm, &a, &cnt};
+    e = cudaLaunchCooperativeKernel((void *)k_sor, dim3(w->sor_grid), dim3(RT), args, 0, s);
+  }
   spiffe_note_launches(1);
   return (int)e;
 }

@@ -1,10 +1,12 @@
-"""The FP64 form's ordered reduction at the sizes where it can go wrong, bit
-for bit against the CPU checker.
+"""The FP64 form's ordered reduction and banded SOR at the sizes where they
+can go wrong, bit for bit against the CPU checker.
 
 * The ordered deposition and charge removal sum each node's particles in
   particle order; the kernel takes 32 entries a warp and follows a run that
   goes on behind them 32 at a time, so runs of 1, 31, 32, 33, ... entries at
   every offset, and meshes with one, two and four entries a particle.
+* The SOR with its rows in shared memory: bands of two rows and of many, the
+  narrowest meshes, rows of one and of several warps, and both kinds of ends.
 """
 import numpy as np
 import pytest
@@ -63,3 +65,44 @@ def test_ordered_sums_in_particle_order(oracle, counts, smear):
     out = g.fields(f)
     for n in ("Q", "Psi", "Ez", "Er"):
         assert np.array_equal(out[n], ref[n]), n
+
+
+@pytest.mark.parametrize("ends", [(abi.NEUMANN, abi.NEUMANN), (abi.DIRICHLET, abi.DIRICHLET),
+                                  (abi.NEUMANN, abi.DIRICHLET)])
+@pytest.mark.parametrize("nz, nr", [(6, 5), (7, 6), (40, 9), (41, 66), (300, 67), (307, 34), (90, 259), (700, 130),
+                                    (24, 1030), (601, 321)])
+def test_sor_is_the_serial_iteration(oracle, nz, nr, ends):
+    f = pillbox(nz, nr, left_bc=ends[0], right_bc=ends[1])
+    rng = np.random.default_rng(nz * 1000 + nr)
+    f["Q"] = rng.normal(size=f.shape) * 1e6
+    f["Psi"] = np.where(rng.uniform(size=f.shape) < 0.5, 0.0, rng.normal(size=f.shape))
+    g = gpu.GpuInstance(f)
+    for limit in (2, 37):  # exactly this many half-sweeps
+        g.upload_fields(f)
+        assert g.solve_poisson(0, 1e-300, limit) == -1
+        ref = f.copy()
+        n, _, _ = oracle.solve_poisson(ref, ref["Psi"], ref["Q"], 1e-300, limit)
+        assert n == -1 and np.array_equal(g.fields(f)["Psi"], ref["Psi"]), limit
+    g.upload_fields(f)
+    n = g.solve_poisson(0, 0.2, 500)  # the stop rule inside the run
+    ref = f.copy()
+    m, _, _ = oracle.solve_poisson(ref, ref["Psi"], ref["Q"], 0.2, 500)
+    assert n == m and np.array_equal(g.fields(f)["Psi"], ref["Psi"])
+
+
+def test_sor_follows_ends_set_after_setup(oracle):
+    """set_mesh may change the end conditions, and with them the update rows."""
+    f = pillbox(60, 40)
+    f["Q"] = np.random.default_rng(4).normal(size=f.shape) * 1e6
+    g = gpu.GpuInstance(f)
+    g.solve_poisson(0, 1e-300, 4)
+    fd = f.copy()
+    fd.mesh.left_bc = abi.DIRICHLET
+    m = g.get_mesh()
+    m.left_bc = abi.DIRICHLET
+    g.set_mesh(m)
+    g.upload_fields(fd)
+    g.solve_poisson(0, 1e-300, 20)
+    ref = fd.copy()
+    oracle.solve_poisson(ref, ref["Psi"], ref["Q"], 1e-300, 20)
+    assert np.array_equal(g.fields(fd)["Psi"], ref["Psi"])
