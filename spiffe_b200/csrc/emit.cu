@@ -16,7 +16,20 @@ namespace {
 
 constexpr int T = 256;
 
-__global__ void __launch_bounds__(T) k_births(DevMesh m, DevFields<double> f, DevBeam64 b, BirthParams p, DevCounts *cnt)
+__device__ __forceinline__ void births_commit(long long total, long long capacity, int mode, DevCounts *cnt)
+{
+  if (cnt->np + total > capacity)
+    return;
+  cnt->np += total;
+  if (mode == SPIFFE_BIRTH_TEST) // inactive and without an ID, test_beam.c:104
+    return;
+  cnt->npActive += total;
+  if (mode != SPIFFE_BIRTH_LIST) // listed particles carry the IDs given at their queueing
+    cnt->nextParticleID += total;
+}
+
+__device__ __forceinline__ void birth(const DevMesh &m, const DevFields<double> &f, const DevBeam64 &b,
+                                      const BirthParams &p, DevCounts *cnt)
 {
   const long long k = (long long)blockIdx.x * T + threadIdx.x;
   if (k >= p.total)
@@ -145,16 +158,19 @@ __global__ void __launch_bounds__(T) k_births(DevMesh m, DevFields<double> f, De
   b.status[ip] = SPIFFE_PART_ACTIVE;
 }
 
+__global__ void __launch_bounds__(T) k_births(DevMesh m, DevFields<double> f, DevBeam64 b, BirthParams p, DevCounts *cnt)
+{
+  birth(m, f, b, p, cnt);
+  if (gridDim.x == 1) { // the births of one block (most emissions): it commits them itself
+    __syncthreads();
+    if (threadIdx.x == 0)
+      births_commit(p.total, b.capacity, p.mode, cnt);
+  }
+}
+
 __global__ void k_births_commit(long long total, long long capacity, int mode, DevCounts *cnt)
 {
-  if (cnt->np + total > capacity)
-    return;
-  cnt->np += total;
-  if (mode == SPIFFE_BIRTH_TEST) // inactive and without an ID, test_beam.c:104
-    return;
-  cnt->npActive += total;
-  if (mode != SPIFFE_BIRTH_LIST) // listed particles carry the IDs given at their queueing
-    cnt->nextParticleID += total;
+  births_commit(total, capacity, mode, cnt);
 }
 
 __global__ void k_antenna(double *J, int P, int direction, long istart, long iend, long iposition, double value)
@@ -176,10 +192,11 @@ extern "C" int spiffe_births64(const DevMesh *m, const DevFields<double> *f, con
 {
   if (p->total <= 0)
     return 0;
-  k_births<<<blocks_for(p->total, T), T, 0, s>>>(*m, *f, *b, *p, cnt);
-  spiffe_note_launches(1);
-  k_births_commit<<<1, 1, 0, s>>>(p->total, b->capacity, p->mode, cnt);
-  spiffe_note_launches(1);
+  const unsigned nb = blocks_for(p->total, T);
+  k_births<<<nb, T, 0, s>>>(*m, *f, *b, *p, cnt);
+  if (nb > 1)
+    k_births_commit<<<1, 1, 0, s>>>(p->total, b->capacity, p->mode, cnt);
+  spiffe_note_launches(nb > 1 ? 2 : 1);
   return (int)cudaGetLastError();
 }
 

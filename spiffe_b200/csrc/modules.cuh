@@ -16,12 +16,13 @@ extern "C" int spiffe_fdtd64_step(const DevMesh *m, const DevFields<double> *f, 
 
 struct Particles64Work {
   uint8_t *lost = nullptr;
-  int *surv = nullptr, *surv_before = nullptr, *map = nullptr;
+  int *lost_list = nullptr, *holes = nullptr, *donors = nullptr;
   int *keys = nullptr, *keys_alt = nullptr;
   double *vals = nullptr, *vals_alt = nullptr;
   void *cub_tmp = nullptr;
   size_t cub_bytes = 0;
   long long capacity = 0;
+  bool met_none = false; // the last push left the on-axis extremes at (+inf, -inf)
 };
 extern "C" int spiffe_particles64_work(Particles64Work *w, long long capacity, bool ordered);
 extern "C" void spiffe_particles64_work_free(Particles64Work *w);

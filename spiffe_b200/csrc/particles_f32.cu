@@ -23,7 +23,7 @@
 
 #include <cfloat>
 
-#include <cub/block/block_radix_sort.cuh>
+#include "compact.cuh"
 
 namespace {
 
@@ -891,25 +891,18 @@ __global__ void k_lost32(DevMesh m, const int16_t *fl, DevBeam32 b, LostLog L)
 
 // ---- compaction
 
-__global__ void k_reset_step_counts32(DevCounts *cnt)
+// The on-axis fields' extremes of the coming push (advance_particles.c:113-114)
+__global__ void k_reset_onaxis32(DevCounts *cnt)
 {
-  cnt->first_lost = 0x7fffffffffffffffLL;
-  cnt->n_lost = 0;
-  cnt->new_active = 0;
-  cnt->pushed += cnt->npActive;
-  cnt->oa_min = INFINITY; // HUGE, advance_particles.c:113-114
+  cnt->oa_min = INFINITY; // HUGE
   cnt->oa_max = -INFINITY;
 }
 
 // The reference's removal: the first lost index ends the beam (:490-518 as released).
-__global__ void k_compact_reference32(DevCounts *cnt)
+__global__ void k_compact_reference32(DevCounts *cnt, int oa)
 {
-  const long long np = cnt->np;
-  cnt->npActive += cnt->new_active;
-  if (cnt->n_lost && cnt->first_lost < np) {
-    cnt->npActive -= np - cnt->first_lost;
-    cnt->np = cnt->first_lost;
-  }
+  const bool cut = cnt->n_lost && cnt->first_lost < cnt->np;
+  end_push(cnt, cut ? cnt->np - cnt->first_lost : 0, cut ? cnt->first_lost : cnt->np, oa);
 }
 
 __device__ __forceinline__ void move32(const DevBeam32 &b, long dst, long src)
@@ -933,101 +926,18 @@ __device__ __forceinline__ void move32(const DevBeam32 &b, long dst, long src)
   b.generation[dst] = b.generation[src];
 }
 
-// Removes exactly the lost particles (order not kept): the lost slots below
-// the new count are refilled from the survivors above it, the k-th hole in
-// ascending index order from the k-th survivor in ascending order, so the
-// result does not depend on the order the push appended the losses (which
-// follows the timing of its blocks).  One block; the lists are built with
-// block-wide prefix counts in chunks; the holes, collected from the push's
-// list, are put in order by a block radix sort when there are at most
-// CT * CT_ITEMS of them, else collected again by a scan of the statuses.
-constexpr int CT = 1024, CT_ITEMS = 4;
+// Removes exactly the lost particles (order not kept).
 __global__ void __launch_bounds__(CT) k_compact_any32(DevBeam32 b, const int32_t *lost_list, DevCounts *cnt,
-                                                       int32_t *holes, int32_t *donors)
+                                                       int32_t *holes, int32_t *donors, int oa)
 {
-  __shared__ int warp_tot[CT / 32];
-  __shared__ int base_sh, n_holes_sh;
-  typedef cub::BlockRadixSort<int, CT, CT_ITEMS> HoleSort;
-  __shared__ typename HoleSort::TempStorage sort_tmp;
-  const long long n_lost = cnt->n_lost, np = cnt->np, new_np = np - n_lost;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (n_lost > 0) {
-    // list 0: holes (lost slots < new_np) from the push's list; list 1:
-    // donors (survivors >= new_np) in index order; list 2: holes again, in
-    // index order, from the statuses (only when too many to sort)
-    for (int list = 0; list < 3; list++) {
-      if (list == 2 && n_holes_sh <= CT * CT_ITEMS)
-        break;
-      if (tid == 0)
-        base_sh = 0;
-      __syncthreads();
-      const long long span = list == 2 ? new_np : n_lost;
-      for (long long c0 = 0; c0 < span; c0 += CT) {
-        const long long i = c0 + tid;
-        bool take = false;
-        int val = 0;
-        if (i < span) {
-          if (list == 0) {
-            val = lost_list[i];
-            take = val < new_np;
-          } else if (list == 1) {
-            val = (int)(new_np + i);
-            take = !(b.status[val] & S32_LOST);
-          } else {
-            val = (int)i;
-            take = b.status[val] & S32_LOST;
-          }
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, take);
-        if (lane == 0)
-          warp_tot[wid] = __popc(bal);
-        __syncthreads();
-        int before = 0, total = 0;
-        for (int w = 0; w < CT / 32; w++) {
-          before += w < wid ? warp_tot[w] : 0;
-          total += warp_tot[w];
-        }
-        const int base = base_sh;
-        if (take)
-          (list == 1 ? donors : holes)[base + before + __popc(bal & ((1u << lane) - 1))] = val;
-        __syncthreads();
-        if (tid == 0)
-          base_sh = base + total;
-        __syncthreads();
-      }
-      if (list == 0) {
-        if (tid == 0)
-          n_holes_sh = base_sh;
-        __syncthreads();
-        const int nh = n_holes_sh;
-        if (nh <= CT * CT_ITEMS) {
-          // the holes in ascending order (INT_MAX pads sort last)
-          int k[CT_ITEMS];
-#pragma unroll
-          for (int q = 0; q < CT_ITEMS; q++) {
-            const int at = tid * CT_ITEMS + q;
-            k[q] = at < nh ? holes[at] : 0x7fffffff;
-          }
-          HoleSort(sort_tmp).Sort(k);
-#pragma unroll
-          for (int q = 0; q < CT_ITEMS; q++) {
-            const int at = tid * CT_ITEMS + q;
-            if (at < nh)
-              holes[at] = k[q];
-          }
-          __syncthreads();
-        }
-      }
-    }
-    const int n_move = base_sh; // equal counts: every hole has a donor
-    for (int k = tid; k < n_move; k += CT)
-      move32(b, holes[k], donors[k]);
-  }
+  const long long n_lost = cnt->n_lost, np = cnt->np;
+  if (n_lost > 0)
+    compact_block<false>(
+        n_lost, np, lost_list, holes, donors, [&](int i) { return (b.status[i] & S32_LOST) != 0; },
+        [&](int dst, int src) { move32(b, dst, src); });
   __syncthreads();
-  if (tid == 0) {
-    cnt->npActive += cnt->new_active - n_lost;
-    cnt->np = new_np;
-  }
+  if (threadIdx.x == 0)
+    end_push(cnt, n_lost, np - n_lost, oa);
 }
 
 // ---- cell sort
@@ -1101,6 +1011,18 @@ __global__ void k_permute(DevBeam32 dst, DevBeam32 src, const int32_t *idx, cons
 }
 
 // ---- births (cathode.c:464-659) into the split beam
+
+__device__ __forceinline__ void births_commit(long long total, long long capacity, int mode, DevCounts *cnt)
+{
+  if (cnt->np + total > capacity)
+    return;
+  cnt->np += total;
+  if (mode == SPIFFE_BIRTH_TEST) // inactive and without an ID, test_beam.c:104
+    return;
+  cnt->npActive += total;
+  if (mode != SPIFFE_BIRTH_LIST) // listed particles carry the IDs given at their queueing
+    cnt->nextParticleID += total;
+}
 
 __global__ void __launch_bounds__(T) k_births32(DevMesh m, DevFields32 f, DevBeam32 b, BirthParams p, DevCounts *cnt,
                                                  S32Scales sc, int deposit)
@@ -1257,18 +1179,16 @@ __global__ void __launch_bounds__(T) k_births32(DevMesh m, DevFields32 f, DevBea
   }
   if (deposit)
     deposit_particle<false>(m, f, on && !test, iz, fz, ir, fr, bz, br, bphi, qs);
+  if (gridDim.x == 1) { // the births of one block (most emissions): it commits them itself
+    __syncthreads();
+    if (threadIdx.x == 0)
+      births_commit(p.total, b.capacity, p.mode, cnt);
+  }
 }
 
 __global__ void k_births_commit32(long long total, long long capacity, int mode, DevCounts *cnt)
 {
-  if (cnt->np + total > capacity)
-    return;
-  cnt->np += total;
-  if (mode == SPIFFE_BIRTH_TEST) // inactive and without an ID, test_beam.c:104
-    return;
-  cnt->npActive += total;
-  if (mode != SPIFFE_BIRTH_LIST) // listed particles carry the IDs given at their queueing
-    cnt->nextParticleID += total;
+  births_commit(total, capacity, mode, cnt);
 }
 
 // interpolateFields at n points (zr[2i], zr[2i+1]) of the split form's
@@ -1461,8 +1381,14 @@ extern "C" int s32_push(const DevMesh *m, const DevFields32 *f, const DevBeam32 
                         const DevScreens *scr, DevCounts *cnt, long long np_bound, int compaction,
                         const S32Scales *sc, Particles32Work *w, cudaStream_t s)
 {
-  k_reset_step_counts32<<<1, 1, 0, s>>>(cnt);
-  spiffe_note_launches(1);
+  if (m->n_onaxis) {
+    k_reset_onaxis32<<<1, 1, 0, s>>>(cnt);
+    spiffe_note_launches(1);
+  }
+  const int oa = !m->n_onaxis;
+  if (np_bound <= 0 && oa && w->met_none)
+    return 0; // no particle, and nothing to reset: an empty push changes no count
+  w->met_none = oa;
   const bool any = compaction != SPIFFE_COMPACT_REFERENCE;
   if (np_bound > 0) {
     if (scr->n && p->screen_momentum == SPIFFE_SCREEN_REFERENCE) {
@@ -1493,9 +1419,9 @@ extern "C" int s32_push(const DevMesh *m, const DevFields32 *f, const DevBeam32 
     }
   }
   if (!any) {
-    k_compact_reference32<<<1, 1, 0, s>>>(cnt);
+    k_compact_reference32<<<1, 1, 0, s>>>(cnt, oa);
   } else {
-    k_compact_any32<<<1, CT, 0, s>>>(*b, w->lost_list, cnt, w->keys, w->idx);
+    k_compact_any32<<<1, CT, 0, s>>>(*b, w->lost_list, cnt, w->keys, w->idx, oa);
   }
   spiffe_note_launches(1);
   return (int)cudaGetLastError();
@@ -1534,9 +1460,11 @@ extern "C" int s32_births(const DevMesh *m, const DevFields32 *f, const DevBeam3
 {
   if (p->total <= 0)
     return 0;
-  k_births32<<<blocks_for(p->total, T), T, 0, s>>>(*m, *f, *b, *p, cnt, *sc, deposit);
-  k_births_commit32<<<1, 1, 0, s>>>(p->total, b->capacity, p->mode, cnt);
-  spiffe_note_launches(2);
+  const unsigned nb = blocks_for(p->total, T);
+  k_births32<<<nb, T, 0, s>>>(*m, *f, *b, *p, cnt, *sc, deposit);
+  if (nb > 1)
+    k_births_commit32<<<1, 1, 0, s>>>(p->total, b->capacity, p->mode, cnt);
+  spiffe_note_launches(nb > 1 ? 2 : 1);
   return (int)cudaGetLastError();
 }
 

@@ -11,6 +11,8 @@
 // ordered mode, in particle order exactly as the serial reference does.
 #include "modules.cuh"
 
+#include "compact.cuh"
+
 namespace {
 
 constexpr int T = 256;
@@ -273,7 +275,7 @@ __global__ void k_snapshot_last(DevBeam64 b, DevCounts *cnt)
 
 // advance_particles' per-particle loop (:131-339) and screen loop (:362-434).
 __global__ void __launch_bounds__(T) k_push(DevMesh m, DevFields<double> f, DevBeam64 b, PushParams p,
-                                             DevScreens scr, DevCounts *cnt, uint8_t *lost_flag)
+                                             DevScreens scr, DevCounts *cnt, uint8_t *lost_flag, int32_t *lost_list)
 {
   const long ip = (long)blockIdx.x * T + threadIdx.x;
   const long np = (long)cnt->np;
@@ -411,8 +413,9 @@ __global__ void __launch_bounds__(T) k_push(DevMesh m, DevFields<double> f, DevB
   if (lost) {
     status &= ~SPIFFE_PART_ACTIVE;
     status |= SPIFFE_PART_LOST;
-    atomic_add_ll(&cnt->n_lost, 1LL);
+    const long long slot = atomic_add_ll(&cnt->n_lost, 1LL);
     atomicMin(&cnt->first_lost, (long long)ip);
+    lost_list[slot] = (int32_t)ip;
   }
   b.status[ip] = status;
   lost_flag[ip] = lost ? 1 : 0;
@@ -802,63 +805,33 @@ __global__ void __launch_bounds__(T) k_ordered_sum(const int *keys, const double
   } while (0)
 
 // Reference compaction: the first lost index ends the beam.
-__global__ void k_compact_reference(DevCounts *cnt)
+__global__ void k_compact_reference(DevCounts *cnt, int oa)
 {
-  const long long np = cnt->np;
-  cnt->npActive += cnt->new_active;
-  if (cnt->n_lost && cnt->first_lost < np) {
-    cnt->npActive -= np - cnt->first_lost;
-    cnt->np = cnt->first_lost;
-  }
+  const bool cut = cnt->n_lost && cnt->first_lost < cnt->np;
+  end_push(cnt, cut ? cnt->np - cnt->first_lost : 0, cut ? cnt->first_lost : cnt->np, oa);
 }
 
 // Swap compaction: survivors at the end refill lost slots at the front, the
 // j-th lost slot (ascending) taking the j-th survivor counted from the end.
-// surv_before[] is an exclusive prefix count of survivors over [0, np).
-__global__ void k_compact_swap_map(const uint8_t *lost, const int *surv_before, const DevCounts *cnt, int *map)
+// One block in one launch, where flags, a scan, a map and the moves took six
+// (3.9 us each of launching, the whole step of a small problem).
+__global__ void __launch_bounds__(CT) k_compact_swap(DevBeam64 b, const uint8_t *lost, const int32_t *lost_list,
+                                                      DevCounts *cnt, int32_t *holes, int32_t *donors, int oa)
 {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long np = cnt->np, n_lost = cnt->n_lost, new_np = np - n_lost;
-  if (i >= np || !n_lost)
-    return;
-  if (i >= new_np && !lost[i]) {
-    const long long d = new_np - surv_before[i] - 1; // descending rank among tail survivors
-    map[d] = (int)i;
-  }
+  const long long n_lost = cnt->n_lost, np = cnt->np;
+  if (n_lost > 0)
+    compact_block<true>(
+        n_lost, np, lost_list, holes, donors, [&](int i) { return lost[i] != 0; },
+        [&](int dst, int src) { MOVE_ALL(dst, src); });
+  __syncthreads();
+  if (threadIdx.x == 0)
+    end_push(cnt, n_lost, np - n_lost, oa);
 }
 
-__global__ void k_compact_swap_move(DevBeam64 b, const uint8_t *lost, const int *surv_before, const DevCounts *cnt,
-                                    const int *map)
+// The on-axis fields' extremes of the coming push (advance_particles.c:113-114)
+__global__ void k_reset_onaxis(DevCounts *cnt)
 {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long np = cnt->np, n_lost = cnt->n_lost, new_np = np - n_lost;
-  if (i >= new_np || !n_lost || !lost[i])
-    return;
-  const long long a = i - surv_before[i]; // ascending rank among front lost slots
-  const int src = map[a];
-  MOVE_ALL(i, src);
-}
-
-__global__ void k_compact_swap_finish(DevCounts *cnt)
-{
-  cnt->npActive += cnt->new_active - cnt->n_lost;
-  cnt->np -= cnt->n_lost;
-}
-
-__global__ void k_survivor_flags(const uint8_t *lost, const DevCounts *cnt, int *surv, long long n)
-{
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n)
-    surv[i] = (i < cnt->np && !lost[i]) ? 1 : 0;
-}
-
-__global__ void k_reset_step_counts(DevCounts *cnt)
-{
-  cnt->first_lost = 0x7fffffffffffffffLL;
-  cnt->n_lost = 0;
-  cnt->new_active = 0;
-  cnt->pushed += cnt->npActive;
-  cnt->oa_min = INFINITY; // HUGE, advance_particles.c:113-114
+  cnt->oa_min = INFINITY; // HUGE
   cnt->oa_max = -INFINITY;
 }
 
@@ -867,7 +840,6 @@ __global__ void k_reset_step_counts(DevCounts *cnt)
 // ------------------------------------------------------------ host entry
 
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
 
 
 extern "C" int spiffe_particles64_work(Particles64Work *w, long long capacity, bool ordered)
@@ -875,9 +847,9 @@ extern "C" int spiffe_particles64_work(Particles64Work *w, long long capacity, b
   cudaError_t e = cudaSuccess;
   if (w->capacity < capacity) {
     cudaFree(w->lost);
-    cudaFree(w->surv);
-    cudaFree(w->surv_before);
-    cudaFree(w->map);
+    cudaFree(w->lost_list);
+    cudaFree(w->holes);
+    cudaFree(w->donors);
     cudaFree(w->keys);
     cudaFree(w->keys_alt);
     cudaFree(w->vals);
@@ -885,14 +857,13 @@ extern "C" int spiffe_particles64_work(Particles64Work *w, long long capacity, b
     cudaFree(w->cub_tmp);
     *w = Particles64Work();
     e = cudaMalloc(&w->lost, capacity + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&w->surv, sizeof(int) * (capacity + 16));
-    if (e == cudaSuccess) e = cudaMalloc(&w->surv_before, sizeof(int) * (capacity + 16));
-    if (e == cudaSuccess) e = cudaMalloc(&w->map, sizeof(int) * (capacity + 16));
-    size_t scan_bytes = 0, sort_bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, w->surv, w->surv_before, (int)capacity);
+    if (e == cudaSuccess) e = cudaMalloc(&w->lost_list, sizeof(int) * (capacity + 16));
+    if (e == cudaSuccess) e = cudaMalloc(&w->holes, sizeof(int) * (capacity + 16));
+    if (e == cudaSuccess) e = cudaMalloc(&w->donors, sizeof(int) * (capacity + 16));
+    size_t sort_bytes = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (int *)nullptr, (int *)nullptr, (double *)nullptr,
                                     (double *)nullptr, (int)(4 * capacity));
-    w->cub_bytes = scan_bytes > sort_bytes ? scan_bytes : sort_bytes;
+    w->cub_bytes = sort_bytes;
     if (e == cudaSuccess) e = cudaMalloc(&w->cub_tmp, w->cub_bytes);
     w->capacity = capacity;
   }
@@ -908,9 +879,9 @@ extern "C" int spiffe_particles64_work(Particles64Work *w, long long capacity, b
 extern "C" void spiffe_particles64_work_free(Particles64Work *w)
 {
   cudaFree(w->lost);
-  cudaFree(w->surv);
-  cudaFree(w->surv_before);
-  cudaFree(w->map);
+  cudaFree(w->lost_list);
+  cudaFree(w->holes);
+  cudaFree(w->donors);
   cudaFree(w->keys);
   cudaFree(w->keys_alt);
   cudaFree(w->vals);
@@ -997,31 +968,26 @@ extern "C" int spiffe_gather_points64(const DevMesh *m, const DevFields<double> 
 extern "C" int spiffe_push64(const DevMesh *m, const DevFields<double> *f, const DevBeam64 *b, const PushHostParams *hp,
                              const DevScreens *scr, DevCounts *cnt, long long np_bound, Particles64Work *w, cudaStream_t s)
 {
-  k_reset_step_counts<<<1, 1, 0, s>>>(cnt);
-  spiffe_note_launches(1);
+  if (m->n_onaxis) {
+    k_reset_onaxis<<<1, 1, 0, s>>>(cnt);
+    spiffe_note_launches(1);
+  }
+  const int oa = !m->n_onaxis;
+  if (np_bound <= 0 && oa && w->met_none)
+    return 0; // no particle, and nothing to reset: an empty push changes no count
+  w->met_none = oa;
   if (np_bound > 0) {
     PushParams p{hp->time, hp->z_forces_start, hp->QoMC, hp->stiffness, hp->tb_epm, hp->tb_z_force,
                  hp->tb_r_force, hp->tb_z_decel, hp->tb_r_decel, hp->screen_momentum, hp->lost};
     if (scr->n && hp->screen_momentum == SPIFFE_SCREEN_REFERENCE)
       { k_snapshot_last<<<1, 1, 0, s>>>(*b, cnt); spiffe_note_launches(1); }
-    k_push<<<blocks_for(np_bound, T), T, 0, s>>>(*m, *f, *b, p, *scr, cnt, w->lost);
+    k_push<<<blocks_for(np_bound, T), T, 0, s>>>(*m, *f, *b, p, *scr, cnt, w->lost, w->lost_list);
     spiffe_note_launches(1);
   }
-  if (hp->compaction == SPIFFE_COMPACT_REFERENCE || np_bound <= 0) {
-    k_compact_reference<<<1, 1, 0, s>>>(cnt);
-    spiffe_note_launches(1);
-  } else {
-    const unsigned nb = blocks_for(np_bound, T);
-    k_survivor_flags<<<nb, T, 0, s>>>(w->lost, cnt, w->surv, np_bound);
-    spiffe_note_launches(1);
-    size_t bytes = w->cub_bytes;
-    cub::DeviceScan::ExclusiveSum(w->cub_tmp, bytes, w->surv, w->surv_before, (int)np_bound, s);
-    k_compact_swap_map<<<nb, T, 0, s>>>(w->lost, w->surv_before, cnt, w->map);
-    spiffe_note_launches(1);
-    k_compact_swap_move<<<nb, T, 0, s>>>(*b, w->lost, w->surv_before, cnt, w->map);
-    spiffe_note_launches(1);
-    k_compact_swap_finish<<<1, 1, 0, s>>>(cnt);
-    spiffe_note_launches(1);
-  }
+  if (hp->compaction == SPIFFE_COMPACT_REFERENCE || np_bound <= 0)
+    k_compact_reference<<<1, 1, 0, s>>>(cnt, oa);
+  else
+    k_compact_swap<<<1, CT, 0, s>>>(*b, w->lost, w->lost_list, cnt, w->holes, w->donors, oa);
+  spiffe_note_launches(1);
   return (int)cudaGetLastError();
 }

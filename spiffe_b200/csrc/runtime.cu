@@ -213,6 +213,7 @@ struct spiffe_gpu_instance {
   DevMesh dm{};
   cudaStream_t stream = nullptr;
   size_t nodes = 0;
+  size_t j_stride = 0; // FP64: doubles from one component of J to the next
   std::vector<int16_t> h_flags;
   int16_t *d_flags = nullptr;
   DevFields<double> f{};
@@ -957,12 +958,19 @@ extern "C" int spiffe_gpu_create(const spiffe_mesh *mesh, const int16_t *flags, 
     return bail(fail(SPIFFE_ERR_NOMEM, "flag allocation failed"));
   DevFields<double> &f = in->f;
   f.flags = in->d_flags;
-  double **tm[] = {&f.Ez, &f.Er, &f.Bphi, &f.Bphi2, &f.Jz, &f.Jr, &f.EzImposed, &f.ErImposed, &f.PsiImposed, &f.Psi, &f.Q};
+  // Jz, Jr (and Jphi) are one array, cleared by one fill a step
+  const size_t pad = in->j_stride = (n + 31) & ~(size_t)31;
+  if ((rc = alloc_field(&f.Jz, (mesh->modes & SPIFFE_FL_TE_FIELDS ? 3 : 2) * pad, s)))
+    return bail(rc);
+  f.Jr = f.Jz + pad;
+  if (mesh->modes & SPIFFE_FL_TE_FIELDS)
+    f.Jphi = f.Jz + 2 * pad;
+  double **tm[] = {&f.Ez, &f.Er, &f.Bphi, &f.Bphi2, &f.EzImposed, &f.ErImposed, &f.PsiImposed, &f.Psi, &f.Q};
   for (double **p : tm)
     if ((rc = alloc_field(p, n, s)))
       return bail(rc);
   if (mesh->modes & SPIFFE_FL_TE_FIELDS) {
-    double **te[] = {&f.Ephi, &f.Jphi, &f.Br, &f.Br2, &f.Bz, &f.Bz2};
+    double **te[] = {&f.Ephi, &f.Br, &f.Br2, &f.Bz, &f.Bz2};
     for (double **p : te)
       if ((rc = alloc_field(p, n, s)))
         return bail(rc);
@@ -987,7 +995,7 @@ extern "C" int spiffe_gpu_destroy(spiffe_gpu_instance *in)
   if (in->s32)
     s32_destroy(in);
   DevFields<double> &f = in->f;
-  void *p[] = {f.Ez, f.Er, f.Bphi, f.Bphi2, f.Jz, f.Jr, f.Ephi, f.Jphi, f.Br, f.Br2, f.Bz, f.Bz2,
+  void *p[] = {f.Ez, f.Er, f.Bphi, f.Bphi2, f.Jz, f.Ephi, f.Br, f.Br2, f.Bz, f.Bz2,
                f.EzImposed, f.ErImposed, f.PsiImposed, f.BzImposed, f.BrImposed, f.Psi, f.Q, in->d_flags,
                in->cnt, in->d_bins, in->d_onaxis_data, in->d_onaxis, in->d_tr_flag, in->d_tr_scratch, in->d_pclog, in->d_status, in->d_moments, in->d_lost, in->d_points,
                in->d_list, in->d_nodes, in->d_node_vals, in->d_samples, in->d_sample_idx, in->d_sample_pts};
@@ -1174,13 +1182,10 @@ extern "C" int spiffe_gpu_zero_current_arrays(spiffe_gpu_instance *in)
     return fail(SPIFFE_ERR_INVALID, "null argument");
   if (in->s32)
     return s32_zero_j(in);
-  const size_t bytes = in->nodes * sizeof(double);
-  if (in->mesh.modes & SPIFFE_FL_TM_FIELDS) {
-    CUDA_TRY(cudaMemsetAsync(in->f.Jz, 0, bytes, in->stream));
-    CUDA_TRY(cudaMemsetAsync(in->f.Jr, 0, bytes, in->stream));
-  }
-  if (in->mesh.modes & SPIFFE_FL_TE_FIELDS)
-    CUDA_TRY(cudaMemsetAsync(in->f.Jphi, 0, bytes, in->stream));
+  const int first = in->mesh.modes & SPIFFE_FL_TM_FIELDS ? 0 : 2, last = in->mesh.modes & SPIFFE_FL_TE_FIELDS ? 3 : 2;
+  if (last > first)
+    CUDA_TRY(cudaMemsetAsync(in->f.Jz + first * in->j_stride, 0, (last - first) * in->j_stride * sizeof(double),
+                             in->stream));
   return 0;
 }
 

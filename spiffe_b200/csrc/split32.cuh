@@ -130,6 +130,7 @@ struct Particles32Work {
   size_t cub_bytes = 0;
   DevBeam32 alt{}; // second beam buffer for the cell sort
   long long capacity = 0;
+  bool met_none = false; // the last push left the on-axis extremes at (+inf, -inf)
 };
 struct Push32Params {
   double time;

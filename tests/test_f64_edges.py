@@ -106,3 +106,38 @@ def test_sor_follows_ends_set_after_setup(oracle):
     ref = fd.copy()
     oracle.solve_poisson(ref, ref["Psi"], ref["Q"], 1e-300, 20)
     assert np.array_equal(g.fields(fd)["Psi"], ref["Psi"])
+
+
+@pytest.mark.parametrize("n, n_lost", [(1, 1), (2, 1), (40, 39), (1500, 1024), (9000, 4096), (20000, 6000), (40000, 33000)])
+def test_swap_compaction_pairs_holes_with_the_last_survivors(n, n_lost):
+    """One block removes the lost: the j-th lost slot takes the j-th survivor
+    counted from the end, whatever the number of losses (none, a block's, more
+    than are sorted), and the counts are ready for the next push."""
+    f = pillbox(60, 50)
+    m = f.mesh
+    rng = np.random.default_rng(n)
+    lost = np.sort(rng.choice(n, n_lost, replace=False))
+    z = np.full(n, 0.5 * (m.zmin + m.zmax))
+    z[lost] = m.zmax - 0.1 * m.dz  # leaves the mesh in one step at pz = 10
+    pz = np.zeros(n)
+    pz[lost] = 10.0
+    vz = np.where(pz > 0, 2.98e8, 0.0)
+    b = abi.Beam(n + 16)
+    b.QoMC = QoMC
+    b.set(n, z=z, r=np.full(n, 10.0 * m.dr), pz=pz, vz=vz, Q=np.full(n, -1e-16), particleID=np.arange(1, n + 1),
+          status=np.full(n, abi.PART_ACTIVE, np.uint64))
+    b.npActive = n
+    g = gpu.GpuInstance(f, capacity=b.capacity)
+    g.upload_beam(b)
+    g.configure_run(space_charge=0, push=abi.push_options(abi.COMPACT_SWAP, abi.SCREEN_PARTICLE))
+    new_np = n - n_lost
+    gone = np.isin(np.arange(n), lost)
+    expect = np.arange(1, n + 1)[:new_np]
+    holes, donors = lost[lost < new_np], np.nonzero(~gone[new_np:])[0] + new_np
+    expect[holes] = donors[::-1] + 1
+    for _ in range(2):  # the second step loses nothing
+        g.run_steps(1)
+        got = g.download_beam(abi.Beam(b.capacity))
+        assert got.np == got.npActive == new_np
+        assert np.array_equal(got["particleID"], expect)
+    g.close()
