@@ -48,14 +48,13 @@
 // phases took two to three times as long) and because no CTA waits for
 // another, so solves of several instances share the SMs.  Values and update
 // order are those of the sweeps run over the whole mesh.
-// Levels of at most MG_TAIL_NODES nodes are worked together by one CTA, the
-// coarsest solved exactly by its precomputed inverse when it has at most
-// MG_MAX_DIRECT unknowns, else by Gauss-Seidel sweeps.  Coefficients are kept
+// The first level of at most MG_MAX_DIRECT unknowns is the coarsest, solved
+// exactly by its precomputed inverse over the whole GPU.  Coefficients are kept
 // per distinct row (class): in a gun nearly all rows of a level are alike, so
 // a band's fit L1 and a thread keeps its columns' in registers.
-// Measured from a cold start to 1e-6 (B200): 3001 x 821 gun, 6 cycles, 1.6 ms
-// -> 1.07 ms; 1500 x 400, 7 cycles, 1.13 -> 0.65; 424 x 232, 9 cycles, 0.99
-// -> 0.61; 601 x 165, 5 cycles, 0.69 -> 0.39.
+// Measured from a cold start to 1e-6 (B200), first form -> here: 3001 x 821
+// gun 1.6 -> 0.78 ms in 5 cycles, 1500 x 400 1.13 -> 0.38 in 5, 424 x 232
+// 0.99 -> 0.48 in 9, 601 x 165 0.69 -> 0.29 in 5.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -72,12 +71,12 @@ namespace {
 
 constexpr int MG_NT = 512;             // threads per CTA
 constexpr int MG_W = MG_NT / 32;       // warps per CTA
-constexpr int MG_TAIL_NODES = 3000;    // levels at most this large are worked by one CTA together
-constexpr int MG_MIN_UNKNOWNS = 64;    // coarsening stops at this many unknowns
+constexpr int MG_MIN_UNKNOWNS = 64;    // a mesh of no more unknowns is not coarsened
 constexpr int MG_NODES_PER_CTA = 4096; // mesh nodes per band below one band per SM
 constexpr int MG_MIN_ROWS = 4;         // own rows of a coarse level's band at least
-constexpr int MG_MAX_DIRECT = 1024;    // a coarsest level of at most this many unknowns is solved exactly
-constexpr int MG_COARSE_SWEEPS = 24;   // sweeps on a larger one
+constexpr int MG_MAX_DIRECT = 2048;    // a level of at most this many unknowns is the coarsest, solved exactly
+constexpr int MG_MAX_BAND = 512;       // where the unknowns' couplings reach no farther than this
+constexpr int MG_COARSE_SWEEPS = 24;   // sweeps on another coarsest level
 constexpr int MG_DOWN = 5, MG_UP = 4;  // halo rows a side of a band on the way down and up
 enum { MG_INVD = 8, MG_DIAG = 9 };
 
@@ -928,98 +927,110 @@ __global__ void __launch_bounds__(MG_NT, 1) k_mg_up0(const __grid_constant__ Mg0
   }
 }
 
-// The smallest levels, lev[0] .. lev[n-1], by one CTA with CTA barriers:
-// descent, the coarsest level's solve, ascent back to lev[0], whose u goes to
-// its v.  With SM the levels' u and f (from soff on) and a residual lie in
-// shared memory, else in global memory.
-struct MgTail {
-  MgLevel lev[MG_MAX_LEVELS];
-  int n;
-  const float *cinv; // the coarsest level's inverse, cn x cn row-major (null: coarse sweeps)
-  const int *cidx;   // its unknowns' array indices on that level
-  int cn;
-};
-
-template <bool SM, class Op> __global__ void __launch_bounds__(MG_NT, 1) k_mg_tail(const __grid_constant__ MgTail a)
+// The coarsest level solved exactly: v = A^-1 f over its n unknowns (array
+// indices idx[]), a warp a row of the inverse.  The rows (16 MB for 2048
+// unknowns, from L2 or at worst in 3 us from HBM) are on their way to
+// registers while f is gathered.  It takes the place of the V-cycle's levels
+// below 2048 unknowns, whose kernel of one CTA was the longest of a cycle on
+// all but the largest meshes, its sweeps being chains of CTA barriers: 34 -> 5.9
+// us a cycle on a 3001 x 821 gun, 26 -> 4.3 on 1500 x 400, 24 -> 3.5 on 601 x
+// 165; and an exact solve there saves cycles (6 -> 5 and 7 -> 5 of a cold start
+// to 1e-6 on the first two).  Below about 2048 unknowns the inverse costs less
+// to read than the two kernels of another level (5 us each).
+__global__ void __launch_bounds__(MG_NT) k_mg_dense(const float *__restrict__ inv, int ld, const int *__restrict__ idx,
+                                                    int n, const float *f, float *v)
 {
-  __shared__ float coarse_f[MG_MAX_DIRECT]; // the coarsest level's f, gathered for its exact solve
-  float *buf = reinterpret_cast<float *>(mg_smem);
-  const int N = a.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  auto uof = [&](int l) { return SM ? buf + a.lev[l].soff : a.lev[l].u; }; // row -1 first
-  auto fof = [&](int l) { return SM ? buf + a.lev[l].soff + (a.lev[l].Z + 2) * a.lev[l].P : a.lev[l].f; };
-  float *R = SM ? buf : a.lev[0].v; // the residual of one level at a time (v is free until the end)
-  for (int l = 0; l < N; l++) {
-    const int n = (a.lev[l].Z + 2) * a.lev[l].P;
-    float *u = uof(l), *f = fof(l);
-    const float *g = a.lev[l].f;
-    for (int k = 4 * tid; k < n; k += 4 * MG_NT) {
-      st4(u + k, make_float4(0.f, 0.f, 0.f, 0.f));
-      if (SM)
-        st4(f + k, l == 0 ? ldcg4(g + k) : make_float4(0.f, 0.f, 0.f, 0.f));
+  __shared__ __align__(16) float x[MG_MAX_DIRECT];
+  constexpr int K = MG_MAX_DIRECT / 128;
+  const int tid = threadIdx.x, lane = tid & 31, row = blockIdx.x * MG_W + (tid >> 5);
+  float4 m[K];
+  const float4 *src = reinterpret_cast<const float4 *>(inv + (size_t)min(row, n - 1) * ld) + lane;
+#pragma unroll
+  for (int k = 0; k < K; k++)
+    m[k] = 128 * k < ld ? __ldg(src + 32 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int at = __ldg(idx + min(row, n - 1));
+  for (int i = tid; i < ld; i += MG_NT)
+    x[i] = i < n ? __ldcg(f + __ldg(idx + i)) : 0.f;
+  __syncthreads();
+  float acc = 0.f;
+#pragma unroll
+  for (int k = 0; k < K; k++)
+    if (128 * k < ld) {
+      const float4 y = ld4(x + 4 * (32 * k + lane));
+      acc += m[k].x * y.x + m[k].y * y.y + (m[k].z * y.z + m[k].w * y.w);
     }
+  for (int o = 16; o > 0; o >>= 1)
+    acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if (lane == 0 && row < n)
+    v[at] = acc;
+}
+
+// The inverse's columns from the banded factors (rows of 2 b + 1 doubles: L
+// below the unit diagonal, 1 / U's diagonal, U above it): a warp takes 32
+// columns through the forward and the backward substitution, a lane a column,
+// the last b rows in shared memory, the forward result in y (n x ld).
+__global__ void __launch_bounds__(32) k_mg_inverse(int n, int b, const double *__restrict__ lu, double *y, float *inv, int ld)
+{
+  extern __shared__ double ring[]; // (b + 1) x 32
+  const int lane = threadIdx.x, c0 = 32 * blockIdx.x, c = c0 + lane, w = 2 * b + 1;
+  for (int i = 0; i <= b; i++)
+    ring[32 * i + lane] = 0;
+  for (int i = 0, at = 0; i < n; i++, at = at == b ? 0 : at + 1) {
+    double acc[4] = {i == c ? 1.0 : 0.0, 0, 0, 0};
+    if (i >= c0) { // zero before
+      const double *l = lu + (size_t)i * w; // l[b - k]: the coupling to row i - k
+      for (int k0 = 1, p = at; k0 <= b; k0 += 4)
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          p = p == 0 ? b : p - 1;
+          if (k0 + q <= b)
+            acc[q] -= __ldg(l + b - k0 - q) * ring[32 * p + lane];
+        }
+    }
+    const double x = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    ring[32 * at + lane] = x;
+    y[(size_t)i * ld + c] = x;
+  }
+  for (int i = 0; i <= b; i++)
+    ring[32 * i + lane] = 0;
+  for (int i = n - 1, at = 0; i >= 0; i--, at = at == b ? 0 : at + 1) {
+    const double *u = lu + (size_t)i * w + b; // u[k]: the coupling to row i + k
+    double acc[4] = {y[(size_t)i * ld + c], 0, 0, 0};
+    for (int k0 = 1, p = at; k0 <= b; k0 += 4)
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        p = p == 0 ? b : p - 1;
+        if (k0 + q <= b)
+          acc[q] -= __ldg(u + k0 + q) * ring[32 * p + lane];
+      }
+    const double x = ((acc[0] + acc[1]) + (acc[2] + acc[3])) * __ldg(u);
+    ring[32 * at + lane] = x;
+    inv[(size_t)i * ld + c] = c < n ? (float)x : 0.f;
+  }
+}
+
+// A coarsest level that has no inverse (one that cannot be coarsened further
+// with more unknowns than MG_MAX_DIRECT): sweeps by one CTA.  With SM u and f
+// lie in shared memory, else in global memory.  The result goes to v.
+template <bool SM, class Op> __global__ void __launch_bounds__(MG_NT, 1) k_mg_coarse(const __grid_constant__ MgLevel L)
+{
+  const int tid = threadIdx.x, n = (L.Z + 2) * L.P;
+  float *u = SM ? reinterpret_cast<float *>(mg_smem) : L.u, *f = SM ? u + n : L.f; // row -1 first
+  for (int k = 4 * tid; k < n; k += 4 * MG_NT) {
+    st4(u + k, make_float4(0.f, 0.f, 0.f, 0.f));
+    if (SM)
+      st4(f + k, ldcg4(L.f + k));
   }
   __syncthreads();
   Op t;
+  t.init(L, f, -1, 0, L.Z);
 #pragma unroll 1
-  for (int l = 0; l < N; l++) {
-    if (l == N - 1 && a.cinv)
-      break;
-    const MgLevel L = a.lev[l];
-    float *u = uof(l), *f = fof(l);
-    t.init(L, f, -1, 0, L.Z);
-    for (int k = 4 * tid; k < (L.Z + 2) * L.P; k += 4 * MG_NT) // halos of the residual
-      st4(R + k, make_float4(0.f, 0.f, 0.f, 0.f));
-    const int sweeps = l == N - 1 ? MG_COARSE_SWEEPS : 2;
-#pragma unroll 1
-    for (int k = 0; k < sweeps; k++) {
-      rows9<0, 0>(L, t, u, f, -1, 0, L.Z);
-      rows9<1, 0>(L, t, u, f, -1, 0, L.Z);
-    }
-    if (l == N - 1)
-      break;
-    t.resid(L, u, f, R, -1, 0, L.Z);
-    __syncthreads();
-    restrict9(L, a.lev[l + 1], R, -1, 0, a.lev[l + 1].Z, fof(l + 1));
-    __syncthreads();
+  for (int k = 0; k < MG_COARSE_SWEEPS; k++) {
+    rows9<0, 0>(L, t, u, f, -1, 0, L.Z);
+    rows9<1, 0>(L, t, u, f, -1, 0, L.Z);
   }
-  if (a.cinv) {
-    // the coarsest level solved exactly: u = A^-1 f over its unknowns
-    const float *f = fof(N - 1);
-    float *u = uof(N - 1);
-    for (int i = tid; i < a.cn; i += MG_NT)
-      coarse_f[i] = f[__ldg(a.cidx + i)];
-    __syncthreads();
-    // a warp per row: coalesced reads of the row, the lanes' partial sums
-    // added by shuffles
-    for (int i = warp; i < a.cn; i += MG_W) {
-      const float *row = a.cinv + (size_t)i * a.cn;
-      float acc = 0.f;
-      for (int k = lane; k < a.cn; k += 32)
-        acc += __ldg(row + k) * coarse_f[k];
-      for (int o = 16; o > 0; o >>= 1)
-        acc += __shfl_down_sync(0xffffffffu, acc, o);
-      if (lane == 0)
-        u[__ldg(a.cidx + i)] = acc;
-    }
-    __syncthreads();
-  }
-#pragma unroll 1
-  for (int l = N - 2; l >= 0; l--) {
-    const MgLevel L = a.lev[l];
-    float *u = uof(l), *f = fof(l);
-    t.init(L, f, -1, 0, L.Z);
-    t.template prolong<false>(L, a.lev[l + 1], u, uof(l + 1), -1);
-    __syncthreads();
-#pragma unroll 1
-    for (int k = 0; k < 2; k++) {
-      rows9<1, 1>(L, t, u, f, -1, 0, L.Z);
-      rows9<0, 1>(L, t, u, f, -1, 0, L.Z);
-    }
-  }
-  const float *u = uof(0);
-  float *v = a.lev[0].v;
-  for (int k = 4 * tid, n = (a.lev[0].Z + 2) * a.lev[0].P; k < n; k += 4 * MG_NT)
-    st4(v + k, ld4(u + k));
+  for (int k = 4 * tid; k < n; k += 4 * MG_NT)
+    st4(L.v + k, ld4(u + k));
 }
 
 // ---- host: the level hierarchy
@@ -1215,71 +1226,64 @@ extern "C" void s32_mg_free(Mg32Work *w)
 }
 
 namespace {
-// The inverse of the coarsest level's operator over its unknowns (Gauss-Jordan
-// with partial pivoting in FP64), for the exact coarse solve; false when the
-// level has more than MG_MAX_DIRECT unknowns or the matrix is singular.
-bool coarse_inverse(const Stencil &S, const MgLevel &D, std::vector<float> &inv, std::vector<int> &idx)
+// The coarsest level's operator over its unknowns as banded LU factors, for
+// k_mg_inverse; false when the level has more than MG_MAX_DIRECT unknowns or
+// couplings beyond MG_MAX_BAND, or a pivot is not negative.  No pivoting: the
+// operator is negative definite in the annulus-weighted inner product, and a
+// Galerkin product keeps that.  The unknowns are numbered along the shorter
+// direction, so the band is that direction's length.
+bool coarse_factor(const Stencil &S, const MgLevel &D, std::vector<double> &lu, int &b, std::vector<int> &idx)
 {
   std::vector<int> num((size_t)S.Z * S.R, -1);
   idx.clear();
-  for (int I = 0; I < S.Z; I++)
-    for (int J = 0; J < S.R; J++)
+  const bool rows = S.R <= S.Z;
+  for (int p = 0; p < (rows ? S.Z : S.R); p++)
+    for (int q = 0; q < (rows ? S.R : S.Z); q++) {
+      const int I = rows ? p : q, J = rows ? q : p;
       if (S.unk[(size_t)I * S.R + J]) {
         num[(size_t)I * S.R + J] = (int)idx.size();
         idx.push_back((I + 1) * D.P + (J & 1) * D.Q + (J >> 1) + 1);
       }
+    }
   const int n = (int)idx.size();
   if (n == 0 || n > MG_MAX_DIRECT)
     return false;
-  std::vector<double> A((size_t)n * n, 0.0), X((size_t)n * n, 0.0);
-  for (int I = 0; I < S.Z; I++)
-    for (int J = 0; J < S.R; J++) {
-      const int r = num[(size_t)I * S.R + J];
-      if (r < 0)
-        continue;
-      for (int k = 0; k < 9; k++) {
-        const int i2 = I + k / 3 - 1, j2 = J + k % 3 - 1;
-        if (i2 < 0 || i2 >= S.Z || j2 < 0 || j2 >= S.R)
-          continue;
-        const int c = num[(size_t)i2 * S.R + j2];
-        if (c >= 0)
-          A[(size_t)r * n + c] += S.at(k, I, J);
+  auto couplings = [&](auto fn) {
+    for (int I = 0; I < S.Z; I++)
+      for (int J = 0; J < S.R; J++) {
+        const int r = num[(size_t)I * S.R + J];
+        for (int k = 0; r >= 0 && k < 9; k++) {
+          const int i2 = I + k / 3 - 1, j2 = J + k % 3 - 1;
+          if (i2 < 0 || i2 >= S.Z || j2 < 0 || j2 >= S.R)
+            continue;
+          const int c = num[(size_t)i2 * S.R + j2];
+          if (c >= 0)
+            fn(r, c, S.at(k, I, J));
+        }
       }
-    }
-  for (int i = 0; i < n; i++)
-    X[(size_t)i * n + i] = 1.0;
-  for (int col = 0; col < n; col++) {
-    int piv = col;
-    for (int r = col + 1; r < n; r++)
-      if (std::fabs(A[(size_t)r * n + col]) > std::fabs(A[(size_t)piv * n + col]))
-        piv = r;
-    if (A[(size_t)piv * n + col] == 0)
+  };
+  b = 1;
+  couplings([&](int r, int c, double) { b = std::max(b, std::abs(r - c)); });
+  if (b > MG_MAX_BAND)
+    return false;
+  const int w = 2 * b + 1;
+  lu.assign((size_t)n * w, 0.0); // (r, c) at r w + b + c - r
+  couplings([&](int r, int c, double v) { lu[(size_t)r * w + b + c - r] += v; });
+  for (int k = 0; k < n; k++) {
+    double *pk = lu.data() + (size_t)k * w + b; // pk[j]: (k, k + j)
+    if (!(pk[0] < 0))
       return false;
-    if (piv != col)
-      for (int k = 0; k < n; k++) {
-        std::swap(A[(size_t)piv * n + k], A[(size_t)col * n + k]);
-        std::swap(X[(size_t)piv * n + k], X[(size_t)col * n + k]);
-      }
-    const double d = 1 / A[(size_t)col * n + col];
-    for (int k = 0; k < n; k++) {
-      A[(size_t)col * n + k] *= d;
-      X[(size_t)col * n + k] *= d;
-    }
-    for (int r = 0; r < n; r++) {
-      if (r == col)
+    pk[0] = 1 / pk[0];
+    const int last = std::min(b, n - 1 - k);
+    for (int i = 1; i <= last; i++) {
+      double *pi = lu.data() + (size_t)(k + i) * w + b - i; // pi[j]: (k + i, k + j)
+      if (pi[0] == 0)
         continue;
-      const double fct = A[(size_t)r * n + col];
-      if (fct == 0)
-        continue;
-      for (int k = 0; k < n; k++) {
-        A[(size_t)r * n + k] -= fct * A[(size_t)col * n + k];
-        X[(size_t)r * n + k] -= fct * X[(size_t)col * n + k];
-      }
+      const double m = pi[0] *= pk[0];
+      for (int j = 1; j <= last; j++)
+        pi[j] -= m * pk[j];
     }
   }
-  inv.assign((size_t)n * n, 0.f);
-  for (size_t k = 0; k < inv.size(); k++)
-    inv[k] = (float)X[k];
   return true;
 }
 } // namespace
@@ -1292,13 +1296,19 @@ std::vector<const void *> mg_smem_kernels()
           (const void *)k_mg_down9<true, Fix9<1>>, (const void *)k_mg_down9<true, Fix9<2>>,
           (const void *)k_mg_down9<true, Run9>,    (const void *)k_mg_up9<true, Fix9<1>>,
           (const void *)k_mg_up9<true, Fix9<2>>,   (const void *)k_mg_up9<true, Run9>,
-          (const void *)k_mg_tail<true, Fix9<2>>,  (const void *)k_mg_tail<true, Run9>};
+          (const void *)k_mg_coarse<true, Fix9<2>>, (const void *)k_mg_coarse<true, Run9>};
 }
+
+// the coarsest level's inverse and its unknowns' array indices, on the device
+struct MgDense {
+  const float *inv;
+  const int *idx;
+  int n, ld;
+};
 
 // The solve as a graph: the residual's kernel, then a WHILE node around a
 // V-cycle that ends with the next residual.
-int mg_graph(Mg32Work *w, Mg0 z, MgTail t, int tail, bool sm, bool tail_sm, float *scratch, size_t budget,
-             size_t tail_bytes)
+int mg_graph(Mg32Work *w, Mg0 z, int last, bool sm, const MgDense *dense, bool coarse_sm, float *scratch, size_t budget)
 {
   MgLevel *lev = w->lev;
   MgCall *call = (MgCall *)w->call;
@@ -1322,9 +1332,9 @@ int mg_graph(Mg32Work *w, Mg0 z, MgTail t, int tail, bool sm, bool tail_sm, floa
                               : (const void *)k_mg_up9<true, Run9>;
   };
   const void *ku0 = sm ? (const void *)k_mg_up0<true> : (const void *)k_mg_up0<false>;
-  const void *kt = !tail_sm                                       ? (const void *)k_mg_tail<false, Run9>
-                   : pairs(lev[tail], lev[tail].Z) <= 2 * MG_NT ? (const void *)k_mg_tail<true, Fix9<2>>
-                                                                  : (const void *)k_mg_tail<true, Run9>;
+  const void *kc = !coarse_sm                                     ? (const void *)k_mg_coarse<false, Run9>
+                   : pairs(lev[last], lev[last].Z) <= 2 * MG_NT ? (const void *)k_mg_coarse<true, Fix9<2>>
+                                                                  : (const void *)k_mg_coarse<true, Run9>;
   cudaError_t e = cudaSuccess;
   // the attribute is process-wide: the kernels' limit, not this instance's need
   for (const void *k : mg_smem_kernels())
@@ -1366,14 +1376,21 @@ int mg_graph(Mg32Work *w, Mg0 z, MgTail t, int tail, bool sm, bool tail_sm, floa
   if (e == cudaSuccess) {
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     prev = nullptr;
-    for (int l = 1; l < tail; l++) {
+    for (int l = 1; l < last; l++) {
       size_t n = floats_of(lev[l].rp, lev[l].P);
       void *a9[] = {&lev[l], &lev[l + 1], &scratch, &n};
       add(body, kd9(lev[l]), lev[l].nb, bytes_of(lev[l].rp, lev[l].P), a9);
     }
-    void *at[] = {&t};
-    add(body, kt, 1, tail_sm ? tail_bytes : 0, at);
-    for (int l = tail - 1; l >= 1; l--) {
+    const MgLevel &C = lev[last];
+    if (dense) {
+      MgDense d = *dense;
+      void *ad[] = {&d.inv, &d.ld, &d.idx, &d.n, (void *)&C.f, (void *)&C.v};
+      add(body, (const void *)k_mg_dense, (d.n + MG_W - 1) / MG_W, 0, ad);
+    } else {
+      void *ac[] = {&lev[last]};
+      add(body, kc, 1, coarse_sm ? 2 * sizeof(float) * (size_t)(C.Z + 2) * C.P : 0, ac);
+    }
+    for (int l = last - 1; l >= 1; l--) {
       size_t n = floats_of(lev[l].rp, lev[l].P);
       void *a9[] = {&lev[l], &lev[l + 1], &scratch, &n};
       add(body, ku9(lev[l]), lev[l].nb, bytes_of(lev[l].rp, lev[l].P), a9);
@@ -1407,7 +1424,7 @@ extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *flags, Mg32Work *w,
   double sz = m->dz, sr = m->dr; // the finest level's spacings so far
   while ((int)lev.size() < MG_MAX_LEVELS) {
     const Stencil &F = lev.back();
-    if (unknowns(F) <= (size_t)MG_MIN_UNKNOWNS)
+    if (unknowns(F) <= (size_t)(lev.size() > 1 ? MG_MAX_DIRECT : MG_MIN_UNKNOWNS))
       break;
     const int cz = sz >= 2 * sr ? 1 : 2, cr = sr >= 2 * sz ? 1 : 2;
     if ((cz == 2 && F.Z < 5) || (cr == 2 && F.R < 5))
@@ -1517,22 +1534,15 @@ extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *flags, Mg32Work *w,
   }
   const size_t o_crow = put(crow.data(), P0 * sizeof(float)), o_drow = put(drow.data(), P0 * sizeof(float));
   const size_t o_cpd = put(cpd.data(), P0 * sizeof(double)), o_cmd = put(cmd.data(), P0 * sizeof(double));
-  std::vector<float> cinv;
+  std::vector<double> lu;
   std::vector<int> cidx;
-  size_t o_cinv = 0, o_cidx = 0;
-  const bool direct = coarse_inverse(lev[L - 1], w->lev[L - 1], cinv, cidx);
-  if (direct) {
-    o_cinv = put(cinv.data(), cinv.size() * sizeof(float));
+  int band_b = 0;
+  size_t o_cidx = 0;
+  const bool direct = coarse_factor(lev[L - 1], w->lev[L - 1], lu, band_b, cidx);
+  const int cn = (int)cidx.size(), ld = (cn + 127) / 128 * 128;
+  if (direct)
     o_cidx = put(cidx.data(), cidx.size() * sizeof(int));
-  }
-
-  // the first level small enough for CTA 0 alone (at least level 1, at most the coarsest)
-  int tail = L - 1;
-  for (int l = 1; l < L; l++)
-    if ((size_t)lev[l].Z * lev[l].R <= (size_t)MG_TAIL_NODES) {
-      tail = l;
-      break;
-    }
+  const int last = L - 1;
 
   // Bands: a level's rows in one band per SM at most, and no more of them than
   // the mesh gives work (a small mesh's solve leaves the other SMs to other
@@ -1568,15 +1578,9 @@ extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *flags, Mg32Work *w,
   };
   int rp0 = 0, nb0 = 0;
   band(m->nz, P0, rp0, nb0);
-  for (int l = 1; l < tail; l++)
+  for (int l = 1; l < last; l++)
     band(w->lev[l].Z, w->lev[l].P, w->lev[l].rp, w->lev[l].nb);
-  // the last levels together: a residual of the largest, each one's u and f
-  size_t soff = (size_t)(lev[tail].Z + 2) * w->lev[tail].P;
-  for (int l = tail; l < L; l++) {
-    w->lev[l].soff = (int)soff;
-    soff += (size_t)2 * (lev[l].Z + 2) * w->lev[l].P;
-  }
-  const bool tail_fits = soff <= budget;
+  const bool coarse_fits = 2 * (size_t)(lev[last].Z + 2) * w->lev[last].P <= budget;
 
   // device memory, one block: the constant data, level 0's u0 and f0 at the
   // mesh pitch, each coarse level's u, f and v of (Z+2) x P floats, the
@@ -1595,7 +1599,9 @@ extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *flags, Mg32Work *w,
   const size_t o_part = bytes;
   bytes += ((size_t)2 * nb0 * sizeof(double) + 255) / 256 * 256;
   const size_t o_call = bytes;
-  bytes += sizeof(MgCall);
+  bytes += (sizeof(MgCall) + 255) / 256 * 256;
+  const size_t o_inv = bytes;
+  bytes += direct ? (size_t)cn * ld * sizeof(float) : 0;
   char *mem = nullptr;
   cudaError_t e = cudaMalloc(&mem, bytes);
   if (e != cudaSuccess)
@@ -1617,8 +1623,27 @@ extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *flags, Mg32Work *w,
   e = cudaMemsetAsync(mem + blob.size(), 0, bytes - blob.size(), s);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(mem, blob.data(), blob.size(), cudaMemcpyHostToDevice, s);
+  char *tmp = nullptr; // the factors and the forward substitution's result
+  const size_t lu_bytes = lu.size() * sizeof(double);
+  if (e == cudaSuccess && direct) {
+    e = cudaMalloc(&tmp, lu_bytes + (size_t)cn * ld * sizeof(double));
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(tmp, lu.data(), lu_bytes, cudaMemcpyHostToDevice, s);
+    const size_t ring = (size_t)(band_b + 1) * 32 * sizeof(double);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_mg_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (MG_MAX_BAND + 1) * 32 * (int)sizeof(double));
+    if (e == cudaSuccess) {
+      k_mg_inverse<<<ld / 32, 32, ring, s>>>(cn, band_b, (const double *)tmp, (double *)(tmp + lu_bytes),
+                                             (float *)(mem + o_inv), ld);
+      spiffe_note_launches(1);
+      e = cudaGetLastError();
+    }
+  }
+  const cudaError_t done = cudaStreamSynchronize(s);
   if (e == cudaSuccess)
-    e = cudaStreamSynchronize(s);
+    e = done;
+  cudaFree(tmp);
   if (e != cudaSuccess) {
     s32_mg_free(w);
     return (int)e;
@@ -1648,15 +1673,9 @@ extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *flags, Mg32Work *w,
   z.cpd = (const double *)(mem + o_cpd);
   z.cmd = (const double *)(mem + o_cmd);
   z.part = (double *)(mem + o_part);
-  MgTail t{};
-  t.n = L - tail;
-  for (int l = tail; l < L; l++)
-    t.lev[l - tail] = w->lev[l];
-  t.cinv = direct ? (const float *)(mem + o_cinv) : nullptr;
-  t.cidx = direct ? (const int *)(mem + o_cidx) : nullptr;
-  t.cn = direct ? (int)cidx.size() : 0;
-  e = (cudaError_t)mg_graph(w, z, t, tail, fits, tail_fits, (float *)(mem + o_scratch), budget * sizeof(float),
-                            soff * sizeof(float));
+  const MgDense dense{(const float *)(mem + o_inv), (const int *)(mem + o_cidx), cn, ld};
+  e = (cudaError_t)mg_graph(w, z, last, fits, direct ? &dense : nullptr, coarse_fits, (float *)(mem + o_scratch),
+                            budget * sizeof(float));
   if (e != cudaSuccess) {
     s32_mg_free(w);
     return (int)e;

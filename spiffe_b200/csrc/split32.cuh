@@ -186,7 +186,6 @@ struct MgLevel {
   int P = 0, Q = 0;    // row pitch; column J of a row lies at (J&1) Q + (J>>1) + 1, P = 2 Q
   int cz = 2, cr = 2;  // coarsening from the level above in z and r: node (I, J) is its (cz I, cr J)
   int rp = 0, nb = 0;  // rows of a band, bands (levels worked by a band a CTA)
-  int soff = 0;        // place of u and f in shared memory, in floats (the levels worked by one CTA)
   float *u = nullptr, *f = nullptr, *v = nullptr; // (Z+2) x P, row I at (I+1) P; halo nodes stay 0.
                                                   // u: pre-smoothed, v: the way up's result
   const float *coef = nullptr; // [class][MG_NCOEF][P]; 1/diagonal 0 marks a held node
