@@ -1221,7 +1221,7 @@ extern "C" void s32_mg_free(Mg32Work *w)
 {
   if (w->exec)
     cudaGraphExecDestroy((cudaGraphExec_t)w->exec);
-  cudaFree(w->mem);
+  dev_free(w->mem);
   *w = Mg32Work();
 }
 
@@ -1296,7 +1296,7 @@ std::vector<const void *> mg_smem_kernels()
           (const void *)k_mg_down9<true, Fix9<1>>, (const void *)k_mg_down9<true, Fix9<2>>,
           (const void *)k_mg_down9<true, Run9>,    (const void *)k_mg_up9<true, Fix9<1>>,
           (const void *)k_mg_up9<true, Fix9<2>>,   (const void *)k_mg_up9<true, Run9>,
-          (const void *)k_mg_coarse<true, Fix9<2>>, (const void *)k_mg_coarse<true, Run9>};
+          (const void *)k_mg_coarse<true, Fix9<2>>};
 }
 
 // the coarsest level's inverse and its unknowns' array indices, on the device
@@ -1332,9 +1332,8 @@ int mg_graph(Mg32Work *w, Mg0 z, int last, bool sm, const MgDense *dense, bool c
                               : (const void *)k_mg_up9<true, Run9>;
   };
   const void *ku0 = sm ? (const void *)k_mg_up0<true> : (const void *)k_mg_up0<false>;
-  const void *kc = !coarse_sm                                     ? (const void *)k_mg_coarse<false, Run9>
-                   : pairs(lev[last], lev[last].Z) <= 2 * MG_NT ? (const void *)k_mg_coarse<true, Fix9<2>>
-                                                                  : (const void *)k_mg_coarse<true, Run9>;
+  const bool coarse_fix = coarse_sm && pairs(lev[last], lev[last].Z) <= 2 * MG_NT;
+  const void *kc = coarse_fix ? (const void *)k_mg_coarse<true, Fix9<2>> : (const void *)k_mg_coarse<false, Run9>;
   cudaError_t e = cudaSuccess;
   // the attribute is process-wide: the kernels' limit, not this instance's need
   for (const void *k : mg_smem_kernels())
@@ -1388,7 +1387,7 @@ int mg_graph(Mg32Work *w, Mg0 z, int last, bool sm, const MgDense *dense, bool c
       add(body, (const void *)k_mg_dense, (d.n + MG_W - 1) / MG_W, 0, ad);
     } else {
       void *ac[] = {&lev[last]};
-      add(body, kc, 1, coarse_sm ? 2 * sizeof(float) * (size_t)(C.Z + 2) * C.P : 0, ac);
+      add(body, kc, 1, coarse_fix ? 2 * sizeof(float) * (size_t)(C.Z + 2) * C.P : 0, ac);
     }
     for (int l = last - 1; l >= 1; l--) {
       size_t n = floats_of(lev[l].rp, lev[l].P);
@@ -1603,7 +1602,7 @@ extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *flags, Mg32Work *w,
   const size_t o_inv = bytes;
   bytes += direct ? (size_t)cn * ld * sizeof(float) : 0;
   char *mem = nullptr;
-  cudaError_t e = cudaMalloc(&mem, bytes);
+  cudaError_t e = dev_malloc(&mem, bytes);
   if (e != cudaSuccess)
     return (int)e;
   w->mem = mem;
@@ -1626,7 +1625,7 @@ extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *flags, Mg32Work *w,
   char *tmp = nullptr; // the factors and the forward substitution's result
   const size_t lu_bytes = lu.size() * sizeof(double);
   if (e == cudaSuccess && direct) {
-    e = cudaMalloc(&tmp, lu_bytes + (size_t)cn * ld * sizeof(double));
+    e = dev_malloc(&tmp, lu_bytes + (size_t)cn * ld * sizeof(double));
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(tmp, lu.data(), lu_bytes, cudaMemcpyHostToDevice, s);
     const size_t ring = (size_t)(band_b + 1) * 32 * sizeof(double);
@@ -1643,7 +1642,7 @@ extern "C" int s32_mg_setup(const DevMesh *m, const int16_t *flags, Mg32Work *w,
   const cudaError_t done = cudaStreamSynchronize(s);
   if (e == cudaSuccess)
     e = done;
-  cudaFree(tmp);
+  dev_free(tmp);
   if (e != cudaSuccess) {
     s32_mg_free(w);
     return (int)e;
