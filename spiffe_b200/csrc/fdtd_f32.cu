@@ -10,6 +10,7 @@
 //     the next step's deposition (fused into the push) starts from zero;
 //   * the per-node flag tests and the FL_LAST_ACTIVE_PT row cut-offs are one
 //     precomputed update-mask byte.
+#include "slab.hpp"
 #include "split32.cuh"
 
 #include <cmath>
@@ -1005,9 +1006,11 @@ extern "C" int s32_fdtd_tables(const DevMesh *m, const int16_t *host_flags, Fdtd
   t->fEphi = (float)(dti * factor);
   cudaError_t e = cudaSuccess;
   if (!t->cpd) {
-    e = cudaMalloc(&t->cpd, sizeof(float) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&t->cmd, sizeof(float) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&t->bzf, sizeof(float) * (nr + 1));
+    DeviceSlab d;
+    d.add(&t->cpd, nr + 1);
+    d.add(&t->cmd, nr + 1);
+    d.add(&t->bzf, nr + 1);
+    e = d.make();
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(t->cpd, cpd.data(), sizeof(float) * (nr + 1), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(t->cmd, cmd.data(), sizeof(float) * (nr + 1), cudaMemcpyHostToDevice, s);
@@ -1020,12 +1023,10 @@ extern "C" int s32_fdtd_tables(const DevMesh *m, const int16_t *host_flags, Fdtd
 
 extern "C" void s32_fdtd_tables_free(Fdtd32Tables *t)
 {
-  cudaFree(t->cpd);
-  cudaFree(t->cmd);
-  cudaFree(t->bzf);
-  cudaFree(t->pub);
-  cudaFree(t->flag);
-  cudaFree(t->arrivals);
+  dev_free(t->cpd); // with cmd and bzf
+  dev_free(t->pub);
+  dev_free(t->flag);
+  dev_free(t->arrivals);
   *t = Fdtd32Tables();
 }
 
@@ -1064,15 +1065,15 @@ static int fused_plan(const DevMesh *m, Fdtd32Tables *t)
   t->bands = (rows + t->rows_per - 1) / t->rows_per;
   // (a new plan follows a new mesh: the buffers are made again for it; the
   // flags start at 0 below every epoch still to come)
-  cudaFree(t->pub);
-  cudaFree(t->flag);
-  cudaFree(t->arrivals);
+  dev_free(t->pub);
+  dev_free(t->flag);
+  dev_free(t->arrivals);
   t->pub = nullptr;
   t->flag = t->arrivals = nullptr;
-  e = cudaMalloc(&t->pub, sizeof(float) * (size_t)t->bands * P);
-  if (e == cudaSuccess) e = cudaMalloc(&t->flag, sizeof(unsigned) * t->bands);
+  e = dev_malloc(&t->pub, sizeof(float) * (size_t)t->bands * P);
+  if (e == cudaSuccess) e = dev_malloc(&t->flag, sizeof(unsigned) * t->bands);
   if (e == cudaSuccess) e = cudaMemset(t->flag, 0, sizeof(unsigned) * t->bands);
-  if (e == cudaSuccess) e = cudaMalloc(&t->arrivals, sizeof(unsigned));
+  if (e == cudaSuccess) e = dev_malloc(&t->arrivals, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(t->arrivals, 0, sizeof(unsigned));
   if (e != cudaSuccess)
     return (int)e;

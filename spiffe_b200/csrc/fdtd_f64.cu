@@ -247,11 +247,13 @@ extern "C" int spiffe_fdtd64_tables(const DevMesh *m, const int16_t *host_flags,
   t->fEphi = 1. / (eps0 * mu0);
   cudaError_t e = cudaSuccess;
   if (!t->cpz) {
-    e = cudaMalloc(&t->cpz, sizeof(double) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&t->cmz, sizeof(double) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&t->bzf, sizeof(double) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&t->cut0, sizeof(int) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&t->cut1, sizeof(int) * (nr + 1));
+    DeviceSlab d;
+    d.add(&t->cpz, nr + 1);
+    d.add(&t->cmz, nr + 1);
+    d.add(&t->bzf, nr + 1);
+    d.add(&t->cut0, nr + 1);
+    d.add(&t->cut1, nr + 1);
+    e = d.make();
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(t->cpz, cpz, sizeof(double) * (nr + 1), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(t->cmz, cmz, sizeof(double) * (nr + 1), cudaMemcpyHostToDevice, s);
@@ -269,11 +271,7 @@ extern "C" int spiffe_fdtd64_tables(const DevMesh *m, const int16_t *host_flags,
 
 extern "C" void spiffe_fdtd64_tables_free(Fdtd64Tables *t)
 {
-  cudaFree(t->cpz);
-  cudaFree(t->cmz);
-  cudaFree(t->bzf);
-  cudaFree(t->cut0);
-  cudaFree(t->cut1);
+  dev_free(t->cpz); // with the others
   *t = Fdtd64Tables();
 }
 

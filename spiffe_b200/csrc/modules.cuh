@@ -4,6 +4,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "slab.hpp"
 
 struct Fdtd64Tables {
   double *cpz = nullptr, *cmz = nullptr, *bzf = nullptr;

@@ -1306,21 +1306,17 @@ extern "C" int s32_beam_alloc(DevBeam32 *b, long long n)
 {
   *b = DevBeam32();
   b->capacity = n;
-  cudaError_t e = cudaSuccess;
-#define AL(x) \
-  if (e == cudaSuccess) e = cudaMalloc(&b->x, sizeof(*b->x) * (size_t)n);
+  DeviceSlab m;
+#define AL(x) m.add(&b->x, (size_t)n);
   AL(cell) AL(fz) AL(fr) AL(pz) AL(pr) AL(rpphi) AL(Q) AL(status) AL(zmin) AL(zmax) AL(rmin) AL(rmax) AL(r0) AL(z0)
   AL(t0) AL(particleID) AL(generation)
 #undef AL
-  return (int)e;
+  return (int)m.make();
 }
 
 extern "C" void s32_beam_free(DevBeam32 *b)
 {
-  void *p[] = {b->cell, b->fz, b->fr, b->pz, b->pr, b->rpphi, b->Q, b->status, b->zmin, b->zmax,
-               b->rmin, b->rmax, b->r0, b->z0, b->t0, b->particleID, b->generation};
-  for (void *q : p)
-    cudaFree(q);
+  dev_free(b->cell);
   *b = DevBeam32();
 }
 
@@ -1340,16 +1336,18 @@ extern "C" int s32_particles_work(Particles32Work *w, long long capacity)
   if (w->capacity >= capacity)
     return 0;
   s32_particles_work_free(w);
-  cudaError_t e = cudaMalloc(&w->lost_list, sizeof(int32_t) * (size_t)(capacity + 16));
-  if (e == cudaSuccess) e = cudaMalloc(&w->keys, sizeof(int32_t) * (size_t)(capacity + 16));
-  if (e == cudaSuccess) e = cudaMalloc(&w->keys_alt, sizeof(int32_t) * (size_t)(capacity + 16));
-  if (e == cudaSuccess) e = cudaMalloc(&w->idx, sizeof(int32_t) * (size_t)(capacity + 16));
-  if (e == cudaSuccess) e = cudaMalloc(&w->idx_alt, sizeof(int32_t) * (size_t)(capacity + 16));
-  size_t sort_bytes = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (uint32_t *)nullptr, (uint32_t *)nullptr, (int32_t *)nullptr,
+  const size_t n = (size_t)(capacity + 16);
+  w->cub_bytes = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, w->cub_bytes, (uint32_t *)nullptr, (uint32_t *)nullptr, (int32_t *)nullptr,
                                   (int32_t *)nullptr, (int)capacity);
-  w->cub_bytes = sort_bytes;
-  if (e == cudaSuccess) e = cudaMalloc(&w->cub_tmp, w->cub_bytes);
+  DeviceSlab m;
+  m.add(&w->lost_list, n);
+  m.add(&w->keys, n);
+  m.add(&w->keys_alt, n);
+  m.add(&w->idx, n);
+  m.add(&w->idx_alt, n);
+  m.add((char **)&w->cub_tmp, w->cub_bytes);
+  cudaError_t e = m.make();
   if (e == cudaSuccess) e = (cudaError_t)s32_beam_alloc(&w->alt, capacity);
   w->capacity = capacity;
   return (int)e;
@@ -1357,12 +1355,7 @@ extern "C" int s32_particles_work(Particles32Work *w, long long capacity)
 
 extern "C" void s32_particles_work_free(Particles32Work *w)
 {
-  cudaFree(w->lost_list);
-  cudaFree(w->keys);
-  cudaFree(w->keys_alt);
-  cudaFree(w->idx);
-  cudaFree(w->idx_alt);
-  cudaFree(w->cub_tmp);
+  dev_free(w->lost_list); // with the others
   s32_beam_free(&w->alt);
   *w = Particles32Work();
 }

@@ -846,47 +846,35 @@ extern "C" int spiffe_particles64_work(Particles64Work *w, long long capacity, b
 {
   cudaError_t e = cudaSuccess;
   if (w->capacity < capacity) {
-    cudaFree(w->lost);
-    cudaFree(w->lost_list);
-    cudaFree(w->holes);
-    cudaFree(w->donors);
-    cudaFree(w->keys);
-    cudaFree(w->keys_alt);
-    cudaFree(w->vals);
-    cudaFree(w->vals_alt);
-    cudaFree(w->cub_tmp);
-    *w = Particles64Work();
-    e = cudaMalloc(&w->lost, capacity + 16);
-    if (e == cudaSuccess) e = cudaMalloc(&w->lost_list, sizeof(int) * (capacity + 16));
-    if (e == cudaSuccess) e = cudaMalloc(&w->holes, sizeof(int) * (capacity + 16));
-    if (e == cudaSuccess) e = cudaMalloc(&w->donors, sizeof(int) * (capacity + 16));
-    size_t sort_bytes = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (int *)nullptr, (int *)nullptr, (double *)nullptr,
+    spiffe_particles64_work_free(w);
+    cub::DeviceRadixSort::SortPairs(nullptr, w->cub_bytes, (int *)nullptr, (int *)nullptr, (double *)nullptr,
                                     (double *)nullptr, (int)(4 * capacity));
-    w->cub_bytes = sort_bytes;
-    if (e == cudaSuccess) e = cudaMalloc(&w->cub_tmp, w->cub_bytes);
+    const size_t n = (size_t)(capacity + 16);
+    DeviceSlab m;
+    m.add(&w->lost, n);
+    m.add(&w->lost_list, n);
+    m.add(&w->holes, n);
+    m.add(&w->donors, n);
+    m.add((char **)&w->cub_tmp, w->cub_bytes);
+    e = m.make();
     w->capacity = capacity;
   }
   if (e == cudaSuccess && ordered && !w->keys) {
-    e = cudaMalloc(&w->keys, sizeof(int) * 4 * w->capacity);
-    if (e == cudaSuccess) e = cudaMalloc(&w->keys_alt, sizeof(int) * 4 * w->capacity);
-    if (e == cudaSuccess) e = cudaMalloc(&w->vals, sizeof(double) * 4 * w->capacity);
-    if (e == cudaSuccess) e = cudaMalloc(&w->vals_alt, sizeof(double) * 4 * w->capacity);
+    const size_t n = 4 * (size_t)w->capacity;
+    DeviceSlab m;
+    m.add(&w->keys, n);
+    m.add(&w->keys_alt, n);
+    m.add(&w->vals, n);
+    m.add(&w->vals_alt, n);
+    e = m.make();
   }
   return (int)e;
 }
 
 extern "C" void spiffe_particles64_work_free(Particles64Work *w)
 {
-  cudaFree(w->lost);
-  cudaFree(w->lost_list);
-  cudaFree(w->holes);
-  cudaFree(w->donors);
-  cudaFree(w->keys);
-  cudaFree(w->keys_alt);
-  cudaFree(w->vals);
-  cudaFree(w->vals_alt);
-  cudaFree(w->cub_tmp);
+  dev_free(w->lost); // with the others of its slab
+  dev_free(w->keys); // with the ordered sums' others
   *w = Particles64Work();
 }
 

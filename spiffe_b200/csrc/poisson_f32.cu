@@ -1143,21 +1143,23 @@ extern "C" int s32_poisson_setup(const DevMesh *m, Poisson32Work *w, long long n
   size_t parts = std::max<size_t>(3 * gx * gy, 4096);
   (void)np_capacity;
   if (e == cudaSuccess && !w->Az) {
-    e = cudaMalloc(&w->Az, sizeof(double) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&w->Ari, sizeof(double) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&w->Aro, sizeof(double) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&w->volume, sizeof(double) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&w->crow, sizeof(float) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&w->drow, sizeof(float) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&w->scalars, sizeof(double) * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&w->qreal_fixed, sizeof(long long));
-    if (e == cudaSuccess) e = cudaMalloc(&w->st, sizeof(PcState));
+    DeviceSlab d;
+    d.add(&w->Az, nr + 1);
+    d.add(&w->Ari, nr + 1);
+    d.add(&w->Aro, nr + 1);
+    d.add(&w->volume, nr + 1);
+    d.add(&w->crow, nr + 1);
+    d.add(&w->drow, nr + 1);
+    d.add(&w->scalars, 8);
+    d.add(&w->qreal_fixed, 1);
+    d.add(&w->st, 1);
+    d.add(&w->iters, 1);
+    d.add(&w->bar, 48);                      // counter, sum slots
+    d.add(&w->dpart, (size_t)sms * 2);       // |rhs|, |r0| per CTA
+    d.add(&w->xbuf, (size_t)2 * sms * 16 * H); // exchange rows, 4 a side
+    d.add(&w->part, parts);
+    e = d.make();
     if (e == cudaSuccess) e = cudaMemsetAsync(w->st, 0, sizeof(PcState), s);
-    if (e == cudaSuccess) e = cudaMalloc(&w->iters, sizeof(long long));
-    if (e == cudaSuccess) e = cudaMalloc(&w->bar, sizeof(unsigned long long) * 48); // counter, sum slots
-    if (e == cudaSuccess) e = cudaMalloc(&w->dpart, sizeof(double) * (size_t)sms * 2); // |rhs|, |r0| per CTA
-    if (e == cudaSuccess) e = cudaMalloc(&w->xbuf, sizeof(float) * (size_t)2 * sms * 16 * H); // exchange rows, 4 a side
-    if (e == cudaSuccess) e = cudaMalloc(&w->part, sizeof(double) * parts);
     w->part_n = parts;
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->Az, Az.data(), sizeof(double) * (nr + 1), cudaMemcpyHostToDevice, s);
@@ -1173,10 +1175,8 @@ extern "C" int s32_poisson_setup(const DevMesh *m, Poisson32Work *w, long long n
 extern "C" void s32_poisson_free(Poisson32Work *w)
 {
   s32_mg_free(&w->mg);
-  void *p[] = {w->Az, w->Ari, w->Aro, w->volume, w->crow, w->drow, w->scalars, w->qreal_fixed, w->st,
-               w->iters, w->bar, w->dpart, w->xbuf, w->part, w->omega};
-  for (void *q : p)
-    cudaFree(q);
+  dev_free(w->Az); // with the others
+  dev_free(w->omega);
   *w = Poisson32Work();
 }
 
@@ -1184,9 +1184,9 @@ static int ensure_omega32(const DevMesh *m, Poisson32Work *w, long long limit, c
 {
   if (w->omega_n >= limit)
     return 0;
-  cudaFree(w->omega);
+  dev_free(w->omega);
   w->omega = nullptr;
-  cudaError_t e = cudaMalloc(&w->omega, sizeof(float) * (size_t)limit);
+  cudaError_t e = dev_malloc(&w->omega, sizeof(float) * (size_t)limit);
   if (e != cudaSuccess)
     return (int)e;
   // Chebyshev acceleration (poisson.c:342-346, :117-119), in FP64 then rounded

@@ -778,20 +778,24 @@ extern "C" int spiffe_poisson64_setup(const DevMesh *m, Poisson64Work *w, long l
   if (parts < 4096)
     parts = 4096;
   if (!w->Az) {
-    e = cudaMalloc(&w->Az, sizeof(double) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&w->Ari, sizeof(double) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&w->Aro, sizeof(double) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&w->volume, sizeof(double) * (nr + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&w->scalars, sizeof(double) * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&w->bar, sizeof(unsigned) * 2);
+    DeviceSlab d;
+    d.add(&w->Az, nr + 1);
+    d.add(&w->Ari, nr + 1);
+    d.add(&w->Aro, nr + 1);
+    d.add(&w->volume, nr + 1);
+    d.add(&w->crow, nr + 1);
+    d.add(&w->drow, nr + 1);
+    d.add(&w->scalars, 8);
+    d.add(&w->bar, 2);
+    d.add(&w->st, 1);
+    d.add(&w->iters, 1);
+    e = d.make();
     if (e == cudaSuccess) e = cudaMemsetAsync(w->bar, 0, sizeof(unsigned) * 2, s);
-    if (e == cudaSuccess) e = cudaMalloc(&w->st, sizeof(PcState));
     if (e == cudaSuccess) e = cudaMemsetAsync(w->st, 0, sizeof(PcState), s);
-    if (e == cudaSuccess) e = cudaMalloc(&w->iters, sizeof(long long));
   }
   if (e == cudaSuccess && w->part_n < parts) {
-    cudaFree(w->part);
-    e = cudaMalloc(&w->part, sizeof(double) * parts);
+    dev_free(w->part);
+    e = dev_malloc(&w->part, sizeof(double) * parts);
     w->part_n = parts;
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->Az, Az, sizeof(double) * (nr + 1), cudaMemcpyHostToDevice, s);
@@ -807,8 +811,6 @@ extern "C" int spiffe_poisson64_setup(const DevMesh *m, Poisson64Work *w, long l
     } else
       crow[ir] = drow[ir] = 1 / (dr * dr);
   }
-  if (e == cudaSuccess && !w->crow) e = cudaMalloc(&w->crow, sizeof(double) * (nr + 1));
-  if (e == cudaSuccess && !w->drow) e = cudaMalloc(&w->drow, sizeof(double) * (nr + 1));
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->crow, crow, sizeof(double) * (nr + 1), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->drow, drow, sizeof(double) * (nr + 1), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -843,7 +845,7 @@ extern "C" int spiffe_poisson64_setup(const DevMesh *m, Poisson64Work *w, long l
       e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes);
       const int used = (rows + R - 1) / R;
       const size_t rs = (size_t)rows * 2 * H, xb = (size_t)4 * used * H;
-      if (e == cudaSuccess) e = cudaMalloc(&w->band_mem, (rs + xb) * sizeof(double) + 32 * sizeof(unsigned long long));
+      if (e == cudaSuccess) e = dev_malloc(&w->band_mem, (rs + xb) * sizeof(double) + 32 * sizeof(unsigned long long));
       if (e == cudaSuccess) {
         w->band_kernel = k;
         w->band_grid = used;
@@ -862,19 +864,10 @@ extern "C" int spiffe_poisson64_setup(const DevMesh *m, Poisson64Work *w, long l
 
 extern "C" void spiffe_poisson64_free(Poisson64Work *w)
 {
-  cudaFree(w->Az);
-  cudaFree(w->Ari);
-  cudaFree(w->Aro);
-  cudaFree(w->volume);
-  cudaFree(w->part);
-  cudaFree(w->scalars);
-  cudaFree(w->omega);
-  cudaFree(w->bar);
-  cudaFree(w->st);
-  cudaFree(w->iters);
-  cudaFree(w->crow);
-  cudaFree(w->drow);
-  cudaFree(w->band_mem);
+  dev_free(w->Az); // with the others
+  dev_free(w->part);
+  dev_free(w->omega);
+  dev_free(w->band_mem);
   *w = Poisson64Work();
 }
 
@@ -883,7 +876,7 @@ static int ensure_omega(const DevMesh *m, Poisson64Work *w, long long limit, cud
 {
   if (w->omega && w->omega_n >= limit)
     return 0;
-  cudaFree(w->omega);
+  dev_free(w->omega);
   const double rz = m->dz / m->dr;
   const double rj = (cos(SPIFFE_PI / m->nz) + rz * rz * cos(SPIFFE_PI / m->nr)) / (1 + rz * rz);
   double *om = new double[limit];
@@ -895,7 +888,7 @@ static int ensure_omega(const DevMesh *m, Poisson64Work *w, long long limit, cud
     else
       omega = 1.0 / (1 - rj * rj * omega / 4);
   }
-  cudaError_t e = cudaMalloc(&w->omega, sizeof(double) * limit);
+  cudaError_t e = dev_malloc(&w->omega, sizeof(double) * limit);
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->omega, om, sizeof(double) * limit, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   delete[] om;

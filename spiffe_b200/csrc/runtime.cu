@@ -213,6 +213,7 @@ struct spiffe_gpu_instance {
   DevMesh dm{};
   cudaStream_t stream = nullptr;
   size_t nodes = 0;
+  char *slab = nullptr; // the arrays made with the instance (fields, flags)
   size_t j_stride = 0; // FP64: doubles from one component of J to the next
   std::vector<int16_t> h_flags;
   int16_t *d_flags = nullptr;
@@ -344,28 +345,27 @@ static void onaxis_terms(spiffe_gpu_instance *in)
 
 static int alloc_field(double **p, size_t n, cudaStream_t s)
 {
-  CUDA_TRY(cudaMalloc(p, n * sizeof(double)));
+  CUDA_TRY(dev_malloc(p, n * sizeof(double)));
   CUDA_TRY(cudaMemsetAsync(*p, 0, n * sizeof(double), s));
   return 0;
 }
 
 static int alloc_beam(DevBeam64 *b, long long n)
 {
-#define BA(x) CUDA_TRY(cudaMalloc(&b->x, sizeof(*b->x) * (size_t)n))
+  DeviceSlab m;
+#define BA(x) m.add(&b->x, (size_t)n)
   BA(z); BA(r); BA(pz); BA(pr); BA(r_pphi); BA(vz); BA(vr); BA(vphi); BA(Q);
   BA(r0); BA(z0); BA(t0); BA(rmin); BA(rmax); BA(zmin); BA(zmax);
   BA(particleID); BA(generation); BA(status);
 #undef BA
+  CUDA_TRY(m.make());
   b->capacity = n;
   return 0;
 }
 
 static void free_beam(DevBeam64 *b)
 {
-  void *p[] = {b->z, b->r, b->pz, b->pr, b->r_pphi, b->vz, b->vr, b->vphi, b->Q, b->r0, b->z0, b->t0,
-               b->rmin, b->rmax, b->zmin, b->zmax, b->particleID, b->generation, b->status};
-  for (void *q : p)
-    cudaFree(q);
+  dev_free(b->z); // with the others
   *b = DevBeam64{};
 }
 
@@ -450,10 +450,10 @@ static int s32_staging(spiffe_gpu_instance *in, size_t n)
   if (S.staging_n >= n)
     return 0;
   CUDA_TRY(cudaStreamSynchronize(in->stream));
-  cudaFree(S.staging);
+  dev_free(S.staging);
   S.staging = nullptr;
   S.staging_n = 0;
-  CUDA_TRY(cudaMalloc(&S.staging, n * sizeof(double)));
+  CUDA_TRY(dev_malloc(&S.staging, n * sizeof(double)));
   S.staging_n = n;
   return 0;
 }
@@ -495,15 +495,8 @@ static int s32_cover_charge(spiffe_gpu_instance *in, double qabs)
 
 static int s32_alloc_f(float **p, size_t n, cudaStream_t s)
 {
-  CUDA_TRY(cudaMalloc(p, n * sizeof(float)));
+  CUDA_TRY(dev_malloc(p, n * sizeof(float)));
   CUDA_TRY(cudaMemsetAsync(*p, 0, n * sizeof(float), s));
-  return 0;
-}
-
-template <typename T> static int s32_alloc_z(T **p, size_t n, cudaStream_t s)
-{
-  CUDA_TRY(cudaMalloc(p, n * sizeof(T)));
-  CUDA_TRY(cudaMemsetAsync(*p, 0, n * sizeof(T), s));
   return 0;
 }
 
@@ -547,39 +540,45 @@ static int s32_create(spiffe_gpu_instance *in, const int16_t *flags)
   const int nz = in->mesh.nz, nr = in->mesh.nr, P = in->dm.pitch;
   const size_t n = s32_nodes(in);
   cudaStream_t s = in->stream;
-  RC_TRY(s32_alloc_z(&in->d_flags, n, s));
+  const bool tm = in->mesh.modes & SPIFFE_FL_TM_FIELDS, te = in->mesh.modes & SPIFFE_FL_TE_FIELDS;
+  DeviceSlab d;
+  d.add(&in->slab, 0);
+  if (tm) // Ez, Er, Bphi, Bphi2 in one block, so one L2 access window can cover them
+    d.add(&S.tm_slab, 4 * n);
+  d.add(&in->d_flags, n);
+  d.add(&S.umask, n);
+  if (tm) {
+    d.add(&S.f.Jz, n);
+    d.add(&S.f.Jr, n);
+  }
+  if (te) {
+    for (float **p : {&S.f.Ephi, &S.f.Br, &S.f.Br2, &S.f.Bz, &S.f.Bz2})
+      d.add(p, n);
+    d.add(&S.f.Jphi, n);
+  }
+  d.add(&S.f.EzImposed, n);
+  d.add(&S.f.ErImposed, n);
+  d.add(&S.f.Psi, n);
+  d.add(&S.f.PsiImposed, n);
+  d.add(&S.f.Q, n);
+  d.add(&S.f.Qp, n);
+  d.add(&S.f.jbox, 2);
+  CUDA_TRY(d.make());
+  CUDA_TRY(cudaMemsetAsync(in->slab, 0, d.bytes(), s));
   CUDA_TRY(cudaMemcpy2DAsync(in->d_flags, (size_t)P * sizeof(int16_t), flags, (size_t)(nr + 1) * sizeof(int16_t),
                              (size_t)(nr + 1) * sizeof(int16_t), (size_t)nz + 1, cudaMemcpyHostToDevice, s));
-  RC_TRY(s32_alloc_z(&S.umask, n, s));
   S.f.flags = in->d_flags;
   S.f.umask = S.umask;
-  if (in->mesh.modes & SPIFFE_FL_TM_FIELDS) {
-    // Ez, Er, Bphi, Bphi2 in one block, so one L2 access window can cover them
-    RC_TRY(s32_alloc_f(&S.tm_slab, 4 * n, s));
+  if (tm) {
     S.f.Ez = S.tm_slab;
     S.f.Er = S.tm_slab + n;
     S.f.Bphi = S.tm_slab + 2 * n;
     S.f.Bphi2 = S.tm_slab + 3 * n;
-    RC_TRY(s32_alloc_z(&S.f.Jz, n, s));
-    RC_TRY(s32_alloc_z(&S.f.Jr, n, s));
     // large problems only: windows of many small instances would compete
     // for one set-aside (a batch's instances are small)
     if (4 * n * sizeof(float) >= ((size_t)32 << 20))
       RC_TRY(s32_l2_window(in, S.tm_slab, 4 * n * sizeof(float)));
   }
-  if (in->mesh.modes & SPIFFE_FL_TE_FIELDS) {
-    float **te[] = {&S.f.Ephi, &S.f.Br, &S.f.Br2, &S.f.Bz, &S.f.Bz2};
-    for (float **p : te)
-      RC_TRY(s32_alloc_f(p, n, s));
-    RC_TRY(s32_alloc_z(&S.f.Jphi, n, s));
-  }
-  RC_TRY(s32_alloc_f(&S.f.EzImposed, n, s));
-  RC_TRY(s32_alloc_f(&S.f.ErImposed, n, s));
-  RC_TRY(s32_alloc_z(&S.f.Psi, n, s));
-  RC_TRY(s32_alloc_z(&S.f.PsiImposed, n, s));
-  RC_TRY(s32_alloc_z(&S.f.Q, n, s));
-  RC_TRY(s32_alloc_z(&S.f.Qp, n, s));
-  CUDA_TRY(cudaMalloc(&S.f.jbox, 2 * sizeof(int)));
   RC_TRY(s32_jbox_set(S.f.jbox, 0x7fffffff, -1, s));
   RC_TRY(s32_beam_alloc(&S.b, in->capacity));
   RC_TRY(s32_particles_work(&S.pw, in->capacity));
@@ -599,11 +598,8 @@ static void s32_destroy(spiffe_gpu_instance *in)
     cudaStreamSetAttribute(in->stream, cudaStreamAttributeAccessPolicyWindow, &a);
     cudaCtxResetPersistingL2Cache();
   }
-  void *p[] = {S.tm_slab, S.f.Ephi, S.f.Br, S.f.Br2, S.f.Bz, S.f.Bz2,
-               S.f.EzImposed, S.f.ErImposed, S.f.BzImposed, S.f.BrImposed, S.f.Jz, S.f.Jr, S.f.Jphi,
-               S.f.Psi, S.f.PsiImposed, S.f.Q, S.f.Qp, S.f.jbox, S.umask, S.staging};
-  for (void *q : p)
-    cudaFree(q);
+  for (void *q : {(void *)S.f.BzImposed, (void *)S.f.BrImposed, (void *)S.staging})
+    dev_free(q);
   s32_beam_free(&S.b);
   s32_particles_work_free(&S.pw);
   s32_poisson_free(&S.pcw);
@@ -934,10 +930,11 @@ extern "C" int spiffe_gpu_create(const spiffe_mesh *mesh, const int16_t *flags, 
   cudaStream_t s = in->stream;
   const size_t n = in->nodes;
   in->capacity = particle_capacity > 1024 ? particle_capacity : 1024;
-  if (cudaMalloc(&in->cnt, sizeof(DevCounts)) != cudaSuccess ||
-      cudaMallocHost(&in->h_cnt, sizeof(DevCounts)) != cudaSuccess ||
-      cudaMallocHost(&in->h_probe, 8 * sizeof(double)) != cudaSuccess)
+  if (dev_malloc(&in->cnt, sizeof(DevCounts)) != cudaSuccess ||
+      spiffe_pinned_malloc((void **)&in->h_cnt, sizeof(DevCounts) + 8 * sizeof(double)) != cudaSuccess)
     return bail(fail(SPIFFE_ERR_NOMEM, "counter allocation failed"));
+  static_assert(sizeof(DevCounts) % sizeof(double) == 0, "doubles follow the counters");
+  in->h_probe = (double *)(in->h_cnt + 1);
   memset(in->h_cnt, 0, sizeof(DevCounts));
   in->h_cnt->nextParticleID = 1;
   in->h_cnt->first_lost = 0x7fffffffffffffffLL;
@@ -953,27 +950,26 @@ extern "C" int spiffe_gpu_create(const spiffe_mesh *mesh, const int16_t *flags, 
     *out = in;
     return 0;
   }
-  if (cudaMalloc(&in->d_flags, n * sizeof(int16_t)) != cudaSuccess ||
-      cudaMemcpyAsync(in->d_flags, flags, n * sizeof(int16_t), cudaMemcpyHostToDevice, s) != cudaSuccess)
-    return bail(fail(SPIFFE_ERR_NOMEM, "flag allocation failed"));
   DevFields<double> &f = in->f;
-  f.flags = in->d_flags;
-  // Jz, Jr (and Jphi) are one array, cleared by one fill a step
-  const size_t pad = in->j_stride = (n + 31) & ~(size_t)31;
-  if ((rc = alloc_field(&f.Jz, (mesh->modes & SPIFFE_FL_TE_FIELDS ? 3 : 2) * pad, s)))
-    return bail(rc);
-  f.Jr = f.Jz + pad;
-  if (mesh->modes & SPIFFE_FL_TE_FIELDS)
-    f.Jphi = f.Jz + 2 * pad;
-  double **tm[] = {&f.Ez, &f.Er, &f.Bphi, &f.Bphi2, &f.EzImposed, &f.ErImposed, &f.PsiImposed, &f.Psi, &f.Q};
-  for (double **p : tm)
-    if ((rc = alloc_field(p, n, s)))
-      return bail(rc);
-  if (mesh->modes & SPIFFE_FL_TE_FIELDS) {
-    double **te[] = {&f.Ephi, &f.Br, &f.Br2, &f.Bz, &f.Bz2};
-    for (double **p : te)
-      if ((rc = alloc_field(p, n, s)))
-        return bail(rc);
+  {
+    // Jz, Jr (and Jphi) lie one behind the other, cleared by one fill a step
+    const bool te = mesh->modes & SPIFFE_FL_TE_FIELDS;
+    const size_t pad = in->j_stride = (n + 31) & ~(size_t)31;
+    DeviceSlab d;
+    d.add(&in->slab, 0);
+    for (double **p : {&f.Jz, &f.Jr, &f.Jphi})
+      if (te || p != &f.Jphi)
+        d.add(p, pad);
+    for (double **p : {&f.Ez, &f.Er, &f.Bphi, &f.Bphi2, &f.EzImposed, &f.ErImposed, &f.PsiImposed, &f.Psi, &f.Q})
+      d.add(p, n);
+    if (te)
+      for (double **p : {&f.Ephi, &f.Br, &f.Br2, &f.Bz, &f.Bz2})
+        d.add(p, n);
+    d.add(&in->d_flags, n);
+    if (d.make() != cudaSuccess || cudaMemsetAsync(in->slab, 0, d.bytes(), s) != cudaSuccess ||
+        cudaMemcpyAsync(in->d_flags, flags, n * sizeof(int16_t), cudaMemcpyHostToDevice, s) != cudaSuccess)
+      return bail(fail(SPIFFE_ERR_NOMEM, "field allocation failed"));
+    f.flags = in->d_flags;
   }
   if ((rc = alloc_beam(&in->b, in->capacity)))
     return bail(rc);
@@ -995,35 +991,22 @@ extern "C" int spiffe_gpu_destroy(spiffe_gpu_instance *in)
   if (in->s32)
     s32_destroy(in);
   DevFields<double> &f = in->f;
-  void *p[] = {f.Ez, f.Er, f.Bphi, f.Bphi2, f.Jz, f.Ephi, f.Br, f.Br2, f.Bz, f.Bz2,
-               f.EzImposed, f.ErImposed, f.PsiImposed, f.BzImposed, f.BrImposed, f.Psi, f.Q, in->d_flags,
+  void *p[] = {in->slab, f.BzImposed, f.BrImposed,
                in->cnt, in->d_bins, in->d_onaxis_data, in->d_onaxis, in->d_tr_flag, in->d_tr_scratch, in->d_pclog, in->d_status, in->d_moments, in->d_lost, in->d_points,
                in->d_list, in->d_nodes, in->d_node_vals, in->d_samples, in->d_sample_idx, in->d_sample_pts};
   for (void *q : p)
-    cudaFree(q);
+    dev_free(q);
   for (int k = 0; k < in->screens.n; k++) {
     DevScreen &sc = in->screens.s[k];
-    for (int c = 0; c < SPIFFE_SCREEN_QUANS; c++)
-      cudaFree(sc.col[c]);
-    cudaFree(sc.rmin);
-    cudaFree(sc.rmax);
-    cudaFree(sc.zmin);
-    cudaFree(sc.zmax);
-    cudaFree(sc.generation);
-    cudaFree(sc.particleID);
-    cudaFree(sc.order);
+    dev_free(sc.col[0]); // with the others
   }
   free_beam(&in->b);
   spiffe_fdtd64_tables_free(&in->fdtd);
   spiffe_particles64_work_free(&in->pw);
   spiffe_poisson64_free(&in->pcw);
   in->timer.release();
-  if (in->h_cnt)
-    cudaFreeHost(in->h_cnt);
-  if (in->h_bins)
-    cudaFreeHost(in->h_bins);
-  if (in->h_probe)
-    cudaFreeHost(in->h_probe);
+  spiffe_pinned_free(in->h_cnt, sizeof(DevCounts) + 8 * sizeof(double));
+  spiffe_pinned_free(in->h_bins, in->bins_n * sizeof(BirthBin));
   if (in->stream)
     cudaStreamDestroy(in->stream);
   delete in;
@@ -1303,7 +1286,7 @@ __global__ void k_pc_log(const PcState *st, const double *driving, long long ste
 static int pc_log(spiffe_gpu_instance *in, const PcState *st, const double *driving)
 {
   if (!in->d_pclog) {
-    CUDA_TRY(cudaMalloc(&in->d_pclog, sizeof(double) * 4 * PCLOG_ROWS + sizeof(unsigned long long)));
+    CUDA_TRY(dev_malloc(&in->d_pclog, sizeof(double) * 4 * PCLOG_ROWS + sizeof(unsigned long long)));
     in->d_pclog_n = (unsigned long long *)(in->d_pclog + 4 * PCLOG_ROWS);
     CUDA_TRY(cudaMemsetAsync(in->d_pclog_n, 0, sizeof(unsigned long long), in->stream));
   }
@@ -1456,15 +1439,17 @@ extern "C" int spiffe_gpu_add_screen(spiffe_gpu_instance *in, double z_position,
   sc.cell = (int)std::floor((z_position - in->mesh.zmin) / in->mesh.dz);
   sc.capacity = capacity;
   const size_t n = (size_t)capacity;
+  DeviceSlab d;
   for (int c = 0; c < SPIFFE_SCREEN_QUANS; c++)
-    CUDA_TRY(cudaMalloc(&sc.col[c], n * sizeof(double)));
-  CUDA_TRY(cudaMalloc(&sc.rmin, n * sizeof(double)));
-  CUDA_TRY(cudaMalloc(&sc.rmax, n * sizeof(double)));
-  CUDA_TRY(cudaMalloc(&sc.zmin, n * sizeof(double)));
-  CUDA_TRY(cudaMalloc(&sc.zmax, n * sizeof(double)));
-  CUDA_TRY(cudaMalloc(&sc.generation, n * sizeof(int16_t)));
-  CUDA_TRY(cudaMalloc(&sc.particleID, n * sizeof(int32_t)));
-  CUDA_TRY(cudaMalloc(&sc.order, n * sizeof(long long)));
+    d.add(&sc.col[c], n);
+  d.add(&sc.rmin, n);
+  d.add(&sc.rmax, n);
+  d.add(&sc.zmin, n);
+  d.add(&sc.zmax, n);
+  d.add(&sc.generation, n);
+  d.add(&sc.particleID, n);
+  d.add(&sc.order, n);
+  CUDA_TRY(d.make());
   in->screens.n++;
   return 0;
 }
@@ -1487,7 +1472,7 @@ extern "C" int spiffe_gpu_screen_moments(spiffe_gpu_instance *in, int32_t is, do
   if (!in || !out || is < 0 || is >= in->screens.n)
     return fail(SPIFFE_ERR_INVALID, "bad screen index");
   if (!in->d_moments)
-    CUDA_TRY(cudaMalloc(&in->d_moments, sizeof(double) * (148 * 9 + 64)));
+    CUDA_TRY(dev_malloc(&in->d_moments, sizeof(double) * (148 * 9 + 64)));
   const int rc = spiffe_screen_moments_device(&in->screens.s[is], &in->cnt->screen_nb[is], in->d_moments, out,
                                               in->stream);
   if (rc)
@@ -1502,13 +1487,13 @@ static int lost_log_size(spiffe_gpu_instance *in, long long capacity)
   if (capacity == in->lost_cap)
     return 0;
   CUDA_TRY(cudaStreamSynchronize(in->stream));
-  cudaFree(in->d_lost);
+  dev_free(in->d_lost);
   in->d_lost = nullptr;
   in->d_lost_n = nullptr;
   in->lost_cap = 0;
   if (capacity == 0)
     return 0;
-  if (cudaMalloc(&in->d_lost, sizeof(LostRecord) * (size_t)capacity + 256) != cudaSuccess)
+  if (dev_malloc(&in->d_lost, sizeof(LostRecord) * (size_t)capacity + 256) != cudaSuccess)
     return fail(SPIFFE_ERR_NOMEM, "lost-particle log of %lld rows does not fit", capacity);
   in->d_lost_n = (unsigned long long *)((char *)in->d_lost + sizeof(LostRecord) * (size_t)capacity);
   CUDA_TRY(cudaMemsetAsync(in->d_lost_n, 0, sizeof(unsigned long long), in->stream));
@@ -1589,10 +1574,10 @@ static int ensure_points(spiffe_gpu_instance *in, size_t n)
 {
   if (n <= in->points_cap)
     return 0;
-  cudaFree(in->d_points);
+  dev_free(in->d_points);
   in->d_points = nullptr;
   const size_t cap = std::max<size_t>(n, 1024);
-  CUDA_TRY(cudaMalloc(&in->d_points, sizeof(double) * 4 * cap));
+  CUDA_TRY(dev_malloc(&in->d_points, sizeof(double) * 4 * cap));
   in->points_cap = cap;
   return 0;
 }
@@ -1737,10 +1722,10 @@ static int list_births(spiffe_gpu_instance *in, const std::vector<double> *col, 
     RC_TRY(grow_beam(in, in->h_cnt->np + (long long)total));
   }
   if (in->list_cap < total) {
-    cudaFree(in->d_list);
+    dev_free(in->d_list);
     in->d_list = nullptr;
     in->list_cap = std::max<size_t>(total, 1024);
-    CUDA_TRY(cudaMalloc(&in->d_list, sizeof(double) * BIRTH_LIST_COLS * in->list_cap));
+    CUDA_TRY(dev_malloc(&in->d_list, sizeof(double) * BIRTH_LIST_COLS * in->list_cap));
   }
   std::vector<double> flat;
   flat.reserve(BIRTH_LIST_COLS * total);
@@ -2144,11 +2129,13 @@ static int ensure_bins(spiffe_gpu_instance *in, size_t n)
 {
   if (in->bins_n >= n)
     return 0;
-  cudaFree(in->d_bins);
-  if (in->h_bins)
-    cudaFreeHost(in->h_bins);
-  CUDA_TRY(cudaMalloc(&in->d_bins, n * sizeof(BirthBin)));
-  CUDA_TRY(cudaMallocHost(&in->h_bins, n * sizeof(BirthBin)));
+  dev_free(in->d_bins);
+  in->d_bins = nullptr;
+  spiffe_pinned_free(in->h_bins, in->bins_n * sizeof(BirthBin)); // (the copies from it ended with d_bins' release)
+  in->h_bins = nullptr;
+  in->bins_n = 0;
+  CUDA_TRY(dev_malloc(&in->d_bins, n * sizeof(BirthBin)));
+  CUDA_TRY(spiffe_pinned_malloc((void **)&in->h_bins, n * sizeof(BirthBin)));
   in->bins_n = n;
   return 0;
 }
@@ -2413,12 +2400,12 @@ extern "C" int spiffe_gpu_add_on_axis_field(spiffe_gpu_instance *in, const doubl
   for (const OnAxisProfile &q : in->onaxis)
     total += q.z.size();
   CUDA_TRY(cudaStreamSynchronize(in->stream)); // the old tables may still be read
-  cudaFree(in->d_onaxis_data);
-  cudaFree(in->d_onaxis);
+  dev_free(in->d_onaxis_data);
+  dev_free(in->d_onaxis);
   in->d_onaxis_data = nullptr;
   in->d_onaxis = nullptr;
-  CUDA_TRY(cudaMalloc(&in->d_onaxis_data, 5 * total * sizeof(double)));
-  CUDA_TRY(cudaMalloc(&in->d_onaxis, in->onaxis.size() * sizeof(OnAxisField)));
+  CUDA_TRY(dev_malloc(&in->d_onaxis_data, 5 * total * sizeof(double)));
+  CUDA_TRY(dev_malloc(&in->d_onaxis, in->onaxis.size() * sizeof(OnAxisField)));
   std::vector<OnAxisField> views;
   double *d = in->d_onaxis_data;
   for (const OnAxisProfile &q : in->onaxis) {
@@ -2448,8 +2435,8 @@ extern "C" int spiffe_gpu_set_translation(spiffe_gpu_instance *in, int32_t enabl
   if (enable && (z_trigger < m.zmin + m.dz || z_trigger > m.zmax - m.dz))
     return fail(SPIFFE_ERR_INVALID, "z_trigger is not in range [zmin+dz, zmax-dz]");
   if (enable && !in->d_tr_flag) {
-    CUDA_TRY(cudaMalloc(&in->d_tr_flag, sizeof(int)));
-    CUDA_TRY(cudaMalloc(&in->d_tr_scratch, (size_t)m.nz * in->dm.pitch * sizeof(double)));
+    CUDA_TRY(dev_malloc(&in->d_tr_flag, sizeof(int)));
+    CUDA_TRY(dev_malloc(&in->d_tr_scratch, (size_t)m.nz * in->dm.pitch * sizeof(double)));
   }
   in->tr_on = enable != 0;
   in->tr_trigger = z_trigger;
@@ -2539,7 +2526,7 @@ extern "C" int spiffe_gpu_status_report(spiffe_gpu_instance *in, spiffe_status_r
   st->t = m.time;
   st->JCathode = in->cathodes.empty() ? 0 : in->cathodes[0].current_density;
   if (!in->d_status) {
-    CUDA_TRY(cudaMalloc(&in->d_status, sizeof(double) * (10 * (size_t)m.nr + 64)));
+    CUDA_TRY(dev_malloc(&in->d_status, sizeof(double) * (10 * (size_t)m.nr + 64)));
   }
   CUDA_TRY(cudaMemsetAsync(in->d_status, 0, sizeof(double) * (10 * (size_t)m.nr + 64), in->stream));
   double v[4 + 23];
@@ -2677,13 +2664,13 @@ static int node_sums(spiffe_gpu_instance *in, const std::vector<long long> &ez, 
   if (!n)
     return 0;
   if (in->nodes_cap < n) {
-    cudaFree(in->d_nodes);
-    cudaFree(in->d_node_vals);
+    dev_free(in->d_nodes);
+    dev_free(in->d_node_vals);
     in->d_nodes = nullptr;
     in->d_node_vals = nullptr;
     in->nodes_cap = std::max<size_t>(n, 256);
-    CUDA_TRY(cudaMalloc(&in->d_nodes, sizeof(long long) * 2 * in->nodes_cap));
-    CUDA_TRY(cudaMalloc(&in->d_node_vals, sizeof(double) * 2 * in->nodes_cap));
+    CUDA_TRY(dev_malloc(&in->d_nodes, sizeof(long long) * 2 * in->nodes_cap));
+    CUDA_TRY(dev_malloc(&in->d_node_vals, sizeof(double) * 2 * in->nodes_cap));
   }
   std::vector<long long> idx(ez);
   idx.insert(idx.end(), er.begin(), er.end());
@@ -2890,12 +2877,12 @@ static int sample_room(spiffe_gpu_instance *in, size_t need)
     return 0;
   const size_t cap = std::max<size_t>(2 * (in->samples_used + need), 4096);
   double *p = nullptr;
-  CUDA_TRY(cudaMalloc(&p, sizeof(double) * cap));
+  CUDA_TRY(dev_malloc(&p, sizeof(double) * cap));
   if (in->samples_used)
     CUDA_TRY(cudaMemcpyAsync(p, in->d_samples, sizeof(double) * in->samples_used, cudaMemcpyDeviceToDevice,
                              in->stream));
   CUDA_TRY(cudaStreamSynchronize(in->stream));
-  cudaFree(in->d_samples);
+  dev_free(in->d_samples);
   in->d_samples = p;
   in->samples_cap = cap;
   return 0;
@@ -2906,13 +2893,13 @@ static int sample_staging(spiffe_gpu_instance *in, size_t n)
   if (n <= in->sample_pts_cap)
     return 0;
   CUDA_TRY(cudaStreamSynchronize(in->stream)); // the old staging may still be read
-  cudaFree(in->d_sample_idx);
-  cudaFree(in->d_sample_pts);
+  dev_free(in->d_sample_idx);
+  dev_free(in->d_sample_pts);
   in->d_sample_idx = nullptr;
   in->d_sample_pts = nullptr;
   in->sample_pts_cap = std::max<size_t>(n, 1024);
-  CUDA_TRY(cudaMalloc(&in->d_sample_idx, sizeof(long long) * in->sample_pts_cap));
-  CUDA_TRY(cudaMalloc(&in->d_sample_pts, sizeof(double) * 2 * in->sample_pts_cap));
+  CUDA_TRY(dev_malloc(&in->d_sample_idx, sizeof(long long) * in->sample_pts_cap));
+  CUDA_TRY(dev_malloc(&in->d_sample_pts, sizeof(double) * 2 * in->sample_pts_cap));
   return 0;
 }
 
