@@ -314,6 +314,38 @@ __device__ __forceinline__ long long atomic_add_ll(long long *p, long long v)
 // Host-side launch helpers.
 inline unsigned blocks_for(long long n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
+// The kernels of a step follow one another on a stream, each reading what the
+// one before wrote, and a launch after a finished kernel costs 1.5 to 3 us of
+// an idle GPU.  launch_next's kernels are therefore brought onto the SMs as
+// soon as the blocks of the kernel before have all begun, and wait there:
+// such a kernel begins with step_begin(), before it reads or writes any
+// memory, which returns when the kernel before has ended and its writes are
+// visible (and so has, by the same rule, every kernel before that).
+// Measured (B200): build-up on 3001 x 821 25 -> 17 us a step, FP64 build-up on
+// 1201 x 329 23 -> 17 us, a small request 10.5 -> 9.0 ms.  The fields that such
+// kernels read are loaded plainly, never by __ldg: they are written while the
+// kernel already waits on the SMs (that costs the push 1.5 us of 38).
+__device__ __forceinline__ void step_begin()
+{
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args)
+{
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // Every host wrapper reports the kernels it queued (a process-wide count the
 // benchmark reads around its timed region).
 extern "C" void spiffe_note_launches(int n);

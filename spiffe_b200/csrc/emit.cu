@@ -175,6 +175,7 @@ __global__ void k_births_commit(long long total, long long capacity, int mode, D
 
 __global__ void k_antenna(double *J, int P, int direction, long istart, long iend, long iposition, double value)
 {
+  step_begin();
   const long i = istart + (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i > iend)
     return;
@@ -206,7 +207,7 @@ extern "C" int spiffe_antenna64(double *J, int pitch, int direction, long istart
   if (iend < istart)
     return 0;
   const long n = iend - istart + 1;
-  k_antenna<<<blocks_for(n, 128), 128, 0, s>>>(J, pitch, direction, istart, iend, iposition, value);
+  launch_next(k_antenna, blocks_for(n, 128), 128, s, J, pitch, direction, istart, iend, iposition, value);
   spiffe_note_launches(1);
   return (int)cudaGetLastError();
 }

@@ -190,8 +190,9 @@ __device__ __forceinline__ void tm_b_node(const DevMesh &m, const DevFields32 &f
 // take the first block indices, so they run beside the tiles.
 constexpr int VX = 32, VY = 8, VW = 4; // lanes per row segment, rows per tile, columns per group
 
-__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+// ldg4: constant tables; ld4: fields (written while the kernel waits in step_begin, so no read-only loads)
 __device__ __forceinline__ float4 ldg4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 __device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
 
 // Work split of one TM kernel.  Groups g = 1..G cover columns 4..4G+3; the
@@ -245,6 +246,7 @@ __device__ __forceinline__ void tm_boundary_node(const TmSplit &t, int nz, int n
 
 __global__ void __launch_bounds__(VX *VY) k_tm_e32(DevMesh m, DevFields32 f, Coef32 c, TmSplit t)
 {
+  step_begin();
   const int nz = m.nz, nr = m.nr, P = m.pitch;
   int jlo, jhi;
   jbox_rows(f.jbox, jlo, jhi);
@@ -274,12 +276,12 @@ __global__ void __launch_bounds__(VX *VY) k_tm_e32(DevMesh m, DevFields32 f, Coe
   longlong2 z01 = make_longlong2(0, 0), z23 = z01, r01 = z01, r23 = z01;
   float bnext = 0.f;
   if (in_row)
-    b0 = ldg4(f.Bphi + i);
+    b0 = ld4(f.Bphi + i);
   if (mine) {
     u = __ldg(reinterpret_cast<const uchar4 *>(f.umask + i));
     ez = ld4(f.Ez + i);
     er = ld4(f.Er + i);
-    bP = ldg4(f.Bphi + i + P);
+    bP = ld4(f.Bphi + i + P);
     cp = ldg4(c.cpd + ir0);
     cm = ldg4(c.cmd + ir0);
     if (jrow) {
@@ -289,7 +291,7 @@ __global__ void __launch_bounds__(VX *VY) k_tm_e32(DevMesh m, DevFields32 f, Coe
       r23 = *reinterpret_cast<const longlong2 *>(f.Jr + i + 2);
     }
     if (threadIdx.x == VX - 1)
-      bnext = __ldg(f.Bphi + i + VW); // ir0 + 4 <= nr - 1: inside the row
+      bnext = f.Bphi[i + VW]; // ir0 + 4 <= nr - 1: inside the row
   }
   const float bsh = __shfl_down_sync(0xffffffffu, b0.x, 1);
   if (!mine)
@@ -320,6 +322,7 @@ __global__ void __launch_bounds__(VX *VY) k_tm_e32(DevMesh m, DevFields32 f, Coe
 
 __global__ void __launch_bounds__(VX *VY) k_tm_b32(DevMesh m, DevFields32 f, Coef32 c, TmSplit t)
 {
+  step_begin();
   const int nz = m.nz, nr = m.nr, P = m.pitch;
   if (c.reset_box)
     jbox_reset(f.jbox);
@@ -346,14 +349,14 @@ __global__ void __launch_bounds__(VX *VY) k_tm_b32(DevMesh m, DevFields32 f, Coe
   uchar4 u = make_uchar4(0, 0, 0, 0);
   float eprev = 0.f;
   if (in_row)
-    ez = ldg4(f.Ez + i);
+    ez = ld4(f.Ez + i);
   if (mine) {
     u = __ldg(reinterpret_cast<const uchar4 *>(f.umask + i));
-    er = ldg4(f.Er + i);
-    erm = ldg4(f.Er + i - P);
+    er = ld4(f.Er + i);
+    erm = ld4(f.Er + i - P);
     b = ld4(f.Bphi + i);
     if (threadIdx.x == 0)
-      eprev = __ldg(f.Ez + i - 1); // ir0 - 1 >= 3: inside the row
+      eprev = f.Ez[i - 1]; // ir0 - 1 >= 3: inside the row
   }
   const float esh = __shfl_up_sync(0xffffffffu, ez.w, 1);
   if (!mine)
@@ -789,6 +792,7 @@ __global__ void k_tm_fused32(DevMesh m, DevFields32 f, Coef32 c, FusedArgs a)
 // Ephi (integrate.c:449-471)
 __global__ void __launch_bounds__(BX *BY) k_te_e32(DevMesh m, DevFields32 f, Coef32 c)
 {
+  step_begin();
   const int ir = blockIdx.x * BX + threadIdx.x, iz = blockIdx.y * BY + threadIdx.y;
   const int nz = m.nz, nr = m.nr, P = m.pitch;
   if (ir > nr || iz > nz)
@@ -813,6 +817,7 @@ __global__ void __launch_bounds__(BX *BY) k_te_e32(DevMesh m, DevFields32 f, Coe
 // Br/Br2 and Bz/Bz2 (integrate.c:473-539)
 __global__ void __launch_bounds__(BX *BY) k_te_b32(DevMesh m, DevFields32 f, Coef32 c)
 {
+  step_begin();
   const int ir = blockIdx.x * BX + threadIdx.x, iz = blockIdx.y * BY + threadIdx.y;
   const int nz = m.nz, nr = m.nr, P = m.pitch;
   if (c.reset_box)
@@ -914,6 +919,7 @@ __global__ void k_from_fixed(int nz, int nr, int P, const long long *src, double
 __global__ void k_antenna32(long long *J, int *jbox, int P, int direction, long istart, long iend, long iposition,
                             long long v)
 {
+  step_begin();
   const long i = istart + (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i > iend)
     return;
@@ -1110,14 +1116,14 @@ extern "C" int s32_fdtd_step(const DevMesh *m, const DevFields32 *f, Fdtd32Table
     const TmSplit te = tm_split(m->nz, m->nr, false), tb = tm_split(m->nz, m->nr, true);
     const int per = VX * VY;
     const dim3 vblock(VX, VY);
-    k_tm_e32<<<te.tiles + (unsigned)((te.nb + per - 1) / per), vblock, 0, s>>>(*m, *f, c, te);
-    k_tm_b32<<<tb.tiles + (unsigned)((tb.nb + per - 1) / per), vblock, 0, s>>>(*m, *f, c, tb);
+    launch_next(k_tm_e32, te.tiles + (unsigned)((te.nb + per - 1) / per), vblock, s, *m, *f, c, te);
+    launch_next(k_tm_b32, tb.tiles + (unsigned)((tb.nb + per - 1) / per), vblock, s, *m, *f, c, tb);
     spiffe_note_launches(2);
   }
   if (m->modes & SPIFFE_FL_TE_FIELDS) {
     c.reset_box = zero_j;
-    k_te_e32<<<grid, block, 0, s>>>(*m, *f, c);
-    k_te_b32<<<grid, block, 0, s>>>(*m, *f, c);
+    launch_next(k_te_e32, grid, block, s, *m, *f, c);
+    launch_next(k_te_b32, grid, block, s, *m, *f, c);
     spiffe_note_launches(2);
   }
   return (int)cudaGetLastError();
@@ -1171,7 +1177,7 @@ extern "C" int s32_antenna(long long *J, int *jbox, int pitch, int direction, lo
   if (iend < istart)
     return 0;
   const long n = iend - istart + 1;
-  k_antenna32<<<blocks_for(n, 128), 128, 0, s>>>(J, jbox, pitch, direction, istart, iend, iposition,
+  launch_next(k_antenna32, blocks_for(n, 128), 128, s, J, jbox, pitch, direction, istart, iend, iposition,
                                                   (long long)std::llround(value / qJ));
   spiffe_note_launches(1);
   return (int)cudaGetLastError();

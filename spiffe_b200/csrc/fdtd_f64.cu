@@ -27,6 +27,7 @@ constexpr int BX = 32, BY = 8;
 // Ez and Er to their final values for this step (integrate.c:323-380).
 __global__ void __launch_bounds__(BX *BY) k_tm_e(DevMesh m, DevFields<double> f, Coef64 c)
 {
+  step_begin();
   const int ir = blockIdx.x * BX + threadIdx.x, iz = blockIdx.y * BY + threadIdx.y;
   const int nz = m.nz, nr = m.nr, P = m.pitch;
   if (ir > nr || iz > nz)
@@ -72,6 +73,7 @@ __global__ void __launch_bounds__(BX *BY) k_tm_e(DevMesh m, DevFields<double> f,
 // Bphi and Bphi2 (integrate.c:383-432), reading the final Ez and Er.
 __global__ void __launch_bounds__(BX *BY) k_tm_b(DevMesh m, DevFields<double> f, Coef64 c)
 {
+  step_begin();
   const int ir = blockIdx.x * BX + threadIdx.x, iz = blockIdx.y * BY + threadIdx.y;
   const int nz = m.nz, nr = m.nr, P = m.pitch;
   if (ir > nr || iz < 1 || iz > nz - 1)
@@ -134,6 +136,7 @@ __global__ void __launch_bounds__(BX *BY) k_tm_b(DevMesh m, DevFields<double> f,
 // Neumann end rows and on the Neumann top row.
 __global__ void __launch_bounds__(BX *BY) k_te_e(DevMesh m, DevFields<double> f, Coef64 c)
 {
+  step_begin();
   const int ir = blockIdx.x * BX + threadIdx.x, iz = blockIdx.y * BY + threadIdx.y;
   const int nz = m.nz, nr = m.nr, P = m.pitch;
   if (ir > nr || iz > nz)
@@ -153,6 +156,7 @@ __global__ void __launch_bounds__(BX *BY) k_te_e(DevMesh m, DevFields<double> f,
 // Br/Br2 and Bz/Bz2 (integrate.c:473-539), reading the final Ephi.
 __global__ void __launch_bounds__(BX *BY) k_te_b(DevMesh m, DevFields<double> f, Coef64 c)
 {
+  step_begin();
   const int ir = blockIdx.x * BX + threadIdx.x, iz = blockIdx.y * BY + threadIdx.y;
   const int nz = m.nz, nr = m.nr, P = m.pitch;
   if (ir > nr || iz > nz)
@@ -281,15 +285,15 @@ extern "C" int spiffe_fdtd64_step(const DevMesh *m, const DevFields<double> *f, 
   Coef64 c{t->cpz, t->cmz, t->bzf, t->cut0, t->cut1, t->fEr, t->topf, t->fEphi};
   dim3 block(BX, BY), grid((m->nr + 1 + BX - 1) / BX, (m->nz + 1 + BY - 1) / BY);
   if (m->modes & SPIFFE_FL_TM_FIELDS) {
-    k_tm_e<<<grid, block, 0, s>>>(*m, *f, c);
+    launch_next(k_tm_e, grid, block, s, *m, *f, c);
     spiffe_note_launches(1);
-    k_tm_b<<<grid, block, 0, s>>>(*m, *f, c);
+    launch_next(k_tm_b, grid, block, s, *m, *f, c);
     spiffe_note_launches(1);
   }
   if (m->modes & SPIFFE_FL_TE_FIELDS) {
-    k_te_e<<<grid, block, 0, s>>>(*m, *f, c);
+    launch_next(k_te_e, grid, block, s, *m, *f, c);
     spiffe_note_launches(1);
-    k_te_b<<<grid, block, 0, s>>>(*m, *f, c);
+    launch_next(k_te_b, grid, block, s, *m, *f, c);
     spiffe_note_launches(1);
   }
   return (int)cudaGetLastError();

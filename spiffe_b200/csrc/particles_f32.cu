@@ -91,7 +91,7 @@ __device__ void gather32(const DevMesh &m, const DevFields32 &f, int iz0, float 
   float Ez = 0, Er = 0, Ephi = 0, Bz = 0, Br = 0, Bphi = 0;
   // 32-bit node offsets (a mesh holds fewer than 2^31 nodes) and read-only loads
 #define N(a, b) ((a) * P + (b))
-#define LD(arr, i) __ldg((arr) + (i))
+#define LD(arr, i) ((arr)[i]) // plain: the fields are written while this kernel waits for its turn (step_begin)
   // Ez and Br (:649-710)
   if (longit) {
     shift(iz0, fz, 0.5f, iz, wr);
@@ -286,8 +286,8 @@ __device__ __forceinline__ bool gather_inner(const DevMesh &m, const DevFields32
   const float wz = tz - (float)hz, wr = tr - (float)hr; // weights of the half-way stencils' upper rows, columns
   const int i = iz * P + ir, iE = i + hz * P, iR = i + hr, iB = iE + hr;
   const uint8_t mE = __ldg(f.umask + iE), mR = __ldg(f.umask + iR);
-#define L4(arr, k) const float arr##0 = __ldg(f.arr + (k)), arr##1 = __ldg(f.arr + (k) + 1), \
-                               arr##2 = __ldg(f.arr + (k) + P), arr##3 = __ldg(f.arr + (k) + P + 1)
+#define L4(arr, k) const float arr##0 = f.arr[k], arr##1 = f.arr[(k) + 1], arr##2 = f.arr[(k) + P], \
+                               arr##3 = f.arr[(k) + P + 1]
   L4(Ez, iE);
   L4(EzImposed, iE);
   L4(Er, iR);
@@ -602,6 +602,7 @@ template <bool DEP, bool DEF>
 __global__ void __launch_bounds__(T, 5) k_push32(DevMesh m, DevFields32 f, DevBeam32 b, Push32Params p, DevScreens scr,
                                                DevCounts *cnt, int32_t *lost_list, S32Scales sc)
 {
+  step_begin();
   const long ip = (long)blockIdx.x * T + threadIdx.x;
   const long np = (long)cnt->np;
   const bool valid = ip < np;
@@ -901,6 +902,7 @@ __global__ void k_reset_onaxis32(DevCounts *cnt)
 // The reference's removal: the first lost index ends the beam (:490-518 as released).
 __global__ void k_compact_reference32(DevCounts *cnt, int oa)
 {
+  step_begin();
   const bool cut = cnt->n_lost && cnt->first_lost < cnt->np;
   end_push(cnt, cut ? cnt->np - cnt->first_lost : 0, cut ? cnt->first_lost : cnt->np, oa);
 }
@@ -930,6 +932,7 @@ __device__ __forceinline__ void move32(const DevBeam32 &b, long dst, long src)
 __global__ void __launch_bounds__(CT) k_compact_any32(DevBeam32 b, const int32_t *lost_list, DevCounts *cnt,
                                                        int32_t *holes, int32_t *donors, int oa)
 {
+  step_begin();
   const long long n_lost = cnt->n_lost, np = cnt->np;
   if (n_lost > 0)
     compact_block<false>(
@@ -1398,13 +1401,13 @@ extern "C" int s32_push(const DevMesh *m, const DevFields32 *f, const DevBeam32 
     int32_t *ll = any ? w->lost_list : nullptr;
     const unsigned nb = blocks_for(np_bound, T);
     if (p->deposit && def)
-      k_push32<true, true><<<nb, T, 0, s>>>(*m, *f, *b, *p, *scr, cnt, ll, *sc);
+      launch_next(k_push32<true, true>, nb, T, s, *m, *f, *b, *p, *scr, cnt, ll, *sc);
     else if (p->deposit)
-      k_push32<true, false><<<nb, T, 0, s>>>(*m, *f, *b, *p, *scr, cnt, ll, *sc);
+      launch_next(k_push32<true, false>, nb, T, s, *m, *f, *b, *p, *scr, cnt, ll, *sc);
     else if (def)
-      k_push32<false, true><<<nb, T, 0, s>>>(*m, *f, *b, *p, *scr, cnt, ll, *sc);
+      launch_next(k_push32<false, true>, nb, T, s, *m, *f, *b, *p, *scr, cnt, ll, *sc);
     else
-      k_push32<false, false><<<nb, T, 0, s>>>(*m, *f, *b, *p, *scr, cnt, ll, *sc);
+      launch_next(k_push32<false, false>, nb, T, s, *m, *f, *b, *p, *scr, cnt, ll, *sc);
     spiffe_note_launches(1);
     if (p->lost.rec) {
       k_lost32<<<blocks_for(p->lost.cap, T), T, 0, s>>>(*m, f->flags, *b, p->lost);
@@ -1412,9 +1415,9 @@ extern "C" int s32_push(const DevMesh *m, const DevFields32 *f, const DevBeam32 
     }
   }
   if (!any) {
-    k_compact_reference32<<<1, 1, 0, s>>>(cnt, oa);
+    launch_next(k_compact_reference32, 1, 1, s, cnt, oa);
   } else {
-    k_compact_any32<<<1, CT, 0, s>>>(*b, w->lost_list, cnt, w->keys, w->idx, oa);
+    launch_next(k_compact_any32, 1, CT, s, *b, w->lost_list, cnt, w->keys, w->idx, oa);
   }
   spiffe_note_launches(1);
   return (int)cudaGetLastError();

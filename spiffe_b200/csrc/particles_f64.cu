@@ -277,6 +277,7 @@ __global__ void k_snapshot_last(DevBeam64 b, DevCounts *cnt)
 __global__ void __launch_bounds__(T) k_push(DevMesh m, DevFields<double> f, DevBeam64 b, PushParams p,
                                              DevScreens scr, DevCounts *cnt, uint8_t *lost_flag, int32_t *lost_list)
 {
+  step_begin();
   const long ip = (long)blockIdx.x * T + threadIdx.x;
   const long np = (long)cnt->np;
   if (ip >= np)
@@ -679,6 +680,7 @@ __global__ void __launch_bounds__(T) k_deposit(DevMesh m, DevFields<double> f, D
                                                 int component, int *keys, double *vals, long long n_slots, int stride,
                                                 int pad)
 {
+  step_begin();
   const long ip = (long)blockIdx.x * T + threadIdx.x;
   const long np = (long)cnt->np;
   if (ip >= np) {
@@ -807,6 +809,7 @@ __global__ void __launch_bounds__(T) k_ordered_sum(const int *keys, const double
 // Reference compaction: the first lost index ends the beam.
 __global__ void k_compact_reference(DevCounts *cnt, int oa)
 {
+  step_begin();
   const bool cut = cnt->n_lost && cnt->first_lost < cnt->np;
   end_push(cnt, cut ? cnt->np - cnt->first_lost : 0, cut ? cnt->first_lost : cnt->np, oa);
 }
@@ -818,6 +821,7 @@ __global__ void k_compact_reference(DevCounts *cnt, int oa)
 __global__ void __launch_bounds__(CT) k_compact_swap(DevBeam64 b, const uint8_t *lost, const int32_t *lost_list,
                                                       DevCounts *cnt, int32_t *holes, int32_t *donors, int oa)
 {
+  step_begin();
   const long long n_lost = cnt->n_lost, np = cnt->np;
   if (n_lost > 0)
     compact_block<true>(
@@ -892,11 +896,11 @@ extern "C" int spiffe_deposit64(const DevMesh *m, const DevFields<double> *f, co
     if (comp == 2 && !(m->modes & SPIFFE_FL_TE_FIELDS))
       continue;
     if (!ordered) {
-      k_deposit<<<nb, T, 0, s>>>(*m, *f, *b, cnt, comp, nullptr, nullptr, 0, stride, nodes);
+      launch_next(k_deposit, nb, T, s, *m, *f, *b, cnt, comp, nullptr, nullptr, 0, stride, nodes);
       spiffe_note_launches(1);
       continue;
     }
-    k_deposit<<<nb, T, 0, s>>>(*m, *f, *b, cnt, comp, w->keys, w->vals, np_bound, stride, nodes);
+    launch_next(k_deposit, nb, T, s, *m, *f, *b, cnt, comp, w->keys, w->vals, np_bound, stride, nodes);
     spiffe_note_launches(1);
     double *J = comp == 0 ? f->Jz : (comp == 1 ? f->Jr : f->Jphi);
     if (int rc = spiffe_ordered_add64(w, stride * np_bound, nodes, J, s))
@@ -969,13 +973,13 @@ extern "C" int spiffe_push64(const DevMesh *m, const DevFields<double> *f, const
                  hp->tb_r_force, hp->tb_z_decel, hp->tb_r_decel, hp->screen_momentum, hp->lost};
     if (scr->n && hp->screen_momentum == SPIFFE_SCREEN_REFERENCE)
       { k_snapshot_last<<<1, 1, 0, s>>>(*b, cnt); spiffe_note_launches(1); }
-    k_push<<<blocks_for(np_bound, T), T, 0, s>>>(*m, *f, *b, p, *scr, cnt, w->lost, w->lost_list);
+    launch_next(k_push, blocks_for(np_bound, T), T, s, *m, *f, *b, p, *scr, cnt, w->lost, w->lost_list);
     spiffe_note_launches(1);
   }
   if (hp->compaction == SPIFFE_COMPACT_REFERENCE || np_bound <= 0)
-    k_compact_reference<<<1, 1, 0, s>>>(cnt, oa);
+    launch_next(k_compact_reference, 1, 1, s, cnt, oa);
   else
-    k_compact_swap<<<1, CT, 0, s>>>(*b, w->lost, w->lost_list, cnt, w->holes, w->donors, oa);
+    launch_next(k_compact_swap, 1, CT, s, *b, w->lost, w->lost_list, cnt, w->holes, w->donors, oa);
   spiffe_note_launches(1);
   return (int)cudaGetLastError();
 }
