@@ -27,33 +27,44 @@ struct Coef32 {
   int reset_box; // this B kernel is the step's last: empty the current box
 };
 
-// rows [lo, hi] of the current box (lo > hi: no current anywhere)
-__device__ __forceinline__ void jbox_rows(const int *jbox, int &lo, int &hi)
+// The current box: rows x..y, columns z..w (x > y: no current anywhere).  J is
+// 32 bytes a node to read and as many to clear, more than the fields' 21, so
+// the box keeps columns too: a bunch near the axis, or an antenna's line, has
+// few of its rows' columns (build-up on 3001 x 821 with an antenna: 2 % less).
+__device__ __forceinline__ int4 jbox_read(const int *jbox) { return *reinterpret_cast<const int4 *>(jbox); }
+__device__ __forceinline__ bool jbox_has(const int4 &b, int iz, int ir0, int ir1) // any of row iz's columns ir0..ir1
 {
-  lo = jbox[0];
-  hi = jbox[1];
+  return iz >= b.x && iz <= b.y && ir1 >= b.z && ir0 <= b.w;
+}
+constexpr int JBOX_NONE = 0x7fffffff;
+__device__ __forceinline__ void jbox_empty(int *jbox)
+{
+  *reinterpret_cast<int4 *>(jbox) = make_int4(JBOX_NONE, -1, JBOX_NONE, -1);
 }
 
 __device__ __forceinline__ void jbox_reset(int *jbox)
 {
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
-    jbox[0] = 0x7fffffff;
-    jbox[1] = -1;
-  }
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0)
+    jbox_empty(jbox);
 }
 
 // ---- the arithmetic of one node, each product and sum rounded on its own
 // (no contraction), shared by the per-node, tiled and fused kernels so that
 // all three give the same bits.
+__device__ __forceinline__ float ez_curl(float cp, float b1, float cm, float b0)
+{
+  return __fsub_rn(__fmul_rn(cp, b1), __fmul_rn(cm, b0));
+}
+__device__ __forceinline__ float er_curl(float fEr, float bP, float b0) { return __fmul_rn(fEr, __fsub_rn(bP, b0)); }
 // Ez (integrate.c:323-344): ez + (kJ jz + (cp b1 - cm b0))
 __device__ __forceinline__ float ez_next(float ez, float kJ, float jz, float cp, float b1, float cm, float b0)
 {
-  return __fadd_rn(ez, __fadd_rn(__fmul_rn(kJ, jz), __fsub_rn(__fmul_rn(cp, b1), __fmul_rn(cm, b0))));
+  return __fadd_rn(ez, __fadd_rn(__fmul_rn(kJ, jz), ez_curl(cp, b1, cm, b0)));
 }
 // Er (integrate.c:362-368): er + (kJ jr - fEr (bP - b0))
 __device__ __forceinline__ float er_next(float er, float kJ, float jr, float fEr, float bP, float b0)
 {
-  return __fadd_rn(er, __fsub_rn(__fmul_rn(kJ, jr), __fmul_rn(fEr, __fsub_rn(bP, b0))));
+  return __fadd_rn(er, __fsub_rn(__fmul_rn(kJ, jr), er_curl(fEr, bP, b0)));
 }
 // dBphi (integrate.c:391-394): dt/dr (ez - ezm) - dt/dz (er - erm)
 __device__ __forceinline__ float dbphi(float dt_dr, float ez, float ezm, float dt_dz, float er, float erm)
@@ -65,17 +76,17 @@ __device__ __forceinline__ float half_step(float b, float dB) { return __fadd_rn
 // ---- TM update, one node at a time: the boundary rows and columns
 // (copies to the axis, the top and the end rows) and the cells next to them.
 
-// Ez and Er of node (iz, ir), 0 <= iz <= nz, 0 <= ir <= nr; J rows jlo..jhi
+// Ez and Er of node (iz, ir), 0 <= iz <= nz, 0 <= ir <= nr; J in the box
 __device__ __forceinline__ void tm_e_node(const DevMesh &m, const DevFields32 &f, const Coef32 &c, int iz, int ir,
-                                          int jlo, int jhi)
+                                          const int4 &box)
 {
   const int nz = m.nz, nr = m.nr, P = m.pitch;
   const size_t i = node(iz, ir, P);
   const bool leftN = m.left_bc == SPIFFE_NEUMANN, rightN = m.right_bc == SPIFFE_NEUMANN;
   const bool ez_row = ir < nr && iz >= 1 && iz <= nz - 1, er_row = iz <= nz - 1;
   // every load before any store, so no store can order the loads behind it;
-  // J is read (and cleared) only on the rows a deposit touched
-  const bool jrow = iz >= jlo && iz <= jhi;
+  // J is read (and cleared) only in the box that deposits touched
+  const bool jrow = jbox_has(box, iz, ir, ir);
   const uint8_t u = f.umask[i];
   const long long jz = jrow ? f.Jz[i] : 0, jr = jrow ? f.Jr[i] : 0;
   const float ez = ez_row ? f.Ez[i] : 0.f, er = er_row ? f.Er[i] : 0.f;
@@ -244,12 +255,11 @@ __device__ __forceinline__ void tm_boundary_node(const TmSplit &t, int nz, int n
   }
 }
 
-__global__ void __launch_bounds__(VX *VY) k_tm_e32(DevMesh m, DevFields32 f, Coef32 c, TmSplit t)
+__global__ void __launch_bounds__(VX *VY, 6) k_tm_e32(DevMesh m, DevFields32 f, Coef32 c, TmSplit t)
 {
   step_begin();
   const int nz = m.nz, nr = m.nr, P = m.pitch;
-  int jlo, jhi;
-  jbox_rows(f.jbox, jlo, jhi);
+  const int4 box = jbox_read(f.jbox);
   // the boundary blocks come first, so they run beside the tiles, not after them
   const int nbb = (int)((t.nb + VX * VY - 1) / (VX * VY));
   if ((int)blockIdx.x < nbb) {
@@ -257,7 +267,7 @@ __global__ void __launch_bounds__(VX *VY) k_tm_e32(DevMesh m, DevFields32 f, Coe
     if (k < t.nb) {
       int iz, ir;
       tm_boundary_node(t, nz, nr, false, k, iz, ir);
-      tm_e_node(m, f, c, iz, ir, jlo, jhi);
+      tm_e_node(m, f, c, iz, ir, box);
     }
     return;
   }
@@ -269,11 +279,10 @@ __global__ void __launch_bounds__(VX *VY) k_tm_e32(DevMesh m, DevFields32 f, Coe
   const int ir0 = g * VW;
   const bool mine = g <= t.G, in_row = ir0 <= nr;
   const size_t i = node(iz, ir0, P);
-  const bool jrow = iz >= jlo && iz <= jhi;
+  const bool jrow = jbox_has(box, iz, ir0, ir0 + VW - 1);
   // every load first; the next group's first Bphi comes from the next lane
   float4 b0 = make_float4(0.f, 0.f, 0.f, 0.f), ez = b0, er = b0, bP = b0, cp = b0, cm = b0;
   uchar4 u = make_uchar4(0, 0, 0, 0);
-  longlong2 z01 = make_longlong2(0, 0), z23 = z01, r01 = z01, r23 = z01;
   float bnext = 0.f;
   if (in_row)
     b0 = ld4(f.Bphi + i);
@@ -284,12 +293,6 @@ __global__ void __launch_bounds__(VX *VY) k_tm_e32(DevMesh m, DevFields32 f, Coe
     bP = ld4(f.Bphi + i + P);
     cp = ldg4(c.cpd + ir0);
     cm = ldg4(c.cmd + ir0);
-    if (jrow) {
-      z01 = *reinterpret_cast<const longlong2 *>(f.Jz + i);
-      z23 = *reinterpret_cast<const longlong2 *>(f.Jz + i + 2);
-      r01 = *reinterpret_cast<const longlong2 *>(f.Jr + i);
-      r23 = *reinterpret_cast<const longlong2 *>(f.Jr + i + 2);
-    }
     if (threadIdx.x == VX - 1)
       bnext = f.Bphi[i + VW]; // ir0 + 4 <= nr - 1: inside the row
   }
@@ -298,26 +301,44 @@ __global__ void __launch_bounds__(VX *VY) k_tm_e32(DevMesh m, DevFields32 f, Coe
     return;
   if (threadIdx.x != VX - 1)
     bnext = bsh;
-  const float jz0 = (float)z01.x, jz1 = (float)z01.y, jz2 = (float)z23.x, jz3 = (float)z23.y;
-  const float jr0 = (float)r01.x, jr1 = (float)r01.y, jr2 = (float)r23.x, jr3 = (float)r23.y;
-  // integrate.c:323-344 and :362-368 on four interior nodes
-  if (u.x & S32_U_EZ) ez.x = ez_next(ez.x, c.kJ, jz0, cp.x, b0.y, cm.x, b0.x);
-  if (u.y & S32_U_EZ) ez.y = ez_next(ez.y, c.kJ, jz1, cp.y, b0.z, cm.y, b0.y);
-  if (u.z & S32_U_EZ) ez.z = ez_next(ez.z, c.kJ, jz2, cp.z, b0.w, cm.z, b0.z);
-  if (u.w & S32_U_EZ) ez.w = ez_next(ez.w, c.kJ, jz3, cp.w, bnext, cm.w, b0.w);
-  if (u.x & S32_U_ER) er.x = er_next(er.x, c.kJ, jr0, c.fEr, bP.x, b0.x);
-  if (u.y & S32_U_ER) er.y = er_next(er.y, c.kJ, jr1, c.fEr, bP.y, b0.y);
-  if (u.z & S32_U_ER) er.z = er_next(er.z, c.kJ, jr2, c.fEr, bP.z, b0.z);
-  if (u.w & S32_U_ER) er.w = er_next(er.w, c.kJ, jr3, c.fEr, bP.w, b0.w);
+  // integrate.c:323-344 and :362-368 on four interior nodes: the curl terms, then J's
+  float4 dz, dr;
+  dz.x = ez_curl(cp.x, b0.y, cm.x, b0.x);
+  dz.y = ez_curl(cp.y, b0.z, cm.y, b0.y);
+  dz.z = ez_curl(cp.z, b0.w, cm.z, b0.z);
+  dz.w = ez_curl(cp.w, bnext, cm.w, b0.w);
+  dr.x = er_curl(c.fEr, bP.x, b0.x);
+  dr.y = er_curl(c.fEr, bP.y, b0.y);
+  dr.z = er_curl(c.fEr, bP.z, b0.z);
+  dr.w = er_curl(c.fEr, bP.w, b0.w);
+  if (jrow) { // few nodes: their J may be waited for
+    longlong2 *Jz = reinterpret_cast<longlong2 *>(f.Jz + i), *Jr = reinterpret_cast<longlong2 *>(f.Jr + i);
+    const longlong2 zero = make_longlong2(0, 0), z01 = Jz[0], z23 = Jz[1], r01 = Jr[0], r23 = Jr[1];
+    dz.x = __fadd_rn(__fmul_rn(c.kJ, (float)z01.x), dz.x);
+    dz.y = __fadd_rn(__fmul_rn(c.kJ, (float)z01.y), dz.y);
+    dz.z = __fadd_rn(__fmul_rn(c.kJ, (float)z23.x), dz.z);
+    dz.w = __fadd_rn(__fmul_rn(c.kJ, (float)z23.y), dz.w);
+    dr.x = __fsub_rn(__fmul_rn(c.kJ, (float)r01.x), dr.x);
+    dr.y = __fsub_rn(__fmul_rn(c.kJ, (float)r01.y), dr.y);
+    dr.z = __fsub_rn(__fmul_rn(c.kJ, (float)r23.x), dr.z);
+    dr.w = __fsub_rn(__fmul_rn(c.kJ, (float)r23.y), dr.w);
+    if (c.zero_j) {
+      Jz[0] = Jz[1] = zero;
+      Jr[0] = Jr[1] = zero;
+    }
+  } else { // kJ 0 adds nothing
+    dr = make_float4(-dr.x, -dr.y, -dr.z, -dr.w);
+  }
+  if (u.x & S32_U_EZ) ez.x = __fadd_rn(ez.x, dz.x);
+  if (u.y & S32_U_EZ) ez.y = __fadd_rn(ez.y, dz.y);
+  if (u.z & S32_U_EZ) ez.z = __fadd_rn(ez.z, dz.z);
+  if (u.w & S32_U_EZ) ez.w = __fadd_rn(ez.w, dz.w);
+  if (u.x & S32_U_ER) er.x = __fadd_rn(er.x, dr.x);
+  if (u.y & S32_U_ER) er.y = __fadd_rn(er.y, dr.y);
+  if (u.z & S32_U_ER) er.z = __fadd_rn(er.z, dr.z);
+  if (u.w & S32_U_ER) er.w = __fadd_rn(er.w, dr.w);
   st4(f.Ez + i, ez);
   st4(f.Er + i, er);
-  if (c.zero_j && jrow) {
-    const longlong2 zero = make_longlong2(0, 0);
-    *reinterpret_cast<longlong2 *>(f.Jz + i) = zero;
-    *reinterpret_cast<longlong2 *>(f.Jz + i + 2) = zero;
-    *reinterpret_cast<longlong2 *>(f.Jr + i) = zero;
-    *reinterpret_cast<longlong2 *>(f.Jr + i + 2) = zero;
-  }
 }
 
 __global__ void __launch_bounds__(VX *VY) k_tm_b32(DevMesh m, DevFields32 f, Coef32 c, TmSplit t)
@@ -522,8 +543,7 @@ __global__ void k_tm_fused32(DevMesh m, DevFields32 f, Coef32 c, FusedArgs a)
     __threadfence();
     if (atomicAdd(a.arrivals, 1u) == (unsigned)a.bands - 1) {
       *a.arrivals = 0;
-      f.jbox[0] = 0x7fffffff;
-      f.jbox[1] = -1;
+      jbox_empty(f.jbox);
     }
   }
   auto jrow = [&](int iz) { return iz >= jlo && iz <= jhi; };
@@ -798,9 +818,7 @@ __global__ void __launch_bounds__(BX *BY) k_te_e32(DevMesh m, DevFields32 f, Coe
   if (ir > nr || iz > nz)
     return;
   const size_t i = node(iz, ir, P);
-  int jlo, jhi;
-  jbox_rows(f.jbox, jlo, jhi);
-  const bool jrow = iz >= jlo && iz <= jhi;
+  const bool jrow = jbox_has(jbox_read(f.jbox), iz, ir, ir);
   const long long jphi = jrow ? f.Jphi[i] : 0;
   if (c.zero_j && jrow)
     f.Jphi[i] = 0;
@@ -928,12 +946,13 @@ __global__ void k_antenna32(long long *J, int *jbox, int P, int direction, long 
   J[nd] += v;
   atomicMin(jbox, nd / P);
   atomicMax(jbox + 1, nd / P);
+  atomicMin(jbox + 2, nd % P);
+  atomicMax(jbox + 3, nd % P);
 }
 
 __global__ void k_jbox_set(int *jbox, int lo, int hi)
 {
-  jbox[0] = lo;
-  jbox[1] = hi;
+  *reinterpret_cast<int4 *>(jbox) = lo <= hi ? make_int4(lo, hi, 0, JBOX_NONE) : make_int4(JBOX_NONE, -1, JBOX_NONE, -1);
 }
 
 // a >>= shift with rounding to nearest: values in old quanta to quanta 2^shift times larger

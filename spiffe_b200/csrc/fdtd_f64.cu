@@ -9,6 +9,7 @@
 // FL_LAST_ACTIVE_PT" rule (integrate.c:345-346) becomes a per-row cut-off
 // index computed once on the host.  Built with -fmad=false so every product
 // and sum rounds as the reference's does.
+#include "divide.cuh"
 #include "modules.cuh"
 
 namespace {
@@ -20,12 +21,23 @@ struct Coef64 {
   double fEr;              // 1/(mu0 eps0 dz), integrate.c:362
   double topf;             // (rmax-dr/2)/(rmax+dr/2), integrate.c:384
   double fEphi;            // 1/(eps0 mu0), integrate.c:450
+  double y_eps, y_dz, y_dr; // 1/eps0, 1/dz, 1/dr
 };
+
+// TM kernels, TAKES: dz and dr lie where div_by holds (else plain divisions).
+// A node's two quotients were most of the instructions of either kernel; they
+// are the reference's divisions by eps0, dr and dz, correctly rounded, by a
+// product and corrections (div_by).
+// FDTD64FIG
+template <bool TAKES> __device__ __forceinline__ double over(double x, double e, double y)
+{
+  return TAKES ? div_by(x, e, y) : x / e;
+}
 
 constexpr int BX = 32, BY = 8;
 
 // Ez and Er to their final values for this step (integrate.c:323-380).
-__global__ void __launch_bounds__(BX *BY) k_tm_e(DevMesh m, DevFields<double> f, Coef64 c)
+template <bool TAKES> __global__ void __launch_bounds__(BX *BY) k_tm_e(DevMesh m, DevFields<double> f, Coef64 c)
 {
   step_begin();
   const int ir = blockIdx.x * BX + threadIdx.x, iz = blockIdx.y * BY + threadIdx.y;
@@ -45,7 +57,7 @@ __global__ void __launch_bounds__(BX *BY) k_tm_e(DevMesh m, DevFields<double> f,
     } else {
       v = f.Ez[i];
       if (iz <= c.cut1[ir] && !(fl & SPIFFE_FL_EZ_ZERO))
-        v += dti * (-f.Jz[i] / eps0 + (c.cpz[ir] * f.Bphi[i + 1] - c.cmz[ir] * f.Bphi[i]));
+        v += dti * (over<TAKES>(-f.Jz[i], eps0, c.y_eps) + (c.cpz[ir] * f.Bphi[i + 1] - c.cmz[ir] * f.Bphi[i]));
     }
     f.Ez[i] = v;
     if (iz == 1)
@@ -60,7 +72,7 @@ __global__ void __launch_bounds__(BX *BY) k_tm_e(DevMesh m, DevFields<double> f,
     if (ir >= 1 && ir <= nr - 1) {
       double v = f.Er[i];
       if (iz <= c.cut0[ir] && !(fl & SPIFFE_FL_ER_ZERO))
-        v += dti * (-f.Jr[i] / eps0 - c.fEr * (f.Bphi[i + P] - f.Bphi[i]));
+        v += dti * (over<TAKES>(-f.Jr[i], eps0, c.y_eps) - c.fEr * (f.Bphi[i + P] - f.Bphi[i]));
       f.Er[i] = zero_row ? 0.0 : v;
       if (ir == 1)
         f.Er[node(iz, 0, P)] = zero_row ? 0.0 : -v;
@@ -71,7 +83,7 @@ __global__ void __launch_bounds__(BX *BY) k_tm_e(DevMesh m, DevFields<double> f,
 }
 
 // Bphi and Bphi2 (integrate.c:383-432), reading the final Ez and Er.
-__global__ void __launch_bounds__(BX *BY) k_tm_b(DevMesh m, DevFields<double> f, Coef64 c)
+template <bool TAKES> __global__ void __launch_bounds__(BX *BY) k_tm_b(DevMesh m, DevFields<double> f, Coef64 c)
 {
   step_begin();
   const int ir = blockIdx.x * BX + threadIdx.x, iz = blockIdx.y * BY + threadIdx.y;
@@ -82,13 +94,15 @@ __global__ void __launch_bounds__(BX *BY) k_tm_b(DevMesh m, DevFields<double> f,
   const bool leftN = m.left_bc == SPIFFE_NEUMANN, rightN = m.right_bc == SPIFFE_NEUMANN;
   const size_t i = node(iz, ir, P);
   if (ir >= 1 && ir <= nr - 2) {
-    double b = f.Bphi[i], b2 = f.Bphi2[i];
+    double b = f.Bphi[i], b2;
     if (iz <= c.cut1[ir] && !(f.flags[i] & SPIFFE_FL_BPHI_ZERO)) {
-      const double dB = dti * ((f.Ez[i] - f.Ez[i - 1]) / dr - (f.Er[i] - f.Er[i - P]) / dz);
+      const double dB = dti * (over<TAKES>(f.Ez[i] - f.Ez[i - 1], dr, c.y_dr) - over<TAKES>(f.Er[i] - f.Er[i - P], dz, c.y_dz));
       b2 = b + dB / 2;
       b += dB;
       f.Bphi2[i] = b2;
       f.Bphi[i] = b;
+    } else {
+      b2 = f.Bphi2[i];
     }
     // axis and top copies of this row
     if (ir == 1) {
@@ -282,12 +296,14 @@ extern "C" void spiffe_fdtd64_tables_free(Fdtd64Tables *t)
 // One advance_field_solutions: TM (E then B), then TE (Ephi then B).
 extern "C" int spiffe_fdtd64_step(const DevMesh *m, const DevFields<double> *f, const Fdtd64Tables *t, cudaStream_t s)
 {
-  Coef64 c{t->cpz, t->cmz, t->bzf, t->cut0, t->cut1, t->fEr, t->topf, t->fEphi};
+  Coef64 c{t->cpz, t->cmz, t->bzf, t->cut0, t->cut1, t->fEr, t->topf, t->fEphi,
+           1 / SPIFFE_EPSILON_O, 1 / m->dz, 1 / m->dr};
+  const bool takes = div_by_takes(m->dz) && div_by_takes(m->dr);
   dim3 block(BX, BY), grid((m->nr + 1 + BX - 1) / BX, (m->nz + 1 + BY - 1) / BY);
   if (m->modes & SPIFFE_FL_TM_FIELDS) {
-    launch_next(k_tm_e, grid, block, s, *m, *f, c);
+    launch_next(takes ? k_tm_e<true> : k_tm_e<false>, grid, block, s, *m, *f, c);
     spiffe_note_launches(1);
-    launch_next(k_tm_b, grid, block, s, *m, *f, c);
+    launch_next(takes ? k_tm_b<true> : k_tm_b<false>, grid, block, s, *m, *f, c);
     spiffe_note_launches(1);
   }
   if (m->modes & SPIFFE_FL_TE_FIELDS) {

@@ -441,6 +441,23 @@ __device__ __forceinline__ void warp_add(long long *J, int nd, long long v)
   }
 }
 
+// Widens the box of nodes holding current (the FDTD reads and clears only
+// those) to the rows rlo..rhi and the columns up to col; a warp skips the
+// atomics when the box already covers it.  Its columns begin at the axis, near
+// which particles mostly are.
+__device__ __forceinline__ void widen_box(int *jbox, int rlo, int rhi, int col)
+{
+  const int4 b = *reinterpret_cast<const int4 *>(jbox);
+  if (rlo < b.x)
+    atomicMin(jbox, rlo);
+  if (rhi > b.y)
+    atomicMax(jbox + 1, rhi);
+  if (b.z > 0)
+    atomicMin(jbox + 2, 0);
+  if (col > b.w)
+    atomicMax(jbox + 3, col);
+}
+
 // Deposits the three components of one particle (or nothing, when !on);
 // called by every lane of the warp.
 template <bool DEF>
@@ -471,17 +488,11 @@ __device__ void deposit_particle(const DevMesh &m, const DevFields32 &f, bool on
       }
     }
   }
-  // widen the box of rows holding current (the FDTD reads and clears only
-  // those rows); a warp skips the atomics when the box already covers it
   lo = __reduce_min_sync(0xffffffffu, lo);
   hi = __reduce_max_sync(0xffffffffu, hi);
-  if ((threadIdx.x & 31) == 0 && lo <= hi) {
-    const int rlo = (int)(lo / (unsigned)m.pitch), rhi = (int)(hi / (unsigned)m.pitch);
-    if (rlo < f.jbox[0])
-      atomicMin(f.jbox, rlo);
-    if (rhi > f.jbox[1])
-      atomicMax(f.jbox + 1, rhi);
-  }
+  const int col = __reduce_max_sync(0xffffffffu, on ? ir + 2 : 0);
+  if ((threadIdx.x & 31) == 0 && lo <= hi)
+    widen_box(f.jbox, (int)(lo / (unsigned)m.pitch), (int)(hi / (unsigned)m.pitch), col);
 }
 
 // deposit_particle<true> of a particle that may be known to lie in a cell
@@ -526,12 +537,9 @@ __device__ __forceinline__ void deposit_inner(const DevMesh &m, const DevFields3
   warp_add(f.Jr, nr_, qr);
   lo = __reduce_min_sync(0xffffffffu, lo);
   hi = __reduce_max_sync(0xffffffffu, hi);
-  if ((threadIdx.x & 31) == 0 && lo <= hi) {
-    if ((int)lo < f.jbox[0])
-      atomicMin(f.jbox, (int)lo);
-    if ((int)hi > f.jbox[1])
-      atomicMax(f.jbox + 1, (int)hi);
-  }
+  const int col = __reduce_max_sync(0xffffffffu, on ? ir + 2 : 0);
+  if ((threadIdx.x & 31) == 0 && lo <= hi)
+    widen_box(f.jbox, (int)lo, (int)hi, col);
 }
 
 // v/c of a particle from its momenta at radius r (setParticleVelocities, :605-620)

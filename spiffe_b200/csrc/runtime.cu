@@ -562,7 +562,7 @@ static int s32_create(spiffe_gpu_instance *in, const int16_t *flags)
   d.add(&S.f.PsiImposed, n);
   d.add(&S.f.Q, n);
   d.add(&S.f.Qp, n);
-  d.add(&S.f.jbox, 2);
+  d.add(&S.f.jbox, 4);
   CUDA_TRY(d.make());
   CUDA_TRY(cudaMemsetAsync(in->slab, 0, d.bytes(), s));
   CUDA_TRY(cudaMemcpy2DAsync(in->d_flags, (size_t)P * sizeof(int16_t), flags, (size_t)(nr + 1) * sizeof(int16_t),

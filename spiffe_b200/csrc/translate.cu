@@ -59,6 +59,8 @@ __global__ void k_jbox_down(int *jbox)
   if (hi < lo) {
     lo = 0x7fffffff;
     hi = -1;
+    jbox[2] = 0x7fffffff;
+    jbox[3] = -1;
   }
   jbox[0] = lo;
   jbox[1] = hi;
