@@ -144,6 +144,7 @@ struct DevFields {
   T *Ephi, *Jphi, *Br, *Br2, *Bz, *Bz2;
   T *EzImposed, *ErImposed, *PsiImposed, *BzImposed, *BrImposed;
   T *Psi, *Q;
+  int *jbox; // the box of current, and (at [4]) the blocks that have read it in a clearing
 };
 
 // FP64 structure-of-arrays beam (BEAM, spiffe.h:201-221).
@@ -308,6 +309,39 @@ __host__ __device__ inline size_t node(int iz, int ir, int pitch) { return (size
 __device__ __forceinline__ long long atomic_add_ll(long long *p, long long v)
 {
   return (long long)atomicAdd((unsigned long long *)p, (unsigned long long)v);
+}
+#endif
+
+#ifdef __CUDACC__
+// The box of nodes that may hold current, on the device: rows x..y, columns
+// z..w (x > y: none).  Deposits widen it, the field update reads J only in it
+// and it alone is cleared: a bunch near the axis, or an antenna's line, covers
+// few of the mesh's nodes, and J is 16 (FP64) or 32 (split form: read and
+// cleared) bytes a node beside the fields' 42 or 21.
+constexpr int JBOX_NONE = 0x7fffffff;
+__device__ __forceinline__ int4 jbox_read(const int *jbox) { return *reinterpret_cast<const int4 *>(jbox); }
+__device__ __forceinline__ bool jbox_has(const int4 &b, int iz, int ir0, int ir1) // any of row iz's columns ir0..ir1
+{
+  return iz >= b.x && iz <= b.y && ir1 >= b.z && ir0 <= b.w;
+}
+__device__ __forceinline__ void jbox_empty(int *jbox)
+{
+  *reinterpret_cast<int4 *>(jbox) = make_int4(JBOX_NONE, -1, JBOX_NONE, -1);
+}
+// Widens the box to the rows rlo..rhi and the columns up to col; a warp skips the
+// atomics when the box already covers it.  Its columns begin at the axis, near
+// which particles mostly are.
+__device__ __forceinline__ void widen_box(int *jbox, int rlo, int rhi, int col)
+{
+  const int4 b = *reinterpret_cast<const int4 *>(jbox);
+  if (rlo < b.x)
+    atomicMin(jbox, rlo);
+  if (rhi > b.y)
+    atomicMax(jbox + 1, rhi);
+  if (b.z > 0)
+    atomicMin(jbox + 2, 0);
+  if (col > b.w)
+    atomicMax(jbox + 3, col);
 }
 #endif
 

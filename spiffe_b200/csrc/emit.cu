@@ -173,17 +173,19 @@ __global__ void k_births_commit(long long total, long long capacity, int mode, D
   births_commit(total, capacity, mode, cnt);
 }
 
-__global__ void k_antenna(double *J, int P, int direction, long istart, long iend, long iposition, double value)
+__global__ void k_antenna(double *J, int *jbox, int P, int direction, long istart, long iend, long iposition, double value)
 {
   step_begin();
   const long i = istart + (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i > iend)
     return;
   // antenna.c:398-415
-  if (direction == 1)
-    J[node((int)iposition, (int)i, P)] += value;
-  else
-    J[node((int)i, (int)iposition, P)] += value;
+  const int iz = (int)(direction == 1 ? iposition : i), ir = (int)(direction == 1 ? i : iposition);
+  J[node(iz, ir, P)] += value;
+  atomicMin(jbox, iz);
+  atomicMax(jbox + 1, iz);
+  atomicMin(jbox + 2, ir);
+  atomicMax(jbox + 3, ir);
 }
 
 } // namespace
@@ -201,13 +203,13 @@ extern "C" int spiffe_births64(const DevMesh *m, const DevFields<double> *f, con
   return (int)cudaGetLastError();
 }
 
-extern "C" int spiffe_antenna64(double *J, int pitch, int direction, long istart, long iend, long iposition, double value,
+extern "C" int spiffe_antenna64(double *J, int *jbox, int pitch, int direction, long istart, long iend, long iposition, double value,
                                 cudaStream_t s)
 {
   if (iend < istart)
     return 0;
   const long n = iend - istart + 1;
-  launch_next(k_antenna, blocks_for(n, 128), 128, s, J, pitch, direction, istart, iend, iposition, value);
+  launch_next(k_antenna, blocks_for(n, 128), 128, s, J, jbox, pitch, direction, istart, iend, iposition, value);
   spiffe_note_launches(1);
   return (int)cudaGetLastError();
 }

@@ -27,21 +27,6 @@ struct Coef32 {
   int reset_box; // this B kernel is the step's last: empty the current box
 };
 
-// The current box: rows x..y, columns z..w (x > y: no current anywhere).  J is
-// 32 bytes a node to read and as many to clear, more than the fields' 21, so
-// the box keeps columns too: a bunch near the axis, or an antenna's line, has
-// few of its rows' columns (build-up on 3001 x 821 with an antenna: 2 % less).
-__device__ __forceinline__ int4 jbox_read(const int *jbox) { return *reinterpret_cast<const int4 *>(jbox); }
-__device__ __forceinline__ bool jbox_has(const int4 &b, int iz, int ir0, int ir1) // any of row iz's columns ir0..ir1
-{
-  return iz >= b.x && iz <= b.y && ir1 >= b.z && ir0 <= b.w;
-}
-constexpr int JBOX_NONE = 0x7fffffff;
-__device__ __forceinline__ void jbox_empty(int *jbox)
-{
-  *reinterpret_cast<int4 *>(jbox) = make_int4(JBOX_NONE, -1, JBOX_NONE, -1);
-}
-
 __device__ __forceinline__ void jbox_reset(int *jbox)
 {
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0)

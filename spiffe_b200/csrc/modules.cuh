@@ -121,7 +121,8 @@ struct BirthParams {
 };
 extern "C" int spiffe_births64(const DevMesh *m, const DevFields<double> *f, const DevBeam64 *b, const BirthParams *p,
                                DevCounts *cnt, cudaStream_t s);
-extern "C" int spiffe_antenna64(double *J, int pitch, int direction, long istart, long iend, long iposition,
+extern "C" int spiffe_zero_j64(const DevMesh *m, double *J, size_t stride, int comps, int *jbox, cudaStream_t s);
+extern "C" int spiffe_antenna64(double *J, int *jbox, int pitch, int direction, long istart, long iend, long iposition,
                                 double value, cudaStream_t s);
 
 // translate_problem (translate.c:51-57, :123-196): *flag = 1 when a particle

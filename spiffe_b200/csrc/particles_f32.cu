@@ -441,23 +441,6 @@ __device__ __forceinline__ void warp_add(long long *J, int nd, long long v)
   }
 }
 
-// Widens the box of nodes holding current (the FDTD reads and clears only
-// those) to the rows rlo..rhi and the columns up to col; a warp skips the
-// atomics when the box already covers it.  Its columns begin at the axis, near
-// which particles mostly are.
-__device__ __forceinline__ void widen_box(int *jbox, int rlo, int rhi, int col)
-{
-  const int4 b = *reinterpret_cast<const int4 *>(jbox);
-  if (rlo < b.x)
-    atomicMin(jbox, rlo);
-  if (rhi > b.y)
-    atomicMax(jbox + 1, rhi);
-  if (b.z > 0)
-    atomicMin(jbox + 2, 0);
-  if (col > b.w)
-    atomicMax(jbox + 3, col);
-}
-
 // Deposits the three components of one particle (or nothing, when !on);
 // called by every lane of the warp.
 template <bool DEF>

@@ -683,17 +683,9 @@ __global__ void __launch_bounds__(T) k_deposit(DevMesh m, DevFields<double> f, D
   step_begin();
   const long ip = (long)blockIdx.x * T + threadIdx.x;
   const long np = (long)cnt->np;
-  if (ip >= np) {
-    if (keys && ip < n_slots)
-      for (int k = 0; k < stride; k++) {
-        keys[stride * ip + k] = pad;
-        vals[stride * ip + k] = 0.0;
-      }
-    return;
-  }
   Contrib c;
   c.n = 0;
-  if (b.status[ip] & SPIFFE_PART_ACTIVE) {
+  if (ip < np && b.status[ip] & SPIFFE_PART_ACTIVE) {
     const double one_over = 1 / (SPIFFE_PI * m.dz * (m.dr * m.dr));
     if (component == 0)
       contrib_jz(m, b.z[ip], b.r[ip], b.vz[ip], b.Q[ip], one_over, c);
@@ -702,11 +694,25 @@ __global__ void __launch_bounds__(T) k_deposit(DevMesh m, DevFields<double> f, D
     else
       contrib_jphi(m, b.z[ip], b.r[ip], b.vphi[ip], b.Q[ip], one_over, c);
   }
+  unsigned lo = 0xffffffffu, hi = 0u; // nodes this lane adds to, and their last column
+  int col = 0;
+  for (int k = 0; k < c.n; k++) {
+    const unsigned nd = (unsigned)c.node[k];
+    lo = min(lo, nd);
+    hi = max(hi, nd);
+    col = max(col, (int)(nd % (unsigned)m.pitch));
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  col = __reduce_max_sync(0xffffffffu, col);
+  if ((threadIdx.x & 31) == 0 && lo <= hi)
+    widen_box(f.jbox, (int)(lo / (unsigned)m.pitch), (int)(hi / (unsigned)m.pitch), col);
   if (keys) {
-    for (int k = 0; k < stride; k++) {
-      keys[stride * ip + k] = k < c.n ? c.node[k] : pad;
-      vals[stride * ip + k] = k < c.n ? c.val[k] : 0.0;
-    }
+    if (ip < n_slots)
+      for (int k = 0; k < stride; k++) {
+        keys[stride * ip + k] = k < c.n ? c.node[k] : pad;
+        vals[stride * ip + k] = k < c.n ? c.val[k] : 0.0;
+      }
     return;
   }
   double *J = component == 0 ? f.Jz : (component == 1 ? f.Jr : f.Jphi);

@@ -952,7 +952,7 @@ extern "C" int spiffe_gpu_create(const spiffe_mesh *mesh, const int16_t *flags, 
   }
   DevFields<double> &f = in->f;
   {
-    // Jz, Jr (and Jphi) lie one behind the other, cleared by one fill a step
+    // Jz, Jr (and Jphi) lie one behind the other, cleared together
     const bool te = mesh->modes & SPIFFE_FL_TE_FIELDS;
     const size_t pad = in->j_stride = (n + 31) & ~(size_t)31;
     DeviceSlab d;
@@ -966,9 +966,12 @@ extern "C" int spiffe_gpu_create(const spiffe_mesh *mesh, const int16_t *flags, 
       for (double **p : {&f.Ephi, &f.Br, &f.Br2, &f.Bz, &f.Bz2})
         d.add(p, n);
     d.add(&in->d_flags, n);
+    d.add(&f.jbox, 8);
     if (d.make() != cudaSuccess || cudaMemsetAsync(in->slab, 0, d.bytes(), s) != cudaSuccess ||
         cudaMemcpyAsync(in->d_flags, flags, n * sizeof(int16_t), cudaMemcpyHostToDevice, s) != cudaSuccess)
       return bail(fail(SPIFFE_ERR_NOMEM, "field allocation failed"));
+    if ((rc = s32_jbox_set(f.jbox, 0x7fffffff, -1, s)))
+      return bail(fail(SPIFFE_ERR_CUDA, "instance setup failed: %s", cudaGetErrorString((cudaError_t)rc)));
     f.flags = in->d_flags;
   }
   if ((rc = alloc_beam(&in->b, in->capacity)))
@@ -1064,6 +1067,8 @@ extern "C" int spiffe_gpu_upload_fields(spiffe_gpu_instance *in, const spiffe_fi
   }
   FIELD_LIST(UP)
 #undef UP
+  if (h->Jz || h->Jr || h->Jphi) // uploaded current may be anywhere
+    RC_TRY(s32_jbox_set(in->f.jbox, 0, 0x7ffffffe, s));
   set_devmesh(in);
   CUDA_TRY(cudaStreamSynchronize(s));
   return 0;
@@ -1167,8 +1172,7 @@ extern "C" int spiffe_gpu_zero_current_arrays(spiffe_gpu_instance *in)
     return s32_zero_j(in);
   const int first = in->mesh.modes & SPIFFE_FL_TM_FIELDS ? 0 : 2, last = in->mesh.modes & SPIFFE_FL_TE_FIELDS ? 3 : 2;
   if (last > first)
-    CUDA_TRY(cudaMemsetAsync(in->f.Jz + first * in->j_stride, 0, (last - first) * in->j_stride * sizeof(double),
-                             in->stream));
+    RC_TRY(spiffe_zero_j64(&in->dm, in->f.Jz + first * in->j_stride, in->j_stride, last - first, in->f.jbox, in->stream));
   return 0;
 }
 
@@ -2484,6 +2488,8 @@ static int translate(spiffe_gpu_instance *in, int32_t *translated)
       return fail(SPIFFE_ERR_CUDA, "translation copy failed");
   if (S && s32_cells_down(S->b.cell, S->f.jbox, in->cnt, in->np_upper, s))
     return fail(SPIFFE_ERR_CUDA, "translation launch failed");
+  if (!S)
+    RC_TRY(s32_jbox_set(in->f.jbox, 0, 0x7ffffffe, s)); // moved current: cleared whole by the next step
   // a screen's cell moves with the particles' cells (the split push finds
   // crossings by cell)
   for (int k = 0; k < in->screens.n; k++)
@@ -3375,7 +3381,7 @@ static int antennas(spiffe_gpu_instance *in, double time)
       rc = s32_antenna(arr, F.jbox, in->dm.pitch, a.direction, a.istart, a.iend, a.iposition, J, in->s32->sc.qJ, in->stream);
     } else {
       double *arr = a.direction == 0 ? in->f.Jz : (a.direction == 1 ? in->f.Jr : in->f.Jphi);
-      rc = spiffe_antenna64(arr, in->dm.pitch, a.direction, a.istart, a.iend, a.iposition, J, in->stream);
+      rc = spiffe_antenna64(arr, in->f.jbox, in->dm.pitch, a.direction, a.istart, a.iend, a.iposition, J, in->stream);
     }
     if (rc)
       return fail(SPIFFE_ERR_CUDA, "antenna launch failed");

@@ -141,3 +141,38 @@ def test_swap_compaction_pairs_holes_with_the_last_survivors(n, n_lost):
         assert got.np == got.npActive == new_np
         assert np.array_equal(got["particleID"], expect)
     g.close()
+
+
+def test_current_is_cleared_and_read_where_it_lies(oracle):
+    """Currents left by an upload, by deposits on top of one another and by
+    earlier, wider deposits: the clearing, and the field update that reads J
+    only in its box, against the checker's whole arrays."""
+    f = pillbox(60, 50)
+    rng = np.random.default_rng(8)
+    for n in ("Ez", "Er", "Bphi", "Jz", "Jr"):
+        f[n] = rng.normal(size=f.shape) * (1e3 if n[0] == "J" else 1.0)
+    ref = f.copy()
+    g = gpu.GpuInstance(f, capacity=4096)
+    g.set_deposit_order(1)
+    wide, narrow = crowded_beam(f, [3] * 200), crowded_beam(f, [5])
+
+    def same(names=("Jz", "Jr", "Ez", "Er", "Bphi")):
+        out = g.fields(f)
+        for n in names:
+            assert np.array_equal(out[n], ref[n]), n
+
+    g.upload_fields(f)
+    g.advance_fields()  # with the uploaded current
+    oracle.advance_fields(ref)
+    same()
+    for beams in ([wide], [narrow], [wide, narrow], [], [narrow]):
+        g.zero_currents()
+        oracle.zero_currents(ref)
+        for b in beams:
+            g.upload_beam(b)
+            g.deposit()
+            oracle.deposit(ref, b)
+        g.advance_fields()
+        oracle.advance_fields(ref)
+        same()
+    g.close()
