@@ -97,3 +97,39 @@ def test_order_of_particles_changes_nothing(kind, nz, nr, modes):
             assert np.array_equal(v, beam[k]), k
         for k in ("Ez", "Er", "Bphi", "Jz", "Jr"):
             assert np.array_equal(out[0][1][k], fields[k]), k
+
+
+@pytest.mark.parametrize("n, n_lost", [(1, 1), (40, 39), (257, 200), (5000, 2047), (262145, 4000), (262145, 5000)])
+def test_the_lost_leave_in_index_order_and_the_counts_are_reset(n, n_lost):
+    """One block removes the lost, with few enough of them to be sorted and
+    with more: the k-th hole takes the k-th survivor above the new count, and
+    the counts are ready for the next push."""
+    cfg = workloads.PillboxConfig()
+    f = geometry.fields_for(cfg.nz, cfg.nr, cfg.zmin, cfg.zmax, cfg.rmax, cfg.geo_text(), modes=MODES)
+    f.mesh.dt = cfg.dt
+    rng = np.random.default_rng(n + n_lost)
+    lost = np.sort(rng.choice(n, n_lost, replace=False))
+    z = np.full(n, 0.5 * (cfg.zmin + cfg.zmax))
+    z[lost] = cfg.zmax - 0.1 * cfg.dz  # leaves the mesh in one step at pz = 10
+    pz = np.zeros(n)
+    pz[lost] = 10.0
+    b = abi.Beam(n + 16)
+    b.QoMC = QoMC
+    b.set(n, z=z, r=np.full(n, 0.2 * cfg.rmax), pz=pz, Q=np.full(n, -1e-16), particleID=np.arange(1, n + 1),
+          status=np.full(n, abi.PART_ACTIVE, np.uint64))
+    b.npActive = n
+    g = gpu.GpuInstance(f, capacity=b.capacity, precision=gpu.PRECISION_SPLIT32)
+    g.set_sort_interval(0)
+    g.upload_beam(b)
+    g.configure_run(space_charge=0, push=abi.push_options(abi.COMPACT_SWAP, abi.SCREEN_PARTICLE))
+    new_np = n - n_lost
+    gone = np.isin(np.arange(n), lost)
+    expect = np.arange(1, n + 1)[:new_np]
+    expect[lost[lost < new_np]] = np.nonzero(~gone[new_np:])[0] + new_np + 1
+    for _ in range(2):  # the second step loses nothing
+        g.run_steps(1)
+        got = g.download_beam(abi.Beam(b.capacity))
+        assert got.np == got.npActive == new_np
+        assert np.array_equal(got["particleID"], expect)
+    assert g.work_counters()["particle_steps"] == n + new_np
+    g.close()
