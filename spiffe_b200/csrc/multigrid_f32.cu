@@ -52,9 +52,12 @@
 // exactly by its precomputed inverse over the whole GPU.  Coefficients are kept
 // per distinct row (class): in a gun nearly all rows of a level are alike, so
 // a band's fit L1 and a thread keeps its columns' in registers.
+// Within a cycle a kernel comes onto the SMs while the one before ends
+// (programmatic edges, step_begin) and has its coefficients in registers by
+// the time that has ended (5 to 9 % of a cycle).
 // Measured from a cold start to 1e-6 (B200), first form -> here: 3001 x 821
-// gun 1.6 -> 0.78 ms in 5 cycles, 1500 x 400 1.13 -> 0.38 in 5, 424 x 232
-// 0.99 -> 0.48 in 9, 601 x 165 0.69 -> 0.29 in 5.
+// gun 1.6 -> 0.75 ms in 5 cycles, 1500 x 400 1.13 -> 0.35 in 5, 424 x 232
+// 0.99 -> 0.46 in 9, 601 x 165 0.69 -> 0.27 in 5.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -296,7 +299,8 @@ template <int K> struct Fix9 {
   float g0[2][K], g1[2][K]; // f/diagonal
   unsigned unk;             // bits 2 (K parity + k), +1: the pair's even and odd nodes are unknowns
 
-  __device__ __forceinline__ void init(const MgLevel &L, const float *F, int r0, int rlo, int rhi)
+  // init: what is constant (before the kernel's turn has come); start: f
+  __device__ __forceinline__ void init(const MgLevel &L, int r0, int rlo, int rhi)
   {
     const int n = (L.R + 1) >> 1;
     rlo = max(rlo, 0);
@@ -313,12 +317,21 @@ template <int K> struct Fix9 {
           j[z][k] = t - q * n;
           at[z][k] = (I - r0) * L.P;
           const float *p = load_coef9(L, __ldg(L.cls + I), j[z][k], c[z][k]);
-          const float i0 = __ldg(p + MG_INVD * L.P), i1 = __ldg(p + MG_INVD * L.P + L.Q);
-          g0[z][k] = i0 * F[at[z][k] + 1 + j[z][k]];
-          g1[z][k] = i1 * F[at[z][k] + L.Q + 1 + j[z][k]];
+          const float i0 = g0[z][k] = __ldg(p + MG_INVD * L.P), i1 = g1[z][k] = __ldg(p + MG_INVD * L.P + L.Q);
           unk |= (i0 != 0.f ? 1u : 0u) << (2 * (K * z + k)) | (i1 != 0.f ? 2u : 0u) << (2 * (K * z + k));
         }
       }
+  }
+  __device__ __forceinline__ void start(const MgLevel &L, const float *F)
+  {
+#pragma unroll
+    for (int z = 0; z < 2; z++)
+#pragma unroll
+      for (int k = 0; k < K; k++)
+        if (row[z][k] != INT_MIN) {
+          g0[z][k] *= F[at[z][k] + 1 + j[z][k]];
+          g1[z][k] *= F[at[z][k] + L.Q + 1 + j[z][k]];
+        }
   }
   template <int CZ, int CR>
   __device__ __forceinline__ void colour(const MgLevel &L, float *U, const float *, int, int ra, int rb)
@@ -381,7 +394,8 @@ struct Run9 {
     j = k < n ? k : -1;
     v = -1;
   }
-  __device__ __forceinline__ void init(const MgLevel &L, const float *, int, int rlo, int rhi)
+  __device__ __forceinline__ void start(const MgLevel &, const float *) {}
+  __device__ __forceinline__ void init(const MgLevel &L, int, int rlo, int rhi)
   {
     n = (L.R + 1) >> 1;
     W = (n + 31) & ~31;
@@ -679,6 +693,7 @@ __global__ void __launch_bounds__(MG_NT, 1) k_mg_down0(const __grid_constant__ M
                                                        MgCall *call, cudaGraphConditionalHandle more, float *scratch,
                                                        size_t scratch_n)
 {
+  step_begin();
   if (call->skip) {
     if (blockIdx.x == 0 && threadIdx.x == 0)
       cudaGraphSetConditional(more, 0);
@@ -774,12 +789,17 @@ __global__ void __launch_bounds__(MG_NT, 1) k_mg_down9(const __grid_constant__ M
   float *buf = band_buf<SM>(scratch, scratch_n);
   const int I0 = blockIdx.x * L.rp, I1 = min(I0 + L.rp, L.Z), r0 = I0 - MG_DOWN, n = I1 - I0 + 2 * MG_DOWN;
   float *U = buf + L.P, *F = U + (L.rp + 2 * MG_DOWN + 1) * L.P; // a zero row on either side of U
-  load9(L, L.f, F, r0, n);
+  Op t;
+  t.init(L, r0, r0, r0 + n);
+  if (!SM) // (the scratch is the kernel's before)
+    step_begin();
   for (int k = 4 * threadIdx.x; k < (n + 2) * L.P; k += 4 * MG_NT)
     st4(buf + k, make_float4(0.f, 0.f, 0.f, 0.f));
+  if (SM)
+    step_begin();
+  load9(L, L.f, F, r0, n);
   __syncthreads();
-  Op t;
-  t.init(L, F, r0, r0, r0 + n);
+  t.start(L, F);
 #pragma unroll 1
   for (int k = 0; k < 4; k += 2) {
     rows9<0, 0>(L, t, U, F, r0, r0 + k, r0 + n - k);
@@ -800,11 +820,13 @@ __global__ void __launch_bounds__(MG_NT, 1) k_mg_up9(const __grid_constant__ MgL
 {
   float *U = band_buf<SM>(scratch, scratch_n), *F = U + (L.rp + 2 * MG_DOWN) * L.P;
   const int I0 = blockIdx.x * L.rp, I1 = min(I0 + L.rp, L.Z), r0 = I0 - MG_UP, n = I1 - I0 + 2 * MG_UP;
+  Op t;
+  t.init(L, r0, r0, r0 + n);
+  step_begin();
   load9(L, L.f, F, r0, n);
   load9(L, L.u, U, r0, n);
   __syncthreads();
-  Op t;
-  t.init(L, F, r0, r0, r0 + n);
+  t.start(L, F);
   t.template prolong<true>(L, C, U, C.v, r0);
   __syncthreads();
 #pragma unroll 1
@@ -858,6 +880,7 @@ template <bool SM>
 __global__ void __launch_bounds__(MG_NT, 1) k_mg_up0(const __grid_constant__ Mg0 z, const __grid_constant__ MgLevel C,
                                                      const MgCall *call, float *scratch, size_t scratch_n)
 {
+  step_begin();
   const int P = z.P, H = P >> 1, K = (H / 4 + 31) >> 5, lane = threadIdx.x & 31;
   const float nan = __int_as_float(0x7fc00000);
   const int a0 = blockIdx.x * z.rp, b0 = min(a0 + z.rp, z.nz), r0 = a0 - MG_UP, n = b0 - a0 + 2 * MG_UP;
@@ -949,6 +972,7 @@ __global__ void __launch_bounds__(MG_NT) k_mg_dense(const float *__restrict__ in
   for (int k = 0; k < K; k++)
     m[k] = 128 * k < ld ? __ldg(src + 32 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
   const int at = __ldg(idx + min(row, n - 1));
+  step_begin();
   for (int i = tid; i < ld; i += MG_NT)
     x[i] = i < n ? __ldcg(f + __ldg(idx + i)) : 0.f;
   __syncthreads();
@@ -1014,6 +1038,7 @@ __global__ void __launch_bounds__(32) k_mg_inverse(int n, int b, const double *_
 // lie in shared memory, else in global memory.  The result goes to v.
 template <bool SM, class Op> __global__ void __launch_bounds__(MG_NT, 1) k_mg_coarse(const __grid_constant__ MgLevel L)
 {
+  step_begin();
   const int tid = threadIdx.x, n = (L.Z + 2) * L.P;
   float *u = SM ? reinterpret_cast<float *>(mg_smem) : L.u, *f = SM ? u + n : L.f; // row -1 first
   for (int k = 4 * tid; k < n; k += 4 * MG_NT) {
@@ -1023,7 +1048,8 @@ template <bool SM, class Op> __global__ void __launch_bounds__(MG_NT, 1) k_mg_co
   }
   __syncthreads();
   Op t;
-  t.init(L, f, -1, 0, L.Z);
+  t.init(L, -1, 0, L.Z);
+  t.start(L, f);
 #pragma unroll 1
   for (int k = 0; k < MG_COARSE_SWEEPS; k++) {
     rows9<0, 0>(L, t, u, f, -1, 0, L.Z);
@@ -1357,7 +1383,13 @@ int mg_graph(Mg32Work *w, Mg0 z, int last, bool sm, const MgDense *dense, bool c
     p.sharedMemBytes = (unsigned)smem;
     p.kernelParams = args;
     cudaGraphNode_t n;
-    e = cudaGraphAddKernelNode(&n, g, prev ? &prev : nullptr, prev ? 1 : 0, &p);
+    e = cudaGraphAddKernelNode(&n, g, nullptr, 0, &p);
+    if (e == cudaSuccess && prev) { // begins while the one before ends (step_begin)
+      cudaGraphEdgeData next{};
+      next.from_port = cudaGraphKernelNodePortProgrammatic;
+      next.type = cudaGraphDependencyTypeProgrammatic;
+      e = cudaGraphAddDependencies_v2(g, &prev, &n, &next, 1);
+    }
     prev = n;
   };
   size_t n0 = floats_of(z.rp, z.P);
