@@ -63,6 +63,7 @@ struct Poisson64Work {
   // does not fit): its grid, rows a band, half-row length, update rows, and
   // the driving term in the bands' order, exchange rows and barrier words
   const void *band_kernel = nullptr;
+  int band_cluster = 0; // its blocks are one cluster of this many
   int band_grid = 0, band_R = 0, band_H = 0, band_lo = 0, band_hi = 0;
   size_t band_smem = 0;
   double *band_mem = nullptr, *band_xb = nullptr;

@@ -4,15 +4,17 @@
 // (poisson.c:17-130) and compute_imposed_Efield (poisson_correction.c:
 // 456-562) as device kernels.  The decision whether to solve (the error-
 // charge threshold, :258-265) is taken on the device, so a correction needs
-// no host round trip.  The red-black SOR runs as one persistent cooperative
-// kernel: each half-sweep updates one colour (the reference's colour test,
-// poisson.c:70), every block reduces its |residual| sum, and after a grid
-// barrier all blocks add the per-block sums in the same fixed order and take
-// the same stop decision (poisson.c:120-121).  Node updates are bit-identical
-// to the reference (a colour's nodes read only the other colour); the stop
-// sum is reduced in a fixed tree order rather than the reference's serial
-// order, which changes the half-sweep count only if the sum lands within
-// rounding distance of the threshold.  Built with -fmad=false.
+// no host round trip.  The red-black SOR runs as one persistent kernel, with
+// the mesh in the SMs' shared memory where it fits (k_sor_band; small meshes
+// in one cluster's) and over global memory where not (k_sor): each half-sweep
+// updates one colour (the reference's colour test, poisson.c:70), every block
+// reduces its |residual| sum, and after a barrier all blocks add the per-block
+// sums in the same fixed order and take the same stop decision
+// (poisson.c:120-121).  Node updates are bit-identical to the reference (a
+// colour's nodes read only the other colour); the stop sum is reduced in a
+// fixed tree order rather than the reference's serial order, which changes the
+// half-sweep count only if the sum lands within rounding distance of the
+// threshold.  Built with -fmad=false.
 #include "divide.cuh"
 #include "modules.cuh"
 
@@ -421,7 +423,8 @@ __global__ void __launch_bounds__(RT) k_sor(DevMesh m, SorArgs s, DevCounts *cnt
 // 1024 threads spilled their prefetched driving terms (8.7 / 12.8), 512 had
 // too few warps (11.7 / 17.9), a barrier of one tagged word a band in place of
 // the counter cost 3 us more.
-constexpr int SB_NT = 768; // threads of a CTA
+constexpr int SB_NT = 768;     // threads of a CTA
+constexpr int SB_CLUSTER = 16; // blocks of the cluster form, at most
 
 struct SorBand {
   int R, H;           // rows of a band; half-row length (doubles)
@@ -431,16 +434,22 @@ struct SorBand {
   unsigned long long *bar; // [0] arrivals, [16] abort
 };
 
-// RK: rows of a band that a thread takes, at most
-template <int RK>
+// RK: rows of a band that a thread takes, at most.  CLUSTER: the grid is one
+// thread-block cluster, whose barrier takes the place of the counter in
+// global memory; the bands write their edge rows and sums straight into the
+// others' shared memory, so that nothing is fetched behind the barrier.  301 x
+// 83: 3.6 -> 2.1 us a half-sweep, of which the barriers are still more than half.
+template <int RK, bool CLUSTER>
 __global__ void __launch_bounds__(SB_NT, 1) k_sor_band(DevMesh m, SorArgs s, SorBand sb, DevCounts *cnt)
 {
   extern __shared__ double2 sb_smem[];
   __shared__ double sh[SB_NT / 32];
   __shared__ double total_sh;
+  __shared__ double part_sh[2][SB_CLUSTER]; // CLUSTER: every band's sum, by colour
   __shared__ int ok_sh;
   if (s.st && !s.st->do_solve)
     return;
+  namespace cg = cooperative_groups;
   double *S = reinterpret_cast<double *>(sb_smem);
   const int nz = m.nz, nr = m.nr, P = m.pitch, H = sb.H, G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
   const int lo = m.left_bc == SPIFFE_DIRICHLET ? 0 : 1, hi = m.right_bc == SPIFFE_DIRICHLET ? nz - 1 : nz - 2;
@@ -483,7 +492,10 @@ __global__ void __launch_bounds__(SB_NT, 1) k_sor_band(DevMesh m, SorArgs s, Sor
         rh[k] = __ldcg(reinterpret_cast<const double2 *>(rs + (size_t)r * 2 * H + ((colour + first + r) & 1) * H + j));
     }
   };
-  __syncthreads();
+  if (CLUSTER)
+    cg::this_cluster().sync(); // every band has its rows before a neighbour writes to them
+  else
+    __syncthreads();
   load_rh(0);
   long long result = -1;
   double total = 0;
@@ -535,11 +547,20 @@ __global__ void __launch_bounds__(SB_NT, 1) k_sor_band(DevMesh m, SorArgs s, Sor
             acc += fabs(ry);
           }
           *reinterpret_cast<double2 *>(x) = v;
-          double *xo = sb.xb + ((size_t)colour * G + b) * 2 * H + j;
-          if (r == 0)
-            __stcg(reinterpret_cast<double2 *>(xo), v);
-          if (r == nrow - 1)
-            __stcg(reinterpret_cast<double2 *>(xo + H), v);
+          if (CLUSTER) {
+            // into the neighbours' halo rows: they read this colour's half of
+            // them in the next half-sweep, behind the barrier
+            if (r == 0 && b > 0)
+              *reinterpret_cast<double2 *>(cg::this_cluster().map_shared_rank(S, b - 1) + (size_t)(sb.R + 1) * 2 * H + h * H + j) = v;
+            if (r == nrow - 1 && b < G - 1)
+              *reinterpret_cast<double2 *>(cg::this_cluster().map_shared_rank(S, b + 1) + h * H + j) = v;
+          } else {
+            double *xo = sb.xb + ((size_t)colour * G + b) * 2 * H + j;
+            if (r == 0)
+              __stcg(reinterpret_cast<double2 *>(xo), v);
+            if (r == nrow - 1)
+              __stcg(reinterpret_cast<double2 *>(xo + H), v);
+          }
         }
       }
     // the next half-sweep's driving terms arrive while the CTA waits
@@ -556,7 +577,11 @@ __global__ void __launch_bounds__(SB_NT, 1) k_sor_band(DevMesh m, SorArgs s, Sor
       double v = tid < SB_NT / 32 ? sh[tid] : 0.0;
       for (int o = 16; o > 0; o >>= 1)
         v += __shfl_down_sync(0xffffffffu, v, o);
-      if (tid == 0) {
+      if (CLUSTER) {
+        v = __shfl_sync(0xffffffffu, v, 0);
+        if (tid < G)
+          cg::this_cluster().map_shared_rank(&part_sh[0][0], tid)[colour * SB_CLUSTER + b] = v;
+      } else if (tid == 0) {
         __stcg(part + b, v);
         int ok = 1;
         asm volatile("fence.acq_rel.gpu;" ::: "memory");
@@ -581,30 +606,39 @@ __global__ void __launch_bounds__(SB_NT, 1) k_sor_band(DevMesh m, SorArgs s, Sor
         ok_sh = ok;
       }
     }
-    __syncthreads();
-    if (!ok_sh)
-      return;
-    if (tid >= SB_NT - 32) { // the last warp: every CTA forms the same sum of the partials
-      double v = 0;
-      for (int k = tid - (SB_NT - 32); k < G; k += 32)
-        v += __ldcg(part + k);
+    if (CLUSTER) {
+      cg::this_cluster().sync();
+      // every warp forms the same sum of the partials
+      double v = (tid & 31) < G ? part_sh[colour][tid & 31] : 0.0;
       for (int o = 16; o > 0; o >>= 1)
         v += __shfl_down_sync(0xffffffffu, v, o);
-      if (tid == SB_NT - 32)
-        total_sh = v;
-    } else { // the others: the neighbours' rows
-      const double *xi = sb.xb + (size_t)colour * G * 2 * H;
-      for (int k = 2 * tid; k < 2 * H; k += 2 * (SB_NT - 32)) {
-        const bool above = k >= H;
-        const int t = above ? k - H : k, nb = above ? b + 1 : b - 1, iz = above ? first + nrow : first - 1;
-        if (nb < 0 || nb >= G)
-          continue;
-        const double2 v = __ldcg(reinterpret_cast<const double2 *>(xi + (size_t)nb * 2 * H + (above ? 0 : H) + t));
-        *reinterpret_cast<double2 *>(S + (size_t)(above ? nrow + 1 : 0) * 2 * H + ((colour + iz) & 1) * H + t) = v;
+      total = __shfl_sync(0xffffffffu, v, 0);
+    } else {
+      __syncthreads();
+      if (!ok_sh)
+        return;
+      if (tid >= SB_NT - 32) { // the last warp: every CTA forms the same sum of the partials
+        double v = 0;
+        for (int k = tid - (SB_NT - 32); k < G; k += 32)
+          v += __ldcg(part + k);
+        for (int o = 16; o > 0; o >>= 1)
+          v += __shfl_down_sync(0xffffffffu, v, o);
+        if (tid == SB_NT - 32)
+          total_sh = v;
+      } else { // the others: the neighbours' rows
+        const double *xi = sb.xb + (size_t)colour * G * 2 * H;
+        for (int k = 2 * tid; k < 2 * H; k += 2 * (SB_NT - 32)) {
+          const bool above = k >= H;
+          const int t = above ? k - H : k, nb = above ? b + 1 : b - 1, iz = above ? first + nrow : first - 1;
+          if (nb < 0 || nb >= G)
+            continue;
+          const double2 v = __ldcg(reinterpret_cast<const double2 *>(xi + (size_t)nb * 2 * H + (above ? 0 : H) + t));
+          *reinterpret_cast<double2 *>(S + (size_t)(above ? nrow + 1 : 0) * 2 * H + ((colour + iz) & 1) * H + t) = v;
+        }
       }
+      __syncthreads();
+      total = total_sh;
     }
-    __syncthreads();
-    total = total_sh;
     if (n > 0 && (total < thr || total == 0)) {
       result = n;
       break;
@@ -635,11 +669,45 @@ int sb_rows(int cols, int R)
 
 const void *sb_kernel(int rows)
 {
-  return rows <= 2   ? (const void *)k_sor_band<2>
-         : rows <= 4 ? (const void *)k_sor_band<4>
-         : rows <= 7 ? (const void *)k_sor_band<7>
-         : rows <= 8 ? (const void *)k_sor_band<8>
+  return rows <= 2   ? (const void *)k_sor_band<2, false>
+         : rows <= 4 ? (const void *)k_sor_band<4, false>
+         : rows <= 7 ? (const void *)k_sor_band<7, false>
+         : rows <= 8 ? (const void *)k_sor_band<8, false>
                      : nullptr;
+}
+
+// The cluster form's bands: a power of two of blocks, each with rows, of at
+// most SB_CLUSTER_ROWS rows a thread; 0 where there is none.  With two rows a
+// thread the sixteen SMs are faster than all with a barrier through L2 (601 x
+// 83: 2.8 against 3.75 us a half-sweep, 201 x 300: 2.7 against 3.35), with
+// three and four no longer (801 x 100: 3.4 against 3.4, 601 x 165: 4.1 against 3.9).
+constexpr int SB_CLUSTER_ROWS = 2;
+int sb_cluster(int rows, int cols, int &R)
+{
+  for (int G = SB_CLUSTER; G > 1; G /= 2) {
+    R = (rows + G - 1) / G;
+    const int per_thread = sb_rows(cols, R);
+    if (per_thread > SB_CLUSTER_ROWS || !per_thread)
+      return 0; // fewer blocks would have more rows
+    if ((rows + R - 1) / R == G)
+      return G;
+  }
+  return 0;
+}
+
+cudaLaunchConfig_t sb_cluster_config(int G, size_t smem, cudaStream_t s, cudaLaunchAttribute *at)
+{
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = (unsigned)G;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(G);
+  c.blockDim = dim3(SB_NT);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return c;
 }
 
 // Ez, Er -= grad Psi (:288-326) with the FDTD boundary copies; one writer per node.
@@ -809,10 +877,28 @@ extern "C" int spiffe_poisson64_setup(const DevMesh *m, Poisson64Work *w, long l
     cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const int lo = m->left_bc == SPIFFE_DIRICHLET ? 0 : 1, hi = m->right_bc == SPIFFE_DIRICHLET ? nz - 1 : nz - 2;
     const int rows = hi - lo + 1, H = ((nr + 2) / 2 + 1) / 2 * 2;
-    const int G = std::max(1, std::min(sms, rows / 2)), R = (rows + G - 1) / G, per_thread = sb_rows(nr - 1, R);
+    int G = std::max(1, std::min(sms, rows / 2)), R = (rows + G - 1) / G, per_thread = sb_rows(nr - 1, R);
     const void *k = per_thread ? sb_kernel(per_thread) : nullptr;
-    const size_t smem = (size_t)(R + 4) * 2 * H * sizeof(double);
+    auto bytes = [&](int r) { return (size_t)(r + 4) * 2 * H * sizeof(double); };
     cudaFuncAttributes fa{};
+    int Rc = 0;
+    const int Gc = sb_cluster(rows, nr - 1, Rc);
+    if (Gc) {
+      const void *kc = (const void *)k_sor_band<SB_CLUSTER_ROWS, true>;
+      cudaLaunchAttribute at{};
+      const cudaLaunchConfig_t c = sb_cluster_config(Gc, bytes(Rc), s, &at);
+      int fits = 0;
+      if (cudaFuncGetAttributes(&fa, kc) == cudaSuccess && bytes(Rc) + fa.sharedSizeBytes <= (size_t)max_smem &&
+          cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes) == cudaSuccess &&
+          cudaFuncSetAttribute(kc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+          cudaOccupancyMaxActiveClusters(&fits, kc, &c) == cudaSuccess && fits > 0) {
+        k = kc;
+        R = Rc;
+        w->band_cluster = Gc;
+      }
+      cudaGetLastError();
+    }
+    const size_t smem = bytes(R);
     if (e == cudaSuccess && k && cudaFuncGetAttributes(&fa, k) == cudaSuccess && smem + fa.sharedSizeBytes <= (size_t)max_smem) {
       e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes);
       const int used = (rows + R - 1) / R;
@@ -925,7 +1011,13 @@ static int launch_sor(const DevMesh *m, Poisson64Work *w, double *Psi, const dou
     if (e != cudaSuccess)
       return (int)e;
     void *args[] = {&mm, &a, &sb, &cnt};
-    e = cudaLaunchCooperativeKernel(w->band_kernel, dim3(w->band_grid), dim3(SB_NT), args, w->band_smem, s);
+    if (w->band_cluster) {
+      cudaLaunchAttribute at{};
+      const cudaLaunchConfig_t c = sb_cluster_config(w->band_grid, w->band_smem, s, &at);
+      e = cudaLaunchKernelExC(&c, w->band_kernel, args);
+    } else {
+      e = cudaLaunchCooperativeKernel(w->band_kernel, dim3(w->band_grid), dim3(SB_NT), args, w->band_smem, s);
+    }
   } else {
     void *args[] = {&mm, &a, &cnt};
     e = cudaLaunchCooperativeKernel((void *)k_sor, dim3(w->sor_grid), dim3(RT), args, 0, s);

@@ -90,6 +90,14 @@ def test_sor_is_the_serial_iteration(oracle, nz, nr, ends):
     assert n == m and np.array_equal(g.fields(f)["Psi"], ref["Psi"])
 
 
+@pytest.mark.parametrize("nz, nr", [(12, 12), (20, 33), (106, 162), (301, 83), (700, 64), (769, 33),  # one cluster
+                                    (770, 100), (300, 411)])  # just too large for one
+def test_sor_of_one_cluster_and_of_the_grid(oracle, nz, nr):
+    """Meshes of two to sixteen bands in one thread-block cluster, with one
+    and with two rows a thread and a short last band, and their neighbours."""
+    test_sor_is_the_serial_iteration(oracle, nz, nr, (abi.NEUMANN, abi.DIRICHLET))
+
+
 def test_sor_follows_ends_set_after_setup(oracle):
     """set_mesh may change the end conditions, and with them the update rows."""
     f = pillbox(60, 40)
