@@ -934,7 +934,7 @@ __global__ void __launch_bounds__(CT) k_compact_any32(DevBeam32 b, const int32_t
     end_push(cnt, n_lost, np - n_lost, oa);
 }
 
-// ---- cell sort
+// ---- the order of the particles
 //
 // By half cell in r, then by z to an eighth of a cell: without smearing a
 // particle's current goes to the nearest half node in r (Jz) and in z (Jr),

@@ -197,7 +197,7 @@ struct S32State {
   // what J holds: unknown, zero, or exactly the deposit of the current
   // particles (left by the push of the previous step inside the loop)
   int j_state = S32_J_UNKNOWN;
-  // cell sort every 40 steps (on the gun, 20 / 40 / 80 / 160: 173.5 /
+  // the particles sorted every 40 steps (on the gun, 20 / 40 / 80 / 160: 173.5 /
   // 170.8 / 170.5 / 171.1 us a step; 10: 178.8)
   long long sort_interval = 40, since_sort = 0;
   double *staging = nullptr; // device FP64 staging for host transfers

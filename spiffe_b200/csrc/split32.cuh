@@ -128,7 +128,7 @@ struct Particles32Work {
   int32_t *keys = nullptr, *keys_alt = nullptr, *idx = nullptr, *idx_alt = nullptr;
   void *cub_tmp = nullptr;
   size_t cub_bytes = 0;
-  DevBeam32 alt{}; // second beam buffer for the cell sort
+  DevBeam32 alt{}; // second beam buffer for the sort
   long long capacity = 0;
   bool met_none = false; // the last push left the on-axis extremes at (+inf, -inf)
 };

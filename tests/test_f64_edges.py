@@ -184,3 +184,35 @@ def test_current_is_cleared_and_read_where_it_lies(oracle):
         oracle.advance_fields(ref)
         same()
     g.close()
+
+
+@pytest.mark.parametrize("nz, nr, spread", [(60, 50, 1.0), (300, 200, 0.1), (300, 200, 1.0)])
+@pytest.mark.parametrize("n", [131072, 131073, 140000])
+def test_unordered_sums_of_many_particles(nz, nr, spread, n):
+    """From 2^17 particles a block sums its particles in shared memory before
+    they go to J, where their nodes span few enough (all meshes and beams here
+    but the last), against the ordered sums.  Either order of n additions is
+    within n eps / 2 of the exact sum of the contributions' magnitudes, which
+    the same beam with positive velocities deposits."""
+    f = pillbox(nz, nr)
+    m = f.mesh
+    rng = np.random.default_rng(n + nr)
+    b = abi.Beam(n)
+    v = rng.normal(size=(2, n)) * 1e8
+    z = (0.45 + spread * rng.uniform(-0.45, 0.55, n)) * (m.zmax - m.zmin) + m.zmin
+    r = spread * rng.uniform(0, 1, n) ** 2 * m.dr * (nr - 1)
+    status = np.where(rng.uniform(size=n) < 0.9, abi.PART_ACTIVE, 0).astype(np.uint64)
+    got = {}
+    for name, order, vel in (("sum", 0, v), ("ordered", 1, v), ("size", 1, np.abs(v))):
+        b.set(n, z=z, r=r, vz=vel[0], vr=vel[1], Q=np.full(n, -1e-15), particleID=np.arange(1, n + 1), status=status)
+        b.npActive, b.nextParticleID, b.QoMC = int((status > 0).sum()), n + 1, QoMC
+        g = gpu.GpuInstance(f, capacity=n)
+        g.set_deposit_order(order)
+        g.upload_beam(b)
+        g.zero_currents()
+        g.deposit()
+        got[name] = g.fields(f)
+        g.close()
+    for k in ("Jz", "Jr"):
+        assert np.any(got["ordered"][k] != 0)
+        assert np.all(np.abs(got["sum"][k] - got["ordered"][k]) <= n * 2.3e-16 * np.abs(got["size"][k])), k
