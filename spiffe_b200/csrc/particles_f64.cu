@@ -725,10 +725,13 @@ __global__ void __launch_bounds__(T) k_deposit(DevMesh m, DevFields<double> f, D
 // from every particle and, a bunch covering some hundred nodes, fall on a few
 // slices of L2 (63 % of one slice's rate, 4 % of the average: 57 to 63 us a
 // component and million particles).  A block whose nodes span more than DTILE
-// adds directly; its nodes are then many.  A million particles, Jz and Jr: 114
-// -> 63 us.
+// adds directly; its nodes are then many.  A million particles, Jz and Jr: 115
+// -> 47 us.
 constexpr int DT = 512, DP = 8, DTILE = 4096;
-constexpr long long DEPOSIT_TILE_MIN = 1 << 17; // (32 blocks) below, too few blocks for the SMs
+// Below this many particles too few blocks for the SMs: a bunch on 3001 x 821
+// 131072 24.7 us against 22.3 straight to J, 524288 24.3 against 74.5; on 601 x
+// 165, whose nodes are fewer, 32768 37 against 26, 131072 38 against 87.
+constexpr long long DEPOSIT_TILE_MIN = 3 << 16;
 __global__ void __launch_bounds__(DT) k_deposit_tile(DevMesh m, DevFields<double> f, DevBeam64 b, const DevCounts *cnt,
                                                       int first, int last)
 {

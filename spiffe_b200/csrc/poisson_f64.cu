@@ -173,8 +173,10 @@ __global__ void __launch_bounds__(RT) k_remove_charge(DevMesh m, DevFields<doubl
       }
     }
   } else {
+    // (without smearing three of the four shares are 0 and change nothing;
+    // adding them took 164 of the kernel's 223 us a million particles)
     for (int k = 0; k < 4; k++)
-      if (at[k] != 0x7fffffff)
+      if (share[k] != 0)
         atomicAdd(f.Q + at[k], -share[k]);
   }
   const double s = block_sum(qreal, sh);

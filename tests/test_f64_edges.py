@@ -187,9 +187,9 @@ def test_current_is_cleared_and_read_where_it_lies(oracle):
 
 
 @pytest.mark.parametrize("nz, nr, spread", [(60, 50, 1.0), (300, 200, 0.1), (300, 200, 1.0)])
-@pytest.mark.parametrize("n", [131072, 131073, 140000])
+@pytest.mark.parametrize("n", [196608, 196609, 200000])
 def test_unordered_sums_of_many_particles(nz, nr, spread, n):
-    """From 2^17 particles a block sums its particles in shared memory before
+    """From 3 2^16 particles a block sums its particles in shared memory before
     they go to J, where their nodes span few enough (all meshes and beams here
     but the last), against the ordered sums.  Either order of n additions is
     within n eps / 2 of the exact sum of the contributions' magnitudes, which
