@@ -671,14 +671,14 @@ __device__ void contrib_jphi(const DevMesh &m, double z, double r, double v, dou
 }
 
 // component: 0 Jz, 1 Jr, 2 Jphi.  keys/vals != nullptr selects the ordered
-// mode: slot stride*ip+k receives contribution k (key = node, or `pad`) for
+// mode: slot stride*ip+k receives contribution k (key = key0 + node, or `pad`) for
 // every ip below the host's bound n_slots, so slots past the live np (after
 // losses) hold padding rather than an earlier step's contributions.  stride
 // is the most contributions the mesh's smearing gives (1, 2 or 4): the sort
 // that follows costs by the slot.
 __global__ void __launch_bounds__(T) k_deposit(DevMesh m, DevFields<double> f, DevBeam64 b, const DevCounts *cnt,
                                                 int component, int *keys, double *vals, long long n_slots, int stride,
-                                                int pad)
+                                                int key0, int pad)
 {
   step_begin();
   const long ip = (long)blockIdx.x * T + threadIdx.x;
@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(T) k_deposit(DevMesh m, DevFields<double> f, D
   if (keys) {
     if (ip < n_slots)
       for (int k = 0; k < stride; k++) {
-        keys[stride * ip + k] = k < c.n ? c.node[k] : pad;
+        keys[stride * ip + k] = k < c.n ? key0 + c.node[k] : pad;
         vals[stride * ip + k] = k < c.n ? c.val[k] : 0.0;
       }
     return;
@@ -995,28 +995,37 @@ extern "C" int spiffe_deposit64(const DevMesh *m, const DevFields<double> *f, co
     return 0;
   const unsigned nb = blocks_for(np_bound, T);
   const int nodes = (m->nz + 1) * m->pitch, stride = spiffe_smear_nodes(m);
+  const int first = m->modes & SPIFFE_FL_TM_FIELDS ? 0 : 2, last = m->modes & SPIFFE_FL_TE_FIELDS ? 3 : 2;
   if (!ordered && stride == 1 && np_bound >= DEPOSIT_TILE_MIN) {
-    const int first = m->modes & SPIFFE_FL_TM_FIELDS ? 0 : 2, last = m->modes & SPIFFE_FL_TE_FIELDS ? 3 : 2;
     if (last > first) {
       launch_next(k_deposit_tile, blocks_for(np_bound, DT * DP), DT, s, *m, *f, *b, cnt, first, last);
       spiffe_note_launches(1);
     }
     return (int)cudaGetLastError();
   }
-  for (int comp = 0; comp < 3; comp++) {
-    if (comp < 2 && !(m->modes & SPIFFE_FL_TM_FIELDS))
-      continue;
-    if (comp == 2 && !(m->modes & SPIFFE_FL_TE_FIELDS))
-      continue;
-    if (!ordered) {
-      launch_next(k_deposit, nb, T, s, *m, *f, *b, cnt, comp, nullptr, nullptr, 0, stride, nodes);
+  double *const J[3] = {f->Jz, f->Jr, f->Jphi};
+  if (!ordered) {
+    for (int comp = first; comp < last; comp++) {
+      launch_next(k_deposit, nb, T, s, *m, *f, *b, cnt, comp, nullptr, nullptr, 0, stride, 0, nodes);
       spiffe_note_launches(1);
-      continue;
     }
-    launch_next(k_deposit, nb, T, s, *m, *f, *b, cnt, comp, w->keys, w->vals, np_bound, stride, nodes);
-    spiffe_note_launches(1);
-    double *J = comp == 0 ? f->Jz : (comp == 1 ? f->Jr : f->Jphi);
-    if (int rc = spiffe_ordered_add64(w, stride * np_bound, nodes, J, s))
+    return (int)cudaGetLastError();
+  }
+  // The components' entries sorted and summed together where the buffers hold
+  // them: J's components lie one behind the other, so a component is a range
+  // of keys.  A call is latency (two passes of the sort, the longest run's
+  // additions), which two components then share: 20,000 particles on 301 x
+  // 83, 75 -> 38 us a component.
+  const long long per = (long long)stride * np_bound, step = last - first > 1 ? J[first + 1] - J[first] : nodes;
+  const int together = (last - first) * stride <= 4 && step >= nodes && (last - first) * step < 0x7fffffff ? last - first : 1;
+  for (int comp = first; comp < last; comp += together) {
+    const int pad = together > 1 ? (int)(together * step) : nodes;
+    for (int k = 0; k < together; k++) {
+      launch_next(k_deposit, nb, T, s, *m, *f, *b, cnt, comp + k, w->keys + k * per, w->vals + k * per, np_bound, stride,
+                  (int)(k * step), pad);
+      spiffe_note_launches(1);
+    }
+    if (int rc = spiffe_ordered_add64(w, together * per, pad, J[comp], s))
       return rc;
   }
   return (int)cudaGetLastError();

@@ -67,6 +67,27 @@ def test_ordered_sums_in_particle_order(oracle, counts, smear):
         assert np.array_equal(out[n], ref[n]), n
 
 
+@pytest.mark.parametrize("smear", [0, abi.FL_RADIAL_SMEAR, abi.FL_RADIAL_SMEAR | abi.FL_LONGIT_SMEAR])
+@pytest.mark.parametrize("modes", [MODES | abi.FL_TE_FIELDS, (MODES | abi.FL_TE_FIELDS) & ~abi.FL_TM_FIELDS])
+def test_ordered_sums_of_every_component(oracle, modes, smear):
+    """Components sorted together, or one by one where the buffers do not hold all."""
+    f = pillbox(60, 50, modes | smear)
+    b = crowded_beam(f, [700, 33, 64] + [3] * 150)
+    g = gpu.GpuInstance(f, capacity=b.capacity)
+    g.set_deposit_order(1)
+    g.upload_beam(b)
+    ref = f.copy()
+    for _ in range(2):
+        g.zero_currents()
+        oracle.zero_currents(ref)
+        g.deposit()
+        oracle.deposit(ref, b)
+        out = g.fields(f)
+        for n in ("Jz", "Jr", "Jphi"):
+            if n in f.a and (n == "Jphi" or modes & abi.FL_TM_FIELDS):
+                assert np.array_equal(out[n], ref[n]), n
+
+
 @pytest.mark.parametrize("ends", [(abi.NEUMANN, abi.NEUMANN), (abi.DIRICHLET, abi.DIRICHLET),
                                   (abi.NEUMANN, abi.DIRICHLET)])
 @pytest.mark.parametrize("nz, nr", [(6, 5), (7, 6), (40, 9), (41, 66), (300, 67), (307, 34), (90, 259), (700, 130),
