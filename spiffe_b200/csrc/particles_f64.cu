@@ -725,14 +725,45 @@ __global__ void __launch_bounds__(T) k_deposit(DevMesh m, DevFields<double> f, D
 // from every particle and, a bunch covering some hundred nodes, fall on a few
 // slices of L2 (63 % of one slice's rate, 4 % of the average: 57 to 63 us a
 // component and million particles).  A block whose nodes span more than DTILE
-// adds directly; its nodes are then many.  A million particles, Jz and Jr: 115
-// -> 47 us.
-constexpr int DT = 512, DP = 8, DTILE = 4096;
-// Below this many particles too few blocks for the SMs: a bunch on 3001 x 821
-// 131072 24.7 us against 22.3 straight to J, 524288 24.3 against 74.5; on 601 x
-// 165, whose nodes are fewer, 32768 37 against 26, 131072 38 against 87.
+// adds directly; its nodes are then many.  A million particles of a
+// bunch, Jz and Jr: 135 -> 42 us in random order, 210 -> 37 in the order of
+// their cells, 37 -> 32 spread over the mesh.  Two blocks of 512 threads an SM:
+// eight particles a thread left one (57 us).
+constexpr int DT = 512, DP = 4, DTILE = DT * DP;
+
+// tile[at] += v for the lanes with at >= 0.  An addition in shared memory is a
+// loop of compare and swap that lanes of one address take in turn, so those of
+// an address that SAME or more lanes share (particles in the order of their
+// cells) are summed by shuffles first.
+constexpr int SAME = 4;
+__device__ __forceinline__ void tile_add(double *tile, int at, double v)
+{
+  const unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned grp = __match_any_sync(all, at);
+  bool single = at >= 0;
+  for (unsigned many = __ballot_sync(all, at >= 0 && __popc(grp) >= SAME); many;) {
+    const int first = __ffs(many) - 1;
+    const unsigned g = __shfl_sync(all, grp, first);
+    const bool in = g >> lane & 1;
+    double x = in ? v : 0.0;
+    for (int o = 16; o > 0; o >>= 1)
+      x += __shfl_xor_sync(all, x, o);
+    if (lane == first)
+      atomicAdd(tile + at, x);
+    if (in)
+      single = false;
+    many &= ~g;
+  }
+  if (single)
+    atomicAdd(tile + at, v);
+}
+
+// Below this many particles too few blocks for the SMs.  200,000 on 3001 x 821:
+// a bunch 17 to 19 us against 33 to 41 straight to J, spread over the mesh 12
+// against 12 (23 in the order of their radii).
 constexpr long long DEPOSIT_TILE_MIN = 3 << 16;
-__global__ void __launch_bounds__(DT) k_deposit_tile(DevMesh m, DevFields<double> f, DevBeam64 b, const DevCounts *cnt,
+__global__ void __launch_bounds__(DT, 2) k_deposit_tile(DevMesh m, DevFields<double> f, DevBeam64 b, const DevCounts *cnt,
                                                       int first, int last)
 {
   step_begin();
@@ -798,11 +829,10 @@ __global__ void __launch_bounds__(DT) k_deposit_tile(DevMesh m, DevFields<double
           tile[t] = 0;
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < DP; k++)
-          if (nd[k] >= 0) {
-            const int row = (int)((unsigned)nd[k] / (unsigned)P);
-            atomicAdd(tile + (row - r0) * W + nd[k] - row * P - c0, v[k]);
-          }
+        for (int k = 0; k < DP; k++) {
+          const int row = (int)((unsigned)max(nd[k], 0) / (unsigned)P);
+          tile_add(tile, nd[k] >= 0 ? (row - r0) * W + nd[k] - row * P - c0 : -1, v[k]);
+        }
         __syncthreads();
         for (int t = tid; t < (int)n; t += DT)
           if (tile[t] != 0) {
