@@ -80,6 +80,8 @@ cudaError_t spiffe_dev_malloc(void **p, size_t bytes)
     trim(m, dev);
     e = cudaMalloc(p, bytes);
   }
+  if (e != cudaSuccess)
+    cudaGetLastError(); // it is returned here, and is not the next call's
   if (e == cudaSuccess && bytes <= KEEP_BLOCK) {
     std::lock_guard<std::mutex> g(m.lock);
     m.used[*p] = Block{dev, bytes};

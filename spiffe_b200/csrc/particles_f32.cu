@@ -1343,7 +1343,8 @@ extern "C" int s32_particles_work(Particles32Work *w, long long capacity)
   m.add((char **)&w->cub_tmp, w->cub_bytes);
   cudaError_t e = m.make();
   if (e == cudaSuccess) e = (cudaError_t)s32_beam_alloc(&w->alt, capacity);
-  w->capacity = capacity;
+  if (e == cudaSuccess)
+    w->capacity = capacity;
   return (int)e;
 }
 
@@ -1368,6 +1369,8 @@ extern "C" int s32_push(const DevMesh *m, const DevFields32 *f, const DevBeam32 
                         const DevScreens *scr, DevCounts *cnt, long long np_bound, int compaction,
                         const S32Scales *sc, Particles32Work *w, cudaStream_t s)
 {
+  if (np_bound > w->capacity)
+    return (int)cudaErrorInvalidValue;
   if (m->n_onaxis) {
     k_reset_onaxis32<<<1, 1, 0, s>>>(cnt);
     spiffe_note_launches(1);
@@ -1422,6 +1425,8 @@ extern "C" int s32_sort(const DevMesh *m, DevBeam32 *b, DevCounts *cnt, long lon
 {
   if (np_bound <= 1)
     return 0;
+  if (np_bound > w->capacity)
+    return (int)cudaErrorInvalidValue;
   const int n = (int)np_bound;
   int sub, rb = 1;
   const int zb = sort_zbits(m->nz, m->nr, sub);

@@ -996,7 +996,8 @@ extern "C" int spiffe_particles64_work(Particles64Work *w, long long capacity, b
     m.add(&w->donors, n);
     m.add((char **)&w->cub_tmp, w->cub_bytes);
     e = m.make();
-    w->capacity = capacity;
+    if (e == cudaSuccess)
+      w->capacity = capacity;
   }
   if (e == cudaSuccess && ordered && !w->keys) {
     const size_t n = 4 * (size_t)w->capacity;
@@ -1048,6 +1049,9 @@ extern "C" int spiffe_deposit64(const DevMesh *m, const DevFields<double> *f, co
   // 83, 75 -> 38 us a component.
   const long long per = (long long)stride * np_bound, step = last - first > 1 ? J[first + 1] - J[first] : nodes;
   const int together = (last - first) * stride <= 4 && step >= nodes && (last - first) * step < 0x7fffffff ? last - first : 1;
+  // (components after the first go to places reckoned from the buffers' start)
+  if (!w->keys || together * per > 4 * w->capacity)
+    return (int)cudaErrorInvalidValue;
   for (int comp = first; comp < last; comp += together) {
     const int pad = together > 1 ? (int)(together * step) : nodes;
     for (int k = 0; k < together; k++) {
@@ -1112,6 +1116,8 @@ extern "C" int spiffe_gather_points64(const DevMesh *m, const DevFields<double> 
 extern "C" int spiffe_push64(const DevMesh *m, const DevFields<double> *f, const DevBeam64 *b, const PushHostParams *hp,
                              const DevScreens *scr, DevCounts *cnt, long long np_bound, Particles64Work *w, cudaStream_t s)
 {
+  if (np_bound > w->capacity)
+    return (int)cudaErrorInvalidValue;
   if (m->n_onaxis) {
     k_reset_onaxis<<<1, 1, 0, s>>>(cnt);
     spiffe_note_launches(1);

@@ -838,7 +838,7 @@ extern "C" int spiffe_poisson64_setup(const DevMesh *m, Poisson64Work *w, long l
   if (e == cudaSuccess && w->part_n < parts) {
     dev_free(w->part);
     e = dev_malloc(&w->part, sizeof(double) * parts);
-    w->part_n = parts;
+    w->part_n = e == cudaSuccess ? parts : 0;
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->Az, Az, sizeof(double) * (nr + 1), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->Ari, Ari, sizeof(double) * (nr + 1), cudaMemcpyHostToDevice, s);
@@ -974,6 +974,8 @@ static int sum_region(const double *a, int rows, int cols, int P, int absval, Po
 static int launch_sor(const DevMesh *m, Poisson64Work *w, double *Psi, const double *rhs, const int16_t *flags,
                       double accuracy, long long limit, PcState *st, long long *iters, DevCounts *cnt, cudaStream_t s)
 {
+  if (!w->part_n)
+    return (int)cudaErrorInvalidValue;
   int rc = ensure_omega(m, w, limit, s);
   if (rc)
     return rc;
@@ -1049,7 +1051,7 @@ extern "C" int spiffe_poisson_correction64(const DevMesh *m, const DevFields<dou
                                            DevCounts *cnt, long long np_bound, const PoissonHostOptions *o,
                                            Poisson64Work *w, Particles64Work *pw, bool ordered, cudaStream_t s)
 {
-  if (ordered && (!pw || !pw->keys || pw->capacity < np_bound))
+  if (!w->part_n || (ordered && (!pw || !pw->keys || pw->capacity < np_bound)))
     return (int)cudaErrorInvalidValue;
   // the particles' own charge leaves Q (:190-242)
   const int stride = spiffe_smear_nodes(m), nodes = (m->nz + 1) * m->pitch;

@@ -393,10 +393,10 @@ static int grow_beam(spiffe_gpu_instance *in, long long need)
   CUDA_TRY(cudaStreamSynchronize(s));
   free_beam(&in->b);
   in->b = nb;
-  in->capacity = cap;
   RC_TRY(spiffe_particles64_work(&in->pw, cap, in->deposit_ordered));
   if (in->pc_ready)
     RC_TRY(spiffe_poisson64_setup(&in->dm, &in->pcw, cap, s));
+  in->capacity = cap; // last: what could not be allocated is asked for again by the next growth
   return 0;
 }
 
@@ -620,8 +620,8 @@ static int s32_grow(spiffe_gpu_instance *in, long long need)
   CUDA_TRY(cudaStreamSynchronize(in->stream));
   s32_beam_free(&S.b);
   S.b = nb;
-  in->capacity = cap;
   RC_TRY(s32_particles_work(&S.pw, cap));
+  in->capacity = cap;
   return 0;
 }
 
@@ -1159,8 +1159,8 @@ extern "C" int spiffe_gpu_set_deposit_order(spiffe_gpu_instance *in, int32_t ord
     return fail(SPIFFE_ERR_INVALID, "null argument");
   if (in->s32)
     return 0; // fixed-point deposition is order-independent already
+  RC_TRY(spiffe_particles64_work(&in->pw, in->capacity, ordered != 0));
   in->deposit_ordered = ordered ? 1 : 0;
-  RC_TRY(spiffe_particles64_work(&in->pw, in->capacity, in->deposit_ordered));
   return 0;
 }
 
