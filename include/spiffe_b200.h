@@ -285,6 +285,12 @@ int spiffe_gpu_set_fdtd_kernel(spiffe_gpu_instance *inst, int32_t kernel);
  * used by other threads during the call. */
 int spiffe_gpu_batch_run(spiffe_gpu_instance *const *inst, int32_t n, const int64_t *steps, int32_t workers,
                          int64_t chunk, double *done_ms);
+/* Device memory of closed instances that the library keeps for new ones on the
+ * calling thread's device: at most 256 MB, given back to the driver when an
+ * allocation of the library fails, and by this call with release != 0, for
+ * other allocators in the process.  *bytes (may be null) receives what was
+ * kept before. */
+int spiffe_gpu_idle_memory(int32_t release, int64_t *bytes);
 /* Work done so far: out[0] particle-steps (active particles summed over
  * pushes), out[1] SOR half-sweeps, out[2] Poisson solves (either solver),
  * out[3] FDTD steps, out[4] multigrid V-cycles; out holds 5 values. */

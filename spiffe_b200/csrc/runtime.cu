@@ -1008,8 +1008,8 @@ extern "C" int spiffe_gpu_destroy(spiffe_gpu_instance *in)
   spiffe_particles64_work_free(&in->pw);
   spiffe_poisson64_free(&in->pcw);
   in->timer.release();
-  spiffe_pinned_free(in->h_cnt, sizeof(DevCounts) + 8 * sizeof(double));
-  spiffe_pinned_free(in->h_bins, in->bins_n * sizeof(BirthBin));
+  spiffe_pinned_free(in->h_cnt);
+  spiffe_pinned_free(in->h_bins);
   if (in->stream)
     cudaStreamDestroy(in->stream);
   delete in;
@@ -2135,7 +2135,7 @@ static int ensure_bins(spiffe_gpu_instance *in, size_t n)
     return 0;
   dev_free(in->d_bins);
   in->d_bins = nullptr;
-  spiffe_pinned_free(in->h_bins, in->bins_n * sizeof(BirthBin)); // (the copies from it ended with d_bins' release)
+  spiffe_pinned_free(in->h_bins); // (the copies from it ended with d_bins' release)
   in->h_bins = nullptr;
   in->bins_n = 0;
   CUDA_TRY(dev_malloc(&in->d_bins, n * sizeof(BirthBin)));

@@ -11,7 +11,7 @@
 cudaError_t spiffe_dev_malloc(void **p, size_t bytes);
 cudaError_t spiffe_dev_free(void *p);
 cudaError_t spiffe_pinned_malloc(void **p, size_t bytes);
-cudaError_t spiffe_pinned_free(void *p, size_t bytes);
+cudaError_t spiffe_pinned_free(void *p);
 
 // in place of cudaMalloc and cudaFree, with their meaning
 template <typename T> inline cudaError_t dev_malloc(T **p, size_t bytes) { return spiffe_dev_malloc((void **)p, bytes); }

@@ -82,6 +82,7 @@ def load():
         "spiffe_gpu_set_profiling": ([H, C.c_int32], C.c_int),
         "spiffe_gpu_phase_times": ([H, P(C.c_double), P(C.c_int64)], C.c_int),
         "spiffe_gpu_launch_count": ([], C.c_int64),
+        "spiffe_gpu_idle_memory": ([C.c_int32, P(C.c_int64)], C.c_int),
         "spiffe_gpu_work_counters": ([H, P(C.c_int64)], C.c_int),
         "spiffe_gpu_set_sort_interval": ([H, C.c_int64], C.c_int),
         "spiffe_gpu_set_poisson_solver": ([H, C.c_int32], C.c_int),
@@ -120,6 +121,14 @@ def select_device(device):
 
 def launch_count():
     return load().spiffe_gpu_launch_count()
+
+
+def idle_memory(release=False):
+    """Device bytes of closed instances kept for new ones on this thread's
+    device; with release they are given back to the driver."""
+    n = C.c_int64()
+    _check(load().spiffe_gpu_idle_memory(int(release), C.byref(n)))
+    return n.value
 
 
 def batch_run(instances, steps, workers=8, chunk=20):

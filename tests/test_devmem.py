@@ -72,3 +72,53 @@ def test_what_is_kept_is_bounded():
     free1, _ = torch.cuda.mem_get_info()
     # 256 MB, and what the driver keeps of its own (2 MB pages of small blocks)
     assert free0 - free1 <= (256 << 20) + (64 << 20)
+
+
+def test_what_is_kept_is_given_back_on_request():
+    import torch
+
+    instance(200, 300, gpu.PRECISION_F64, 1)[0].close()
+    torch.cuda.synchronize()
+    kept = gpu.idle_memory()
+    assert 0 < kept <= 256 << 20
+    free0, _ = torch.cuda.mem_get_info()
+    assert gpu.idle_memory(release=True) == kept
+    free1, _ = torch.cuda.mem_get_info()
+    assert free1 - free0 >= 0.9 * kept - (2 << 20)  # the driver's pages of small blocks may be shared
+    assert gpu.idle_memory() == 0
+    a = result(60, 50, gpu.PRECISION_SPLIT32, 2)
+    assert all(np.array_equal(x, y) for x, y in zip(a, result(60, 50, gpu.PRECISION_SPLIT32, 2)))
+
+
+RESET = """
+import ctypes, glob, sys
+sys.path[:0] = [{root!r}, {root!r} + "/tests"]
+import numpy as np
+from spiffe_b200 import gpu
+from test_devmem import result
+jobs = [(60, 50, p, 3) for p in (gpu.PRECISION_F64, gpu.PRECISION_SPLIT32)]
+before = [result(*j) for j in jobs]
+assert gpu.idle_memory() > 0
+rt = ctypes.CDLL(glob.glob("/usr/local/cuda/lib64/libcudart.so*")[0])
+assert rt.cudaDeviceReset() == 0
+assert gpu.idle_memory() == 0
+after = [result(*j) for j in jobs + jobs]
+for a, b in zip(before + before, after):
+    assert all(np.array_equal(x, y) for x, y in zip(a, b))
+print("same")
+"""
+
+
+def test_a_program_may_reset_its_device_between_instances():
+    """The reset ends the context and the memory kept in it: new instances must
+    not be given its addresses."""
+    import glob
+    import os
+    import subprocess
+    import sys
+
+    if not glob.glob("/usr/local/cuda/lib64/libcudart.so*"):
+        pytest.skip("no CUDA runtime library to reset the device with")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, "-c", RESET.format(root=root)], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0 and out.stdout.strip() == "same", out.stdout + out.stderr
