@@ -20,7 +20,9 @@ stream and device state and the kernels of different instances overlap.
   of the running requests' device footprints stays within a budget: first
   come first served, with backfill (a later request that fits may start
   while the head of the queue waits for memory, unless the head has already
-  been passed over ``max_bypass`` times); it reports each request's latency
+  been passed over ``max_bypass`` times); memory that the library keeps from
+  closed instances counts too, and is given back where a request would not
+  fit beside it; it reports each request's latency
   (arrival to result) and their percentiles.
 
 Each instance's arithmetic does not depend on what else runs: a result is
@@ -39,17 +41,20 @@ import numpy as np
 from . import abi, workloads
 
 # device bytes of an instance: a fixed part (allocation granularity, solver
-# scratch, the 16 MB at most of the multigrid's coarsest inverse), per mesh
+# scratch; split form: the 16 MB at most of the multigrid's coarsest inverse,
+# and the factors that it is made from at set-up), per mesh
 # node (split form: FP32 E/B and imposed fields, int64 current and particle
 # charge, FP64 Psi/PsiImposed/Q, flags, update mask, FP64 staging, and the
 # multigrid levels: FP32 correction and residual on the mesh, three arrays a
 # quarter the size on the next level, a sixteenth on the one after, padded
 # rows, coefficients of the distinct rows) and per particle slot (the split
 # particle layout, a second copy for the sort, sort keys, transfer staging).
-# An upper estimate.
-FIXED_BYTES = 33 << 20
+# An upper estimate, of the set-up too: on a B200 the driver's memory of guns
+# and pillboxes of 1,271 to 601,901 nodes and 4,416 to 610,452 slots, with a
+# screen as large as the beam, lay 6-90 % below it (tests/test_serve.py).
+FIXED_BYTES = {"split32": 20 << 20, "f64": 16 << 20}
 NODE_BYTES = {"split32": 200, "f64": 260}
-PARTICLE_BYTES = {"split32": 360, "f64": 460}
+PARTICLE_BYTES = {"split32": 300, "f64": 460}
 RECORD_BYTES = 112  # one screen record slot
 
 
@@ -98,7 +103,7 @@ def draw_requests(n, steps=5000, seed=1234, size_scale=1.0, particle_scale=1.0):
 
 def footprint_bytes(req, precision="split32"):
     """Device bytes an instance of this request occupies (an upper estimate)."""
-    return FIXED_BYTES + req.nodes * NODE_BYTES[precision] + req.capacity * (PARTICLE_BYTES[precision] +
+    return FIXED_BYTES[precision] + req.nodes * NODE_BYTES[precision] + req.capacity * (PARTICLE_BYTES[precision] +
                                                                             RECORD_BYTES)
 
 
@@ -181,11 +186,12 @@ class Server:
 
     ``execute(request) -> result`` does the work (default: build, run the
     request's steps, collect, close); ``footprint(request) -> bytes`` sizes
-    it.  Both can be replaced, so the admission logic is testable without a
-    GPU."""
+    it; ``idle(release) -> bytes`` is the memory kept from closed instances,
+    given back with release.  All can be replaced, so the admission logic is
+    testable without a GPU."""
 
     def __init__(self, budget_bytes, workers=16, precision="split32", backfill=True, max_bypass=8,
-                 execute=None, footprint=None):
+                 execute=None, footprint=None, idle=None):
         self.budget = float(budget_bytes)
         self.workers = int(workers)
         self.precision = precision
@@ -193,6 +199,7 @@ class Server:
         self.max_bypass = int(max_bypass)
         self.execute = execute or self._execute
         self.footprint = footprint or (lambda r: footprint_bytes(r, precision))
+        self.idle = idle or (self._idle if execute is None else lambda release: 0)
 
     def _execute(self, req):
         g, _ = build(req, self.precision)
@@ -200,6 +207,18 @@ class Server:
         out = collect(g, req)
         g.close()
         return out
+
+    @staticmethod
+    def _idle(release):
+        from . import gpu
+
+        return gpu.idle_memory(release)
+
+    def _make_room(self, in_use):
+        """Closed instances' memory stays within what in_use leaves of the
+        budget (a request's own blocks are at most its footprint when it ends)."""
+        if self.idle(False) > self.budget - in_use:
+            self.idle(True)
 
     def _pick(self, queue, in_use, bypassed):
         """Index in `queue` of the request to start next, or None."""
@@ -261,6 +280,7 @@ class Server:
                         req = queue.pop(k)
                         fp = self.footprint(req)
                         in_use[0] += fp
+                        self._make_room(in_use[0])
                         peak[0] = max(peak[0], in_use[0])
                         running[0] += 1
                         t_start = time.perf_counter() - t0
