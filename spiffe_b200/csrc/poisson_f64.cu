@@ -1007,9 +1007,11 @@ static int launch_sor(const DevMesh *m, Poisson64Work *w, double *Psi, const dou
   DevMesh mm = *m;
   cudaError_t e;
   // (end conditions set after the set-up move the update rows: the bands
-  // follow those they were laid out for)
+  // follow those they were laid out for; and they divide by the diagonals
+  // through their reciprocals, which gives the quotients' bits in div_by's
+  // range)
   const int lo = m->left_bc == SPIFFE_DIRICHLET ? 0 : 1, hi = m->right_bc == SPIFFE_DIRICHLET ? m->nz - 1 : m->nz - 2;
-  if (w->band_kernel && lo == w->band_lo && hi == w->band_hi) {
+  if (w->band_kernel && lo == w->band_lo && hi == w->band_hi && div_by_takes(-a.e) && div_by_takes(-a.e2c_axis)) {
     SorBand sb{w->band_R, w->band_H, 1 / a.e, 1 / a.e2c_axis, w->band_mem, w->band_xb, w->band_bar};
     e = cudaMemsetAsync(w->band_bar, 0, 32 * sizeof(unsigned long long), s);
     if (e != cudaSuccess)

@@ -237,3 +237,64 @@ def test_unordered_sums_of_many_particles(nz, nr, spread, n):
     for k in ("Jz", "Jr"):
         assert np.any(got["ordered"][k] != 0)
         assert np.all(np.abs(got["sum"][k] - got["ordered"][k]) <= n * 2.3e-16 * np.abs(got["size"][k])), k
+
+
+# numerators of the divisions by dr, dz, eps0 and the SOR's diagonals: ordinary
+# ones; quotients that are subnormal, or lie half way between two subnormals
+# (powers of two apart); near overflow
+SCALES = [1.0, 2.0 ** -941, 1e-290, 1e-305, 2.0 ** -1030, 2.0 ** -1074, 2.0 ** 899, 2.0 ** 950, 1e300]
+
+
+def scaled(rng, shape, scale):
+    """Random values around a scale (whole multiples of the smallest subnormal
+    where that is the scale), zeros of both signs among them."""
+    x = np.round(rng.normal(size=shape) * 64) * scale
+    return np.where(rng.uniform(size=shape) < 0.05, np.copysign(0.0, x), x)
+
+
+@pytest.mark.parametrize("scale", SCALES)
+@pytest.mark.parametrize("dz, dr", [(None, None), (4.0, 2.0), (6.0, 3.0), (2.0 ** -60, 2.0 ** 60), (2.0 ** -61, 2.0 ** 61)])
+def test_field_update_divides_as_the_reference_does(oracle, scale, dz, dr):
+    """The update's quotients are formed from reciprocals: the same bits at
+    every size of numerator, infinities and NaN among them, for the divisors
+    that take that way and for those beyond them."""
+    f = pillbox(33, 29)
+    if dz:
+        f.mesh.dz, f.mesh.dr = dz, dr
+    f.mesh.dt = 0.25 if scale > 1e200 or scale < 1e-200 else 1e-13
+    rng = np.random.default_rng(7)
+    for n in ("Ez", "Er", "Bphi", "Jz", "Jr"):
+        f[n] = scaled(rng, f.shape, scale)
+    f["Ez"][11, 7], f["Jz"][13, 9], f["Er"][20, 11] = np.inf, -np.inf, np.nan
+    g = gpu.GpuInstance(f)
+    g.upload_fields(f)
+    ref = f.copy()
+    for _ in range(2):
+        g.advance_fields()
+        oracle.advance_fields(ref)
+    out = g.fields(f)
+    for n in ("Ez", "Er", "Bphi", "Bphi2"):
+        assert np.array_equal(out[n], ref[n], equal_nan=True), n
+    g.close()
+
+
+@pytest.mark.parametrize("nz, nr", [(40, 31), (300, 411)])  # one cluster, the grid
+@pytest.mark.parametrize("dz, dr, scale", [(None, None, s) for s in SCALES] +
+                         # beyond the divisors of the reciprocal's way: quotients are subnormal where the numerators
+                         # are not, here half way between two subnormals in one of twenty nodes
+                         [(2.0 ** -70, 2.0 ** -71, 2.0 ** k) for k in (-881, -890, -900)])
+def test_sor_divides_as_the_reference_does(oracle, nz, nr, dz, dr, scale):
+    f = pillbox(nz, nr)
+    if dz:
+        f.mesh.dz, f.mesh.dr = dz, dr
+    rng = np.random.default_rng(9)
+    f["Q"] = scaled(rng, f.shape, scale) if not dz else rng.integers(1, 1 << 53, f.shape) * (scale * 2.0 ** -53)
+    f["Psi"] = np.zeros(f.shape)
+    g = gpu.GpuInstance(f)
+    for limit in (2, 9):
+        g.upload_fields(f)
+        ref = f.copy()
+        n, _, _ = oracle.solve_poisson(ref, ref["Psi"], ref["Q"], 1e-300, limit)
+        assert g.solve_poisson(0, 1e-300, limit) == n
+        assert np.array_equal(g.fields(f)["Psi"], ref["Psi"], equal_nan=True), limit
+    g.close()
