@@ -191,7 +191,7 @@ struct DevCounts {
   long long sor_halfsweeps, sor_solves;   // red-black half-sweeps and Poisson solves run (either solver)
   long long mg_cycles;                    // multigrid V-cycles run
   unsigned int error;                     // SPIFFE_DEV_ERR_* bits
-  unsigned int pad;
+  unsigned int compacting;                // blocks of the compaction that have read the counts
 };
 
 // One particle lost in a push, with what the loss epilogue of

@@ -1,5 +1,6 @@
-// spiffe_b200/csrc/compact.cuh -- removal of the particles lost in a push, by
-// one block: the common part of the two forms' compaction kernels.
+// spiffe_b200/csrc/compact.cuh -- removal of the particles lost in a push: by
+// one block, the common part of the two forms' compaction kernels, and a burst
+// by every block of a grid.
 #pragma once
 
 #include <cub/block/block_radix_sort.cuh>
@@ -52,11 +53,10 @@ __device__ __forceinline__ int collect(long long span, int32_t *out, Take take, 
 // the push appended the losses, which follows the timing of its blocks.  The
 // holes, collected from the push's list, are put in order by a block radix
 // sort when there are at most CT * CT_ITEMS of them, else collected again from
-// all slots, CT_SCAN a thread (a burst of losses: a particle is lost once, so
-// what one block takes longer for it than the grid would, about a nanosecond
-// a loss, is little beside the particle's pushes).  is_lost(i): slot i was
-// lost in this push; move(dst, src) copies a particle.  Called by all CT
-// threads of one block.
+// all slots, CT_SCAN a thread (one block takes 4 to 35 ns a loss of a burst: the
+// split form, whose particle is lost once; the FP64 form shares a burst among
+// blocks, below).  is_lost(i): slot i was lost in this push; move(dst, src)
+// copies a particle.  Called by all CT threads of one block.
 template <bool REVERSE, class Lost, class Move>
 __device__ __forceinline__ void compact_block(long long n_lost, long long np, const int32_t *lost_list, int32_t *holes,
                                               int32_t *donors, Lost is_lost, Move move)
@@ -92,6 +92,104 @@ __device__ __forceinline__ void compact_block(long long n_lost, long long np, co
       [&](long long i) { return (int)(new_np + i); });
   __syncthreads();
   for (int k = tid; k < n_holes; k += CT)
+    move(holes[k], donors[REVERSE ? n_holes - 1 - k : k]);
+}
+
+// ---- a burst of losses, by every block of a grid
+//
+// The same pairing from the flags lost[] (bytes 0 or 1, readable to the end of
+// the 16-byte word that holds the last).  A block takes the holes of a chunk of
+// slots; it counts for itself the holes before and after its chunk and finds the
+// survivors of its holes' ranks in the tail, so no block waits for another: the
+// flags of a million particles are 1 MB from L2, some 10 us a block.
+
+// Which of the slots i .. i+15 (i a multiple of 16) that lie in [lo, hi) have lost[] == want: bits 0 .. 15
+__device__ __forceinline__ unsigned flags16(const uint8_t *lost, int i, int lo, int hi, bool want)
+{
+  const uint4 x = *reinterpret_cast<const uint4 *>(lost + i);
+  auto four = [](unsigned v) { return ((v & 0x01010101u) * 0x01020408u) >> 24 & 15u; }; // a bit a byte
+  unsigned m = four(x.x) | four(x.y) << 4 | four(x.z) << 8 | four(x.w) << 12;
+  if (!want)
+    m ^= 0xffffu;
+  if (i < lo)
+    m &= 0xffffu << (lo - i);
+  if (i + 16 > hi)
+    m &= (1u << max(hi - i, 0)) - 1;
+  return m;
+}
+
+// the calling thread's share of the number of lost in [lo, hi)
+__device__ __forceinline__ int count_lost(const uint8_t *lost, int lo, int hi)
+{
+  int n = 0;
+#pragma unroll 4
+  for (int i = (lo & ~15) + 16 * (int)threadIdx.x; i < hi; i += 16 * CT)
+    n += __popc(flags16(lost, i, lo, hi, true));
+  return n;
+}
+
+// out[rank] = slot for the slots of [lo, hi) with lost[] == want that have ranks
+// r0 .. r1-1; the first of them all has rank `rank`.  A warp takes a run of slots.
+__device__ __forceinline__ void place(const uint8_t *lost, int lo, int hi, bool want, int rank, int r0, int r1, int32_t *out)
+{
+  __shared__ int found[CT / 32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int first = lo >> 4, last = (hi + 15) >> 4, per = ((last - first + CT / 32 - 1) / (CT / 32) + 31) & ~31;
+  const int k0 = first + w * per, k1 = min(k0 + per, last);
+  int n = 0;
+#pragma unroll 4
+  for (int k = k0 + lane; k < k1; k += 32)
+    n += __popc(flags16(lost, 16 * k, lo, hi, want));
+  n = __reduce_add_sync(0xffffffffu, n);
+  if (lane == 0)
+    found[w] = n;
+  __syncthreads();
+  for (int v = 0; v < w; v++)
+    rank += found[v];
+  __syncthreads(); // found[] is used again
+  if (rank >= r1 || rank + n <= r0)
+    return;
+  for (int k = k0 + lane; k - lane < k1 && rank < r1; k += 32) {
+    unsigned m = k < k1 ? flags16(lost, 16 * k, lo, hi, want) : 0u;
+    int upto = __popc(m);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, d);
+      upto += lane >= d ? v : 0;
+    }
+    for (int at = rank + upto - __popc(m); m; m &= m - 1, at++)
+      if (at >= r0 && at < r1)
+        out[at] = 16 * k + __ffs(m) - 1;
+    rank += __shfl_sync(0xffffffffu, upto, 31);
+  }
+}
+
+template <bool REVERSE, class Move>
+__device__ __forceinline__ void compact_burst(int n_lost, int np, const uint8_t *lost, int32_t *holes, int32_t *donors, Move move)
+{
+  __shared__ int sum[3];
+  const int new_np = np - n_lost, tid = threadIdx.x;
+  const int chunk = ((new_np + (int)gridDim.x - 1) / (int)gridDim.x + 15) & ~15;
+  const int a0 = (int)min((long long)blockIdx.x * chunk, (long long)new_np), a1 = (int)min((long long)a0 + chunk, (long long)new_np);
+  if (tid < 3)
+    sum[tid] = 0;
+  __syncthreads();
+  int n[3] = {count_lost(lost, 0, a0), count_lost(lost, a0, a1), count_lost(lost, a1, new_np)};
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    n[k] = __reduce_add_sync(0xffffffffu, n[k]);
+    if ((tid & 31) == 0 && n[k])
+      atomicAdd(sum + k, n[k]);
+  }
+  __syncthreads();
+  const int h0 = sum[0], own = sum[1], n_holes = h0 + own + sum[2];
+  if (!own)
+    return;
+  const int d0 = REVERSE ? n_holes - h0 - own : h0;
+  place(lost, a0, a1, true, h0, h0, h0 + own, holes);
+  place(lost, new_np, np, false, 0, d0, d0 + own, donors);
+  __syncthreads();
+  for (int k = h0 + tid; k < h0 + own; k += CT)
     move(holes[k], donors[REVERSE ? n_holes - 1 - k : k]);
 }
 

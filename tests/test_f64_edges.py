@@ -137,11 +137,14 @@ def test_sor_follows_ends_set_after_setup(oracle):
     assert np.array_equal(g.fields(fd)["Psi"], ref["Psi"])
 
 
-@pytest.mark.parametrize("n, n_lost", [(1, 1), (2, 1), (40, 39), (1500, 1024), (9000, 4096), (20000, 6000), (40000, 33000)])
+@pytest.mark.parametrize("n, n_lost", [(1, 1), (2, 1), (40, 39), (1500, 1024), (9000, 4096), (20000, 6000), (40000, 33000),
+                                       (32769, 1024), (32769, 1025), (32784, 32783), (50001, 50001), (99999, 50000),
+                                       (300000, 1500), (300000, 298000), (1100000, 400000)])
 def test_swap_compaction_pairs_holes_with_the_last_survivors(n, n_lost):
-    """One block removes the lost: the j-th lost slot takes the j-th survivor
-    counted from the end, whatever the number of losses (none, a block's, more
-    than are sorted), and the counts are ready for the next push."""
+    """The j-th lost slot takes the j-th survivor counted from the end, whatever
+    the number of losses (none, a block's, more than are sorted, a burst shared
+    by two and by all blocks, everything), and the counts are ready for the next
+    push."""
     f = pillbox(60, 50)
     m = f.mesh
     rng = np.random.default_rng(n)
