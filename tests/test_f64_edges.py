@@ -214,21 +214,50 @@ def test_current_is_cleared_and_read_where_it_lies(oracle):
 @pytest.mark.parametrize("n", [196608, 196609, 200000])
 def test_unordered_sums_of_many_particles(nz, nr, spread, n):
     """From 3 2^16 particles a block sums its particles in shared memory before
-    they go to J, where their nodes span few enough (all meshes and beams here
-    but the last), against the ordered sums.  Either order of n additions is
-    within n eps / 2 of the exact sum of the contributions' magnitudes, which
-    the same beam with positive velocities deposits."""
+    they go to J, where their nodes span few enough (the beam of a tenth of the
+    mesh; the others go to J one by one)."""
     f = pillbox(nz, nr)
     m = f.mesh
     rng = np.random.default_rng(n + nr)
-    b = abi.Beam(n)
-    v = rng.normal(size=(2, n)) * 1e8
     z = (0.45 + spread * rng.uniform(-0.45, 0.55, n)) * (m.zmax - m.zmin) + m.zmin
     r = spread * rng.uniform(0, 1, n) ** 2 * m.dr * (nr - 1)
-    status = np.where(rng.uniform(size=n) < 0.9, abi.PART_ACTIVE, 0).astype(np.uint64)
+    unordered_is_ordered(f, z, r, np.where(rng.uniform(size=n) < 0.9, abi.PART_ACTIVE, 0), rng)
+
+
+@pytest.mark.parametrize("modes", [MODES, MODES | abi.FL_TE_FIELDS, (MODES | abi.FL_TE_FIELDS) & ~abi.FL_TM_FIELDS])
+@pytest.mark.parametrize("rows, cols, a_cell, order", [(32, 64, 0, "random"), (33, 63, 0, "random"), (32, 65, 0, "random"),
+                                                       (1, 1, 0, "random"), (300, 2, 0, "random"), (32, 64, 0, "cells"),
+                                                       (500, 60, 6, "cells"), (500, 60, 16, "cells"), (40, 40, 200, "cells")])
+def test_unordered_sums_of_a_block(rows, cols, a_cell, order, modes):
+    """Blocks of 2048 particles that span 2048 nodes (the most that a block sums
+    itself) and a few more, in random order and in the order of their cells,
+    where whole warps or groups of two to thirty lanes of a warp add to one
+    node; a tenth of the particles is inactive."""
+    n = 200000
+    f = pillbox(520, 70, modes)
+    rng = np.random.default_rng(rows * cols + a_cell)
+    if order == "random":
+        cell = rng.integers(0, rows * cols, n)
+    elif a_cell:  # about a_cell particles in each of the first cells
+        cell = np.repeat(np.arange(n), rng.integers(a_cell // 2, a_cell * 3 // 2 + 1, n))[:n] % (rows * cols)
+    else:
+        cell = np.sort(rng.integers(0, rows * cols, n))
+    # the nearest nodes of both components' stencils are the cell's own
+    z, r = 3 + cell % rows + rng.uniform(0.1, 0.4, n), cell // rows + rng.uniform(0.1, 0.4, n)
+    unordered_is_ordered(f, z * f.mesh.dz + f.mesh.zmin, r * f.mesh.dr,
+                         np.where(rng.uniform(size=n) < 0.9, abi.PART_ACTIVE, 0), rng)
+
+
+def unordered_is_ordered(f, z, r, status, rng):
+    """The deposition against the ordered sums.  Either order of n additions is
+    within n eps / 2 of the exact sum of the contributions' magnitudes, which
+    the same beam with positive velocities deposits."""
+    n, status = len(z), status.astype(np.uint64)
+    b = abi.Beam(n)
+    v = rng.normal(size=(3, n)) * 1e8
     got = {}
     for name, order, vel in (("sum", 0, v), ("ordered", 1, v), ("size", 1, np.abs(v))):
-        b.set(n, z=z, r=r, vz=vel[0], vr=vel[1], Q=np.full(n, -1e-15), particleID=np.arange(1, n + 1), status=status)
+        b.set(n, z=z, r=r, vz=vel[0], vr=vel[1], vphi=vel[2], Q=np.full(n, -1e-15), particleID=np.arange(1, n + 1), status=status)
         b.npActive, b.nextParticleID, b.QoMC = int((status > 0).sum()), n + 1, QoMC
         g = gpu.GpuInstance(f, capacity=n)
         g.set_deposit_order(order)
@@ -237,7 +266,8 @@ def test_unordered_sums_of_many_particles(nz, nr, spread, n):
         g.deposit()
         got[name] = g.fields(f)
         g.close()
-    for k in ("Jz", "Jr"):
+    names = ("Jz", "Jr") * bool(f.mesh.modes & abi.FL_TM_FIELDS) + ("Jphi",) * bool(f.mesh.modes & abi.FL_TE_FIELDS)
+    for k in names:
         assert np.any(got["ordered"][k] != 0)
         assert np.all(np.abs(got["sum"][k] - got["ordered"][k]) <= n * 2.3e-16 * np.abs(got["size"][k])), k
 

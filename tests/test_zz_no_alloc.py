@@ -7,8 +7,8 @@ C ABI on device arrays this test owns, twice in a row -- the second call
 warm-starts from the first's result with a new driving term, so the shared
 scratch array is reused with stale contents -- and each result is compared
 with spiffe_gpu_solve_poisson_cyl on an instance holding the same inputs.
-Both run the same kernel with the same grid, so the comparison is exact
-(the tolerance the other SOR parity tests use).
+Both update a node with the same operations on the same values, so the
+comparison is exact (the tolerance the other SOR parity tests use).
 """
 import ctypes as C
 
