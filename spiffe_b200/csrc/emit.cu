@@ -16,18 +16,6 @@ namespace {
 
 constexpr int T = 256;
 
-__device__ __forceinline__ void births_commit(long long total, long long capacity, int mode, DevCounts *cnt)
-{
-  if (cnt->np + total > capacity)
-    return;
-  cnt->np += total;
-  if (mode == SPIFFE_BIRTH_TEST) // inactive and without an ID, test_beam.c:104
-    return;
-  cnt->npActive += total;
-  if (mode != SPIFFE_BIRTH_LIST) // listed particles carry the IDs given at their queueing
-    cnt->nextParticleID += total;
-}
-
 __device__ __forceinline__ void birth(const DevMesh &m, const DevFields<double> &f, const DevBeam64 &b,
                                       const BirthParams &p, DevCounts *cnt)
 {

@@ -27,8 +27,8 @@ struct Coef64 {
 // TM kernels, TAKES: dz and dr lie where div_by holds (else plain divisions).
 // A node's two quotients were most of the instructions of either kernel; they
 // are the reference's divisions by eps0, dr and dz, correctly rounded, by a
-// product and corrections (div_by).
-// FDTD64FIG
+// product and corrections (div_by): a step 11.0 -> 10.2 us on 1201 x 329, 48.6 ->
+// 45.3 on 3001 x 821 and 6.3 either way on 301 x 83, which is launches.
 template <bool TAKES> __device__ __forceinline__ double over(double x, double e, double y)
 {
   return TAKES ? div_by(x, e, y) : x / e;

@@ -108,6 +108,20 @@ struct BirthBin {
 #define SPIFFE_BIRTH_TEST 3
 #define SPIFFE_BIRTH_LIST 4 // explicit particles (secondary electrons): list holds BIRTH_LIST_COLS rows of total
 #define BIRTH_LIST_COLS 10  // z, r, pz, pr, vz, vr, Q, t0, generation, particleID
+#ifdef __CUDACC__
+// the counts after births of either form that fit the arrays
+__device__ __forceinline__ void births_commit(long long total, long long capacity, int mode, DevCounts *cnt)
+{
+  if (cnt->np + total > capacity)
+    return;
+  cnt->np += total;
+  if (mode == SPIFFE_BIRTH_TEST) // inactive and without an ID, test_beam.c:104
+    return;
+  cnt->npActive += total;
+  if (mode != SPIFFE_BIRTH_LIST) // listed particles carry the IDs given at their queueing
+    cnt->nextParticleID += total;
+}
+#endif
 struct BirthParams {
   long long total;
   uint64_t key, counter_base;

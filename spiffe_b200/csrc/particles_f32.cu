@@ -1006,18 +1006,6 @@ __global__ void k_permute(DevBeam32 dst, DevBeam32 src, const int32_t *idx, cons
 
 // ---- births (cathode.c:464-659) into the split beam
 
-__device__ __forceinline__ void births_commit(long long total, long long capacity, int mode, DevCounts *cnt)
-{
-  if (cnt->np + total > capacity)
-    return;
-  cnt->np += total;
-  if (mode == SPIFFE_BIRTH_TEST) // inactive and without an ID, test_beam.c:104
-    return;
-  cnt->npActive += total;
-  if (mode != SPIFFE_BIRTH_LIST) // listed particles carry the IDs given at their queueing
-    cnt->nextParticleID += total;
-}
-
 __global__ void __launch_bounds__(T) k_births32(DevMesh m, DevFields32 f, DevBeam32 b, BirthParams p, DevCounts *cnt,
                                                  S32Scales sc, int deposit)
 {

@@ -761,9 +761,17 @@ __device__ __forceinline__ void tile_add(double *tile, int at, double v)
     atomicAdd(tile + at, v);
 }
 
-// Below this many particles too few blocks for the SMs.  200,000 on 3001 x 821:
-// a bunch 17 to 19 us against 33 to 41 straight to J, spread over the mesh 12
-// against 12 (23 in the order of their radii).
+// The line is where a beam spread over the mesh, whose blocks find more nodes
+// than a tile has, loses little: its blocks add straight to J all the same, later.
+// Jz and Jr in us, straight to J / block sums (a bunch in random order, in cell
+// order; spread, spread in the order of radii):
+//                 3001 x 821                          301 x 83
+//    32,768  10/17  11/19   9/12   9/15     52/21   66/16   8/16   8/18
+//   131,072  23/17  27/19  10/12  10/23    192/21  246/16  13/17  13/16
+//   196,608  32/17  40/18  12/12  12/23    286/21  366/16  17/17  17/17
+//   262,144  41/17  53/18  13/13  13/23    378/21  486/16  21/17  21/16
+// (601 x 165 between them.)  A bunch gains well below the line, on a coarse mesh
+// from 16,384 particles; which of the two a beam is the host does not know.
 constexpr long long DEPOSIT_TILE_MIN = 3 << 16;
 __global__ void __launch_bounds__(DT, 2) k_deposit_tile(DevMesh m, DevFields<double> f, DevBeam64 b, const DevCounts *cnt,
                                                       int first, int last)

@@ -669,6 +669,10 @@ int sb_rows(int cols, int R)
   return groups ? (R + groups - 1) / groups : 0;
 }
 
+// An instance holds the driving terms of all a thread's rows in registers, so one
+// with rows to spare spills more: 36 bytes a thread with seven, 68 with eight, none
+// with four (3001 x 821, seven rows a thread: 8.3 us a half-sweep, 8.5 with the
+// instance for eight; 2400 x 900, seven: 7.6 and 7.9).  Five and six take seven's.
 const void *sb_kernel(int rows)
 {
   return rows <= 2   ? (const void *)k_sor_band<2, false>

@@ -197,8 +197,9 @@ struct S32State {
   // what J holds: unknown, zero, or exactly the deposit of the current
   // particles (left by the push of the previous step inside the loop)
   int j_state = S32_J_UNKNOWN;
-  // the particles sorted every 40 steps (on the gun, 20 / 40 / 80 / 160: 173.5 /
-  // 170.8 / 170.5 / 171.1 us a step; 10: 178.8)
+  // the particles sorted every 40 steps (640 steps of the gun, every 10 / 20 / 40 /
+  // 80 / 160 / 320: 108.5 / 101 / 97.4 / 95.9 / 95.5 / 95.3 us a step; a beam whose
+  // particles pass one another sooner loses its order sooner)
   long long sort_interval = 40, since_sort = 0;
   double *staging = nullptr; // device FP64 staging for host transfers
   size_t staging_n = 0;
