@@ -953,11 +953,11 @@ __global__ void k_compact_reference(DevCounts *cnt, int oa)
 // j-th lost slot (ascending) taking the j-th survivor counted from the end.
 // One launch, where flags, a scan, a map and the moves took six (3.9 us each of
 // launching, the whole step of a small problem).  Few losses are the first
-// block's; of a burst every block takes a part (one block alone took 8 ns a loss
-// and more: a push of two million that loses half 8.7 ms, now 1.0, as with the
-// six launches; a million that lose 20,000 a push 0.59 -> 0.16).  The last block
-// to have read the counts sets them for the next push.  A push without losses
-// takes 0.4 us more with 4 to 64 blocks than with 1 and none with 2.
+// block's, and the others end at once; of a burst every block takes a part (one
+// block alone took 8 ns a loss and more: a push of two million that loses half
+// 8.7 ms, now 1.0, as with the six launches; a million that lose 20,000 a push
+// 0.59 -> 0.16).  In a burst the last block to have read the counts sets them for
+// the next push.
 constexpr int BURST = 1024; // losses
 // blocks for a burst of at most n particles
 unsigned burst_blocks(long long n)
@@ -968,24 +968,29 @@ __global__ void __launch_bounds__(CT) k_compact_swap(DevBeam64 b, const uint8_t 
                                                       DevCounts *cnt, int32_t *holes, int32_t *donors, int oa)
 {
   step_begin();
-  const long long n_lost = cnt->n_lost, np = cnt->np;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    bool last = true;
-    if (gridDim.x > 1) {
-      __threadfence();
-      last = atomicAdd(&cnt->compacting, 1u) == gridDim.x - 1;
-      if (last)
-        cnt->compacting = 0;
-    }
-    if (last)
-      end_push(cnt, n_lost, np - n_lost, oa);
-  }
+  // (without a burst the first block may have set the count to 0 already when
+  // another reads it: no burst either way)
+  const long long n_lost = *(volatile long long *)&cnt->n_lost, np = *(volatile long long *)&cnt->np;
   auto move = [&](int dst, int src) { move64(b, dst, src); };
-  if (n_lost > BURST && gridDim.x > 1)
+  if (n_lost > BURST && gridDim.x > 1) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (atomicAdd(&cnt->compacting, 1u) == gridDim.x - 1) {
+        cnt->compacting = 0;
+        end_push(cnt, n_lost, np - n_lost, oa);
+      }
+    }
     compact_burst<true>((int)n_lost, (int)np, lost, holes, donors, move);
-  else if (n_lost > 0 && blockIdx.x == 0)
+    return;
+  }
+  if (blockIdx.x > 0)
+    return;
+  if (n_lost > 0)
     compact_block<true>(n_lost, np, lost_list, holes, donors, [&](int i) { return lost[i] != 0; }, move);
+  __syncthreads();
+  if (threadIdx.x == 0)
+    end_push(cnt, n_lost, np - n_lost, oa);
 }
 
 // The on-axis fields' extremes of the coming push (advance_particles.c:113-114)
