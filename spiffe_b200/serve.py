@@ -212,7 +212,10 @@ class Server:
     def _idle(release):
         from . import gpu
 
-        return gpu.idle_memory(release)
+        try:
+            return gpu.idle_memory(release)
+        except gpu.SpiffeGpuError:  # no device: each request reports it
+            return 0
 
     def _make_room(self, in_use):
         """Closed instances' memory stays within what in_use leaves of the

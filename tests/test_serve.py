@@ -169,6 +169,16 @@ def test_footprint_bounds_the_device_memory(precision):
         assert 0 < used <= bound, (r, used, bound)
 
 
+def test_requests_report_a_missing_device_themselves():
+    import torch
+
+    if torch.cuda.is_available():
+        pytest.skip("a GPU is present")
+    reqs = serve.draw_requests(2, steps=1, size_scale=0.2, particle_scale=0.01)
+    rows = serve.Server(1 << 34, workers=2).serve(reqs, rate=1000.0)
+    assert all("SpiffeGpuError" in o["error"] for o in rows)
+
+
 def test_memory_of_closed_instances_is_within_the_budget():
     """What stays from closed requests is given back before a request that
     would not fit beside it starts, and only then."""
